@@ -101,6 +101,18 @@ NF_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort
   }
 }
 
+// One lane of a converged warp, known to the compiler as one: tcgen05 and TMA instructions take their operands from the
+// warp's uniform registers, and inside `if (lane == 0)` every operand costs moves that an elected lane does not pay.
+NF_DEVICE bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(on));
+  return on != 0;
+}
+
 NF_DEVICE void report_status(unsigned int* status, unsigned int code) {
   if (status != nullptr) atomicCAS(status, 0u, code);
 }

@@ -359,7 +359,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* smem = smem_al + 1024;     // ring slots
 
-  const int warp = threadIdx.x >> 5;
+  // The warp number by a shuffle: the compiler then knows that a role's loop counters are the same in all lanes of a warp
+  // and keeps the operands of TMA and tcgen05 instructions in uniform registers (see elect_one). With roles of one thread
+  // (`lane == 0`) the issue of a k-block's four pair MMAs took longer than the MMAs: 2048 x 8192 x 28672 went from 745 to
+  // 619 us (1.29 -> 1.55 PFLOP/s), 2048 x 10240 x 8192 from 255 to 228, 1024 x 8192 x 8192 from 121 to 104.
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
   static_assert(CG == 1 || MT == 1, "CTA pairs cover one M tile per CTA");
@@ -419,8 +423,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer ----------------
+  if (warp == 0) {
+    // ---------------- TMA producer (the whole warp walks the tiles, an elected lane issues) ----------------
     // ring position kept as (slot, phase) counters: the stage count is a runtime value and a
     // division per k-block would sit on this thread's issue path
     uint32_t it = 0, ph = 0;
@@ -439,7 +443,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int need = (CG == 2) ? min(m_tiles - 1, m_grp * 2 + static_cast<int>(rank)) : m_grp * MT + mt_valid - 1;
         const int first = (CG == 2) ? need : m_grp * MT;
         for (int mt_i = max(first, gate_seen + 1); mt_i <= need && ok; ++mt_i) {
-          if (!wait_gate(p, mt_i, abort_flag)) {
+          if (!__all_sync(0xffffffffu, wait_gate(p, mt_i, abort_flag))) {
             report_status(p.status, NF_ST_TIMEOUT_PEER_FLAG);
             raise_abort();
             ok = false;
@@ -449,7 +453,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (need > gate_seen) gate_seen = need;
       }
       for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it, s = (s + 1 == STAGES) ? 0 : s + 1, ph ^= (s == 0)) {
-        if (!wait_or_abort(&empty_bar[s], ph ^ 1, abort_flag)) {
+        if (!__all_sync(0xffffffffu, wait_or_abort(&empty_bar[s], ph ^ 1, abort_flag))) {
           report_status(p.status, NF_ST_TIMEOUT_SMEM_EMPTY);
           raise_abort();
           ok = false;
@@ -457,34 +461,37 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         uint8_t* sa = smem + s * STAGE_BYTES;
         uint8_t* sb = sa + A_BYTES;
-        if (CG == 2) {
-          // Both CTAs' bytes are counted on the even CTA's barrier, which its MMA thread waits on.
-          // A tile past the last row or column is still copied in full (zero filled).
-          const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), 0);
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * (A_TILE_BYTES + B_BYTES));
-          if (gated_epi(EPI))
-            tma_load_2d_pair(sb, rank == 0 ? &tmB0 : &tmB1, fb, kb * BK, nb.col0);
-          else if (WIDE) {
-            const int qrows = BN / 4;
-            tma_load_2d_pair(sb, &tmB0, fb, kb * BK, nb.col0 + static_cast<int>(rank) * qrows);
-            tma_load_2d_pair(sb + qrows * (BK * 2), &tmB0, fb, kb * BK,
-                             nb.col0 + BN / 2 + static_cast<int>(rank) * qrows);
-          } else
-            tma_load_2d_pair(sb, &tmB0, fb, kb * BK, nb.col0 + static_cast<int>(rank) * (BN / 2));
-          tma_load_2d_pair(sa, &tmA, fb, nb.a_k0 + kb * BK, (m_grp * 2 + static_cast<int>(rank)) * BM);
-          continue;
-        }
-        mbar_expect_tx(&full_bar[s], mt_valid * A_TILE_BYTES + B_BYTES);
-        if (gated_epi(EPI)) {
-          tma_load_2d(sb, &tmB0, &full_bar[s], kb * BK, nb.col0);
-          tma_load_2d(sb + B_BYTES / 2, &tmB1, &full_bar[s], kb * BK, nb.col0);
-        } else {
-          tma_load_2d(sb, &tmB0, &full_bar[s], kb * BK, nb.col0);
-        }
+        if (elect_one()) {
+          if (CG == 2) {
+            // Both CTAs' bytes are counted on the even CTA's barrier, which its MMA thread waits on.
+            // A tile past the last row or column is still copied in full (zero filled).
+            const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), 0);
+            if (leader) mbar_expect_tx(&full_bar[s], 2 * (A_TILE_BYTES + B_BYTES));
+            if (gated_epi(EPI))
+              tma_load_2d_pair(sb, rank == 0 ? &tmB0 : &tmB1, fb, kb * BK, nb.col0);
+            else if (WIDE) {
+              const int qrows = BN / 4;
+              tma_load_2d_pair(sb, &tmB0, fb, kb * BK, nb.col0 + static_cast<int>(rank) * qrows);
+              tma_load_2d_pair(sb + qrows * (BK * 2), &tmB0, fb, kb * BK,
+                               nb.col0 + BN / 2 + static_cast<int>(rank) * qrows);
+            } else
+              tma_load_2d_pair(sb, &tmB0, fb, kb * BK, nb.col0 + static_cast<int>(rank) * (BN / 2));
+            tma_load_2d_pair(sa, &tmA, fb, nb.a_k0 + kb * BK, (m_grp * 2 + static_cast<int>(rank)) * BM);
+          } else {
+            mbar_expect_tx(&full_bar[s], mt_valid * A_TILE_BYTES + B_BYTES);
+            if (gated_epi(EPI)) {
+              tma_load_2d(sb, &tmB0, &full_bar[s], kb * BK, nb.col0);
+              tma_load_2d(sb + B_BYTES / 2, &tmB1, &full_bar[s], kb * BK, nb.col0);
+            } else {
+              tma_load_2d(sb, &tmB0, &full_bar[s], kb * BK, nb.col0);
+            }
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-          if (mt < mt_valid)
-            tma_load_2d(sa + mt * A_TILE_BYTES, &tmA, &full_bar[s], nb.a_k0 + kb * BK, (m_grp * MT + mt) * BM);
+            for (int mt = 0; mt < MT; ++mt)
+              if (mt < mt_valid)
+                tma_load_2d(sa + mt * A_TILE_BYTES, &tmA, &full_bar[s], nb.a_k0 + kb * BK, (m_grp * MT + mt) * BM);
+          }
+        }
+        __syncwarp();
       }
     }
     if (CG == 2 && ok) {
@@ -514,9 +521,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
     }
-  } else if (warp == 1 && lane == 0 && leader) {
+  } else if (warp == 1 && leader) {
     // ---------------- MMA issuer (the even CTA of a pair issues for both) ----------------
     const uint32_t idesc = umma_idesc_bf16(BM * CG, WIDE ? BN / 2 : BN);
+    const uint32_t ring_addr = smem_u32(smem);
     uint32_t tcount = 0, ph = 0;
     int s = 0;
     bool ok = true;
@@ -528,7 +536,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int mt_valid = (CG == 2) ? 1 : min(MT, m_tiles - m_grp * MT);
       const uint32_t acc = (ACC_BUFS == 2) ? (tcount & 1) : 0;
       const uint32_t acc_ph = (ACC_BUFS == 2) ? ((tcount >> 1) & 1) : (tcount & 1);
-      if (!wait_or_abort(&tmem_empty[acc], acc_ph ^ 1, abort_flag)) {
+      if (!__all_sync(0xffffffffu, wait_or_abort(&tmem_empty[acc], acc_ph ^ 1, abort_flag))) {
         report_status(p.status, NF_ST_TIMEOUT_TMEM_EMPTY);
         raise_abort();
         break;
@@ -536,45 +544,42 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
       for (int kb = sg.kb0; kb < sg.kb1; ++kb, s = (s + 1 == STAGES) ? 0 : s + 1, ph ^= (s == 0)) {
-        if (!wait_or_abort(&full_bar[s], ph, abort_flag)) {
+        if (!__all_sync(0xffffffffu, wait_or_abort(&full_bar[s], ph, abort_flag))) {
           report_status(p.status, NF_ST_TIMEOUT_SMEM_FULL);
           raise_abort();
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-        const uint32_t b_addr = a_addr + A_BYTES;
+        if (elect_one()) {
+          const uint64_t a_desc = umma_desc_k_sw128(ring_addr + s * STAGE_BYTES);
+          const uint64_t b_desc = a_desc + (A_BYTES >> 4);
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          if (mt < mt_valid) {
+          for (int mt = 0; mt < MT; ++mt) {
+            if (mt < mt_valid) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-              const uint64_t da = umma_desc_k_sw128(a_addr + mt * A_TILE_BYTES + k * UMMA_K * 2);
-              const uint64_t db = umma_desc_k_sw128(b_addr + k * UMMA_K * 2);
-              if (CG == 2) umma_bf16_ss_pair(d_tmem, da, db, idesc, (kb != sg.kb0 || k != 0) ? 1u : 0u);
-              else umma_bf16_ss(d_tmem + mt * BN, da, db, idesc, (kb != sg.kb0 || k != 0) ? 1u : 0u);
-              if (WIDE)   // second half of the tile: the weight rows staged behind the first quarter
-                umma_bf16_ss_pair(d_tmem + BN / 2, da,
-                                  umma_desc_k_sw128(b_addr + (BN / 4) * (BK * 2) + k * UMMA_K * 2), idesc,
-                                  (kb != sg.kb0 || k != 0) ? 1u : 0u);
+              for (int k = 0; k < BK / UMMA_K; ++k) {
+                const uint32_t on = (kb != sg.kb0 || k != 0) ? 1u : 0u;
+                const uint64_t da = a_desc + ((mt * A_TILE_BYTES + k * UMMA_K * 2) >> 4);
+                const uint64_t db = b_desc + (k * UMMA_K * 2 >> 4);
+                if (CG == 2) umma_bf16_ss_pair(d_tmem, da, db, idesc, on);
+                else umma_bf16_ss(d_tmem + mt * BN, da, db, idesc, on);
+                if (WIDE)   // second half of the tile: the weight rows staged behind the first quarter
+                  umma_bf16_ss_pair(d_tmem + BN / 2, da, db + static_cast<uint64_t>((BN / 4) * (BK * 2) >> 4), idesc, on);
+              }
             }
           }
+          // the stage is free (in both CTAs of a pair) once these MMAs have read it
+          if (CG == 2) umma_commit_pair_both(&empty_bar[s]);
+          else umma_commit(&empty_bar[s]);
         }
-        // the stage is free (in both CTAs of a pair) once these MMAs have read it
-        if (CG == 2) {
-          umma_commit_pair_both(&empty_bar[s]);
-        } else {
-          umma_commit(&empty_bar[s]);
-        }
+        __syncwarp();
       }
-      if (ok) {
-        if (CG == 2) {
-          umma_commit_pair_both(&tmem_full[acc]);
-        } else {
-          umma_commit(&tmem_full[acc]);
-        }
+      if (ok && elect_one()) {
+        if (CG == 2) umma_commit_pair_both(&tmem_full[acc]);
+        else umma_commit(&tmem_full[acc]);
       }
+      __syncwarp();
       ++tcount;
     }
   } else if (warp >= 2) {
