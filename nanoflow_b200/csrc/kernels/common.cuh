@@ -223,6 +223,17 @@ NF_DEVICE void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[32]) {
 #pragma unroll
   for (int i = 16; i < 32; ++i) r[i] = 0u;
 }
+// 32 lanes x 16 consecutive fp32 columns into 16 registers.
+NF_DEVICE void tmem_ld_32x32b_x16n(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 NF_DEVICE void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Registers -> TMEM, same shape as the x32 load: thread t writes lane (base_lane + t), 32 columns.
 NF_DEVICE void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -292,15 +303,15 @@ NF_DEVICE void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrives once on the barrier at `bar`'s offset in both CTAs of the pair when every pair MMA issued
-// so far by this thread has completed.
-NF_DEVICE void umma_commit_pair_both(uint64_t* bar) {
-  const uint16_t mask = 3;
+// Arrives once on the barrier at `bar`'s offset in the CTAs of `mask` (both CTAs of the pair) when every pair MMA
+// issued so far by this thread has completed.
+NF_DEVICE void umma_commit_pair_mask(uint64_t* bar, uint16_t mask) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)), "h"(mask)
       : "memory");
 }
+NF_DEVICE void umma_commit_pair_both(uint64_t* bar) { umma_commit_pair_mask(bar, 3); }
 
 // Shared-memory matrix descriptor for a K-major tile stored with the 128-byte swizzle that TMA
 // SWIZZLE_128B produces: rows of 128 bytes, 8-row groups 1024 bytes apart.

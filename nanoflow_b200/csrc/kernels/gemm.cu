@@ -1031,6 +1031,44 @@ sk_fixup_kernel(DevParams p, FixupGeom f) {
   }
 }
 
+#include "gemm_few_rows.cuh"
+
+// The caller's parameters as the kernels take them; geometry and work distribution are filled in by the launchers.
+inline DevParams dev_params(const nfk_gemm_params& g, bool linear) {
+  DevParams p{};
+  p.D = reinterpret_cast<__nv_bfloat16*>(g.D);
+  p.C = reinterpret_cast<const __nv_bfloat16*>(g.C);
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
+  p.bias2 = reinterpret_cast<const __nv_bfloat16*>(g.bias2);
+  p.ldd = g.ldd;
+  p.ldc = g.ldc;
+  p.beta = g.beta;
+  p.M = g.M;
+  p.N = g.N;
+  p.K = g.K;
+  p.status = g.status;
+  for (int r = 0; r < 8; ++r) p.rs_heap[r] = reinterpret_cast<char*>(g.rs_heap[r]);
+  p.rs_rank = g.rs_rank;
+  p.rs_nranks = g.rs_nranks;
+  p.rs_rows_cap = g.rs_rows_cap;
+  p.rs_epoch = g.rs_epoch;
+  p.rs_slab_off = g.rs_slab_off;
+  p.rs_flag_off = g.rs_flag_off;
+  p.gate_flags = g.gate_flags;
+  p.gate_epoch = g.gate_epoch;
+  p.gate_nranks = g.gate_nranks;
+  p.D32 = reinterpret_cast<float*>(g.D32);
+  p.ld32 = g.ld32;
+  p.f32_col0 = g.f32_col0;
+  p.d32_wide = (reinterpret_cast<uintptr_t>(g.D32) & 31) == 0 && g.ld32 % 8 == 0;
+  p.act = GatedAct{g.act, g.act_limit, g.act_alpha, g.act_shift};
+  p.lin_act = linear ? g.lin_act : NFK_LIN_NONE;
+  p.groups = g.groups > 1 ? g.groups : 1;
+  p.group_n = g.N / p.groups;
+  p.group_k = g.group_k;
+  return p;
+}
+
 constexpr int kSmemMax = 227 * 1024;
 
 // Stream-K tail: with `tiles` tiles on `workers` workers, the tiles_dp tiles of the full waves are
@@ -1140,48 +1178,18 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   }
   if (sk.q == 0 && workers > units) workers = units;
   const int ctas = workers * CG;
-  DevParams p;
-  p.D = reinterpret_cast<__nv_bfloat16*>(g.D);
-  p.C = reinterpret_cast<const __nv_bfloat16*>(g.C);
-  p.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
-  p.bias2 = reinterpret_cast<const __nv_bfloat16*>(g.bias2);
+  DevParams p = dev_params(g, EPI == 0);
   p.partial = split_k > 1 ? reinterpret_cast<float*>(g.workspace) : nullptr;
   p.sk_partial = sk.q > 0 ? reinterpret_cast<float*>(g.workspace) : nullptr;
   p.sk_tiles_dp = sk.tiles_dp;
   p.sk_q = sk.q;
   p.sk_max_pieces = sk.max_pieces;
-  p.ldd = g.ldd;
-  p.ldc = g.ldc;
-  p.beta = g.beta;
-  p.M = g.M;
-  p.N = g.N;
-  p.K = g.K;
   p.split_k = split_k;
-  p.status = g.status;
   p.bn = geo.bn;
   p.stages = geo.stages;
   p.acc_bufs = geo.acc_bufs;
   p.tmem_cols = geo.tmem_cols;
-  for (int r = 0; r < 8; ++r) p.rs_heap[r] = reinterpret_cast<char*>(g.rs_heap[r]);
-  p.rs_rank = g.rs_rank;
-  p.rs_nranks = g.rs_nranks;
-  p.rs_rows_cap = g.rs_rows_cap;
-  p.rs_epoch = g.rs_epoch;
-  p.rs_slab_off = g.rs_slab_off;
-  p.rs_flag_off = g.rs_flag_off;
   p.rs_staged = rs_staged ? 1 : 0;
-  p.gate_flags = g.gate_flags;
-  p.gate_epoch = g.gate_epoch;
-  p.gate_nranks = g.gate_nranks;
-  p.D32 = reinterpret_cast<float*>(g.D32);
-  p.ld32 = g.ld32;
-  p.f32_col0 = g.f32_col0;
-  p.d32_wide = (reinterpret_cast<uintptr_t>(g.D32) & 31) == 0 && g.ld32 % 8 == 0;
-  p.act = GatedAct{g.act, g.act_limit, g.act_alpha, g.act_shift};
-  p.lin_act = EPI == 0 ? g.lin_act : NFK_LIN_NONE;
-  p.groups = groups;
-  p.group_n = group_n;
-  p.group_k = g.group_k;
   if (CG == 2) {
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(ctas);
@@ -1254,6 +1262,84 @@ int launch_mt(const nfk_gemm_params& g, int bn, int mt, int cg, int split_k, boo
     case 4: return launch<4, EPI, 1>(g, bn, split_k, stream_k, stream);
     default: return NF_ERR_UNSUPPORTED;
   }
+}
+
+template <bool GATED, int CG>
+int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t stream) {
+  const int groups = g.groups > 1 ? g.groups : 1;
+  CUtensorMap tmW0, tmW1, tmX;
+  int rc = make_tmap_bf16_2d(&tmW0, g.B, g.N, g.K, g.ldb, GATED ? 64 : 128, BK);
+  if (rc != NF_OK) return rc;
+  tmW1 = tmW0;
+  if (GATED) {
+    rc = make_tmap_bf16_2d(&tmW1, g.B2, g.N, g.K, g.ldb, 64, BK);
+    if (rc != NF_OK) return rc;
+  }
+  rc = make_tmap_bf16_2d(&tmX, g.A, g.M, g.K + static_cast<uint64_t>(groups - 1) * g.group_k, g.lda, f.nt / CG, BK);
+  if (rc != NF_OK) return rc;
+  static bool attr_set_dev[kMaxDevices] = {false};
+  bool& attr_set = attr_set_dev[device_slot()];
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(gemm_few_rows_kernel<GATED, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) !=
+        cudaSuccess)
+      return NF_ERR_CUDA;
+    (void)cudaFuncSetAttribute(gemm_few_rows_kernel<GATED, CG>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               cudaSharedmemCarveoutMaxShared);
+    (void)cudaGetLastError();
+    attr_set = true;
+  }
+  FewParams fp;
+  fp.d = dev_params(g, !GATED);
+  fp.d.stages = f.stages;
+  fp.d.tmem_cols = f.tmem_cols;
+  fp.nt = f.nt;
+  fp.tok_tiles = f.tok_tiles;
+  fp.split = f.split;
+  fp.kb_per = f.kb_per;
+  fp.round_tokens = f.round_tokens;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(f.n_tiles * f.tok_tiles * f.split * CG);
+  lc.blockDim = dim3(kFewThreads);
+  lc.dynamicSmemBytes = f.smem_bytes;
+  lc.stream = stream;
+  cudaLaunchAttribute la[1];
+  la[0].id = cudaLaunchAttributeClusterDimension;
+  la[0].val.clusterDim.x = f.split * CG;
+  la[0].val.clusterDim.y = 1;
+  la[0].val.clusterDim.z = 1;
+  lc.attrs = la;
+  lc.numAttrs = f.split * CG > 1 ? 1 : 0;
+  if (cudaLaunchKernelEx(&lc, gemm_few_rows_kernel<GATED, CG>, tmW0, tmW1, tmX, fp) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
+  }
+  if (!GATED && g.norm_w != nullptr) return nfk_rmsnorm(g.norm_out, g.D, g.norm_w, g.M, g.N, g.norm_eps, stream);
+  return NF_OK;
+}
+
+// Whether the few-rows kernel takes this call. Forms that fix how the tile kernel cuts its work (a pinned shape, a CTA or
+// shared-memory budget, gated input, reduce-scatter) stay with it, and so does a norm of rows that are not contiguous.
+bool few_rows_takes(const nfk_gemm_params& g) {
+  if (g.rows_kernel == 2 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
+  if (g.num_ctas > 0 || g.smem_budget_kb > 0 || g.stream_k != 0) return false;
+  if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
+  if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
+  if (g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0) return false;
+  // Measured (4096 to 28672 columns of K, us, tile kernel with its best shape -> this one). Gated: 48 rows 54 -> 46 and
+  // 170 -> 150, 192 rows 75 -> 68 and 212 -> 208, 333 rows 109 -> 110. Linear: 48 rows 17 -> 16, 81 -> 77; 96 rows 42 -> 39,
+  // 34 -> 31, 128 rows 16 -> 19, 93 -> 88. Very many tiles (an output head, 1002): 1 row 179 -> 156, 48 rows 170 -> 170,
+  // 96 rows 174 -> 199: the tokens that each tile stages beside its weights.
+  if (g.epilogue == NFK_EPI_SWIGLU) return g.M <= 256;
+  return g.M <= (g.N <= 65536 ? 96 : 48);
+}
+
+int few_rows(const nfk_gemm_params& g, cudaStream_t stream) {
+  const bool gated = g.epilogue == NFK_EPI_SWIGLU;
+  const int groups = g.groups > 1 ? g.groups : 1;
+  const FewPlan f = few_rows_plan(g.M, g.N, g.K, gated, groups, groups > 1 ? 1 : g.cta_group, g.split_k);
+  if (f.split < 1 || f.split * f.cg > 8 || f.stages < 2) return NF_ERR_BAD_ARG;
+  if (gated) return f.cg == 2 ? launch_few_rows<true, 2>(g, f, stream) : launch_few_rows<true, 1>(g, f, stream);
+  return f.cg == 2 ? launch_few_rows<false, 2>(g, f, stream) : launch_few_rows<false, 1>(g, f, stream);
 }
 
 // Tile-shape choice when the caller leaves it open: a small cost model over the candidate shapes.
@@ -1471,6 +1557,7 @@ extern "C" int nfk_gemm_bf16(const nfk_gemm_params* g, cudaStream_t stream) {
       if (g->rs_heap[r] == nullptr) return NF_ERR_BAD_ARG;
   }
 
+  if (few_rows_takes(*g)) return few_rows(*g, stream);
   Shape s;
   const int rcs = resolve_shape(*g, swiglu, rs, s);
   if (rcs != NF_OK) return rcs;

@@ -87,6 +87,8 @@ typedef struct nfk_gemm_params {
   int lin_act;          // linear epilogue: NFK_LIN_*, applied to the finished columns
   float act_limit, act_alpha, act_shift;   // constants of NFK_ACT_CAPPED
   const void* bias2;    // gated epilogue: [N] bf16 bias of the up half (`bias` is the gate half's), null = none
+  int rows_kernel;      // the kernel for few rows (gemm_few_rows.cuh): 0 = by rule; 1 = it (`cta_group` 1 / 2 and `split_k`
+                        // as given, 0 = choose); 2 = the tile kernel
 } nfk_gemm_params;
 
 int nfk_gemm_bf16(const nfk_gemm_params* p, cudaStream_t stream);
