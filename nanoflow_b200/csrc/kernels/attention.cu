@@ -126,6 +126,48 @@ __device__ __forceinline__ DecodeRange decode_range(const nfk_attn_params& p, in
   return r;
 }
 
+// Chunks before each request (first_chunk[0 .. req_count]) by a scan of the block; returns their number.
+constexpr int kDecListed = 512;
+static_assert(kDecListed == 4 * kDecThreads, "four requests per thread");
+__device__ __forceinline__ int list_chunks(const nfk_attn_params& p, int* first_chunk) {
+  __shared__ int warp_sum_of[kDecThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = threadIdx.x * 4;
+  int n[4], mine = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    n[j] = 0;
+    if (r0 + j < p.req_count) {
+      const int req = p.req_begin + r0 + j;
+      const int np = p.kv_indptr[req + 1] - p.kv_indptr[req];
+      const int seen = np - decode_range(p, req, np, p.kv_last_page_len[req]).skip;
+      n[j] = max(0, min(p.max_chunks, (seen + p.chunk_pages - 1) / p.chunk_pages));
+    }
+    mine += n[j];
+  }
+  int sum = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += v;
+  }
+  if (lane == 31) warp_sum_of[warp] = sum;
+  __syncthreads();
+  int before = sum - mine, all = 0;
+#pragma unroll
+  for (int w = 0; w < kDecThreads / 32; ++w) {
+    if (w < warp) before += warp_sum_of[w];
+    all += warp_sum_of[w];
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    first_chunk[r0 + j] = before;
+    before += n[j];
+  }
+  if (threadIdx.x == kDecThreads - 1) first_chunk[kDecListed] = before;
+  __syncthreads();
+  return all;
+}
+
 // EXT: sink in the denominator, capped scores, distance bias, chunks, page lists that start inside the sequence, queries in
 // wider rows, probabilities as a bf16 pair (in an instantiation of its own).
 template <int HD, int ST, bool EXT>
@@ -137,7 +179,12 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.q_heads / p.kv_heads;
   const int max_chunks = p.chunk_pages > 0 ? p.max_chunks : 1;
-  const long long total = static_cast<long long>(p.req_count) * p.kv_heads * max_chunks;
+  // Work items: (request, kv head, chunk). With chunks, only those that hold pages are listed, if the requests fit the list:
+  // requests of very different length then leave no run of empty items to walk through.
+  __shared__ int first_chunk[kDecListed + 1];
+  const bool listed = max_chunks > 1 && p.req_count <= kDecListed;
+  long long total = static_cast<long long>(p.req_count) * p.kv_heads * max_chunks;
+  if (listed) total = static_cast<long long>(list_chunks(p, first_chunk)) * p.kv_heads;
   const __nv_bfloat16* qbase = reinterpret_cast<const __nv_bfloat16*>(p.q);
   const __nv_bfloat16* pool = reinterpret_cast<const __nv_bfloat16*>(p.kv_pool);
   __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(p.out);
@@ -152,9 +199,19 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
     long long fetched = 0;
     if (threadIdx.x == 0) fetched = static_cast<long long>(gridDim.x) + atomicAdd(&counters[0], 1u);
     do {
-    const int chunk = static_cast<int>(item % max_chunks);
-    const int kvh = static_cast<int>((item / max_chunks) % p.kv_heads);
-    const int bl = static_cast<int>(item / (static_cast<long long>(max_chunks) * p.kv_heads));
+    int chunk, kvh, bl;
+    if (listed) {
+      const int entry = static_cast<int>(item / p.kv_heads);
+      kvh = static_cast<int>(item) - entry * p.kv_heads;
+      bl = 0;                                                 // last request that starts at or before the entry
+      for (int step = kDecListed / 2; step > 0; step >>= 1)
+        if (bl + step < p.req_count && first_chunk[bl + step] <= entry) bl += step;
+      chunk = entry - first_chunk[bl];
+    } else {
+      chunk = static_cast<int>(item % max_chunks);
+      kvh = static_cast<int>((item / max_chunks) % p.kv_heads);
+      bl = static_cast<int>(item / (static_cast<long long>(max_chunks) * p.kv_heads));
+    }
     const int req = p.req_begin + bl;
     const int pg0 = p.kv_indptr[req];
     const int np = p.kv_indptr[req + 1] - pg0;
@@ -190,14 +247,19 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
 
     // This warp's pages: c_begin + warp, + 4, + 8, ...
     const int my_n = (c_end - c_begin - warp + 3) / 4;  // may be <= 0
+    // Page numbers are fetched 32 at a time, one per lane: a load per page in front of its copies would put the latency of
+    // the page table into every step of the loop.
+    int pages = 0;
     auto issue = [&](int i) {
       if (i < my_n) {
-        const int pslot = c_begin + warp + 4 * i;
-        int page = p.kv_indices[pg0 + pslot];
-        if (page < 0 || page >= p.num_pages) {
-          if (lane == 0) report_status(p.status, NF_ST_BAD_INDEX);
-          page = 0;
+        if ((i & 31) == 0) {
+          pages = i + lane < my_n ? p.kv_indices[pg0 + c_begin + warp + 4 * (i + lane)] : 0;
+          if (pages < 0 || pages >= p.num_pages) {
+            report_status(p.status, NF_ST_BAD_INDEX);
+            pages = 0;
+          }
         }
+        const int page = __shfl_sync(0xffffffffu, pages, i & 31);
         const __nv_bfloat16* kp =
             pool + ((static_cast<long long>(page) * 2) * p.kv_heads + kvh) * (kPage * HD);
         const __nv_bfloat16* vp = kp + static_cast<long long>(p.kv_heads) * (kPage * HD);

@@ -1318,13 +1318,14 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
 }
 
 // Whether the few-rows kernel takes this call. Forms that fix how the tile kernel cuts its work (a pinned shape, a CTA or
-// shared-memory budget, gated input, reduce-scatter) stay with it, and so does a norm of rows that are not contiguous.
+// shared-memory budget, gated input, reduce-scatter) stay with it, and so do a norm of rows that are not contiguous and a
+// caller without a workspace, who gets one sum in the order of k.
 bool few_rows_takes(const nfk_gemm_params& g) {
   if (g.rows_kernel == 2 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
   if (g.num_ctas > 0 || g.smem_budget_kb > 0 || g.stream_k != 0) return false;
   if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
   if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
-  if (g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0) return false;
+  if (g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0 || g.workspace == nullptr) return false;
   // Measured (4096 to 28672 columns of K, us, tile kernel with its best shape -> this one). Gated: 48 rows 54 -> 46 and
   // 170 -> 150, 192 rows 75 -> 68 and 212 -> 208, 333 rows 109 -> 110. Linear: 48 rows 17 -> 16, 81 -> 77; 96 rows 42 -> 39,
   // 34 -> 31, 128 rows 16 -> 19, 93 -> 88. Very many tiles (an output head, 1002): 1 row 179 -> 156, 48 rows 170 -> 170,

@@ -83,8 +83,11 @@ def test_same_sum_every_time_and_rows_independent():
     assert torch.equal(outw[:, :4096], ops.gemm(a[:40].contiguous(), w, rows_kernel=1)) and not outw[:, 4096:].any()
 
 
-def test_rule_gives_small_batches_to_it_and_keeps_pinned_shapes():
+def test_rule_gives_small_batches_to_it_and_keeps_other_forms():
+    """With a workspace a small batch goes to it; without one, or with a pinned shape, to the tile kernel (one sum in the
+    order of k, here the same for every width of the tile)."""
     a, w = _data(64, 2048, 1024)
-    assert torch.equal(ops.gemm(a, w), ops.gemm(a, w, rows_kernel=1))
-    pinned = ops.gemm(a, w, tile_m=1, tile_n=128, split_k=1)
-    assert torch.equal(pinned, ops.gemm(a, w, tile_m=1, tile_n=128, split_k=1, rows_kernel=2))
+    ws = torch.empty(1 << 22, device="cuda")
+    assert torch.equal(ops.gemm(a, w, workspace=ws), ops.gemm(a, w, rows_kernel=1))
+    plain = ops.gemm(a, w, rows_kernel=2)
+    assert torch.equal(plain, ops.gemm(a, w)) and torch.equal(plain, ops.gemm(a, w, workspace=ws, tile_m=1, tile_n=128, split_k=1))
