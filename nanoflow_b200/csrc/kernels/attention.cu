@@ -182,6 +182,8 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
   // Work items: (request, kv head, chunk). With chunks, only those that hold pages are listed, if the requests fit the list:
   // requests of very different length then leave no run of empty items to walk through.
   __shared__ int first_chunk[kDecListed + 1];
+  let_next_start();
+  await_previous();
   const bool listed = max_chunks > 1 && p.req_count <= kDecListed;
   long long total = static_cast<long long>(p.req_count) * p.kv_heads * max_chunks;
   if (listed) total = static_cast<long long>(list_chunks(p, first_chunk)) * p.kv_heads;
@@ -425,6 +427,8 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
 
 template <int HD>
 __global__ void attn_decode_merge_kernel(nfk_attn_params p) {
+  let_next_start();
+  await_previous();
   const int bl = blockIdx.x / p.q_heads, head = blockIdx.x % p.q_heads;
   const int req = p.req_begin + bl;
   const int np = p.kv_indptr[req + 1] - p.kv_indptr[req];
@@ -657,13 +661,13 @@ int launch_decode_st(const nfk_attn_params* p, cudaStream_t stream) {
   if (ctas > total) ctas = total;
   static std::atomic<unsigned int> launch_seq{0};
   const int slot = static_cast<int>(launch_seq.fetch_add(1u) % kDecodeCounterSlots);
-  attn_decode_kernel<HD, ST, EXT><<<static_cast<int>(ctas), kDecThreads, Cfg::SMEM_BYTES, stream>>>(*p, slot);
-  if (cudaGetLastError() != cudaSuccess) return NF_ERR_CUDA;
-  if (p->chunk_pages > 0 && max_chunks > 1) {
-    attn_decode_merge_kernel<HD><<<p->req_count * p->q_heads, HD, 0, stream>>>(*p);
-    if (cudaGetLastError() != cudaSuccess) return NF_ERR_CUDA;
-  }
-  return NF_OK;
+  cudaError_t e = launch_early(attn_decode_kernel<HD, ST, EXT>, static_cast<int>(ctas), kDecThreads, Cfg::SMEM_BYTES, stream, 1,
+                               *p, slot);
+  if (e == cudaSuccess && p->chunk_pages > 0 && max_chunks > 1)
+    e = launch_early(attn_decode_merge_kernel<HD>, p->req_count * p->q_heads, HD, 0, stream, 1, *p);
+  if (e == cudaSuccess) return NF_OK;
+  (void)cudaGetLastError();
+  return NF_ERR_CUDA;
 }
 
 template <int HD>

@@ -330,6 +330,15 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// ---- launches that overlap the end of the kernel before them ------------------------------------------
+// A kernel launched by launch_early may start while the kernel before it on the stream still runs, as soon as every CTA
+// of that one has called let_next_start() (or has ended). await_previous() returns when all earlier work is complete and
+// visible; every CTA calls it before its first access to memory that earlier work writes or reads, and no CTA ends
+// without having called it, so that completion stays transitive along a stream. A kernel that allocates tensor memory
+// calls let_next_start() after that: the next kernel cannot then take columns that it still needs.
+NF_DEVICE void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+NF_DEVICE void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- misc -----------------------------------------------------------------------------------------
 NF_DEVICE float warp_sum(float v) {
 #pragma unroll
@@ -346,6 +355,29 @@ NF_DEVICE float2 unpack_bf16x2(uint32_t u) {
 }
 
 #endif  // __CUDACC__
+
+#ifdef __CUDACC__
+// kernel<<<grid, block, smem, stream>>>(args...), allowed to start early (see let_next_start), in clusters of `cluster` CTAs.
+template <class... P, class... A>
+inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, int cluster,
+                                A... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(block);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute la[2];
+  la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  la[0].val.programmaticStreamSerializationAllowed = 1;
+  la[1].id = cudaLaunchAttributeClusterDimension;
+  la[1].val.clusterDim.x = cluster;
+  la[1].val.clusterDim.y = 1;
+  la[1].val.clusterDim.z = 1;
+  lc.attrs = la;
+  lc.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
+}
+#endif
 
 // ---- host: facts about the current device, asked once per device ----------------------------------
 // Number of SMs of the current device (grids are sized from it). Falls back to a B200's 148 when no

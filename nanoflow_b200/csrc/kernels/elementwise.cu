@@ -34,6 +34,8 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* resid,
                const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, int rows,
                int cols, float eps) {
   __shared__ float red[32];
+  let_next_start();
+  await_previous();
   const int nvec = cols >> 3;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * cols);
@@ -111,6 +113,8 @@ __global__ void embedding_kernel(__nv_bfloat16* __restrict__ out,
                                  const int* __restrict__ feedback_src,
                                  const int* __restrict__ prev_tokens, int* ids_out, int n_tokens,
                                  int hidden, int vocab, unsigned int* status) {
+  let_next_start();
+  await_previous();
   const int nvec = hidden >> 3;
   for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
     int id = host_ids != nullptr ? host_ids[t] : 0;
@@ -133,6 +137,8 @@ __global__ void gather_rows_kernel(__nv_bfloat16* __restrict__ out,
                                    const __nv_bfloat16* __restrict__ in,
                                    const int* __restrict__ rows_idx, int n, int cols,
                                    long long ld_in, int in_rows, unsigned int* status) {
+  let_next_start();
+  await_previous();
   const int nvec = cols >> 3;
   for (int r = blockIdx.x; r < n; r += gridDim.x) {
     int s = rows_idx[r];
@@ -213,6 +219,8 @@ argmax_kernel(int* __restrict__ idx_out, float* __restrict__ val_out,
               int col_offset) {
   __shared__ float s_val[kArgmaxThreads / 32];
   __shared__ int s_idx[kArgmaxThreads / 32];
+  let_next_start();
+  await_previous();
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* lr = logits + static_cast<long long>(row) * ld;
     float best = -INFINITY;
@@ -303,6 +311,11 @@ inline int grid_for(int rows) {
   return rows < cap ? (rows > 0 ? rows : 1) : cap;
 }
 inline int ok_or_cuda() { return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA; }
+inline int started(cudaError_t e) {
+  if (e == cudaSuccess) return NF_OK;
+  (void)cudaGetLastError();
+  return NF_ERR_CUDA;
+}
 inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace
@@ -317,9 +330,8 @@ extern "C" int nfk_rmsnorm(void* out, const void* x, const void* w, int rows, in
   if (!out || !x || !w || rows < 0 || cols <= 0 || cols % 8 != 0 ||
       cols > kNormMaxVec * 8 * kNormThreads || !al16(out) || !al16(x) || !al16(w))
     return NF_ERR_BAD_ARG;
-  rmsnorm_kernel<false><<<grid_for(rows), kNormThreads, 0, stream>>>(
-      (bf16*)out, nullptr, (const bf16*)x, (const bf16*)w, rows, cols, eps);
-  return ok_or_cuda();
+  return started(launch_early(rmsnorm_kernel<false>, grid_for(rows), kNormThreads, 0, stream, 1, (bf16*)out,
+                              (bf16*)nullptr, (const bf16*)x, (const bf16*)w, rows, cols, eps));
 }
 
 extern "C" int nfk_add_rmsnorm(void* out, void* resid, const void* x, const void* w, int rows,
@@ -328,9 +340,8 @@ extern "C" int nfk_add_rmsnorm(void* out, void* resid, const void* x, const void
   if (!out || !x || !w || !resid || rows < 0 || cols <= 0 || cols % 8 != 0 ||
       cols > kNormMaxVec * 8 * kNormThreads || !al16(out) || !al16(x) || !al16(w) || !al16(resid))
     return NF_ERR_BAD_ARG;
-  rmsnorm_kernel<true><<<grid_for(rows), kNormThreads, 0, stream>>>(
-      (bf16*)out, (bf16*)resid, (const bf16*)x, (const bf16*)w, rows, cols, eps);
-  return ok_or_cuda();
+  return started(launch_early(rmsnorm_kernel<true>, grid_for(rows), kNormThreads, 0, stream, 1, (bf16*)out, (bf16*)resid,
+                              (const bf16*)x, (const bf16*)w, rows, cols, eps));
 }
 
 extern "C" int nfk_embedding(void* out, const void* table, const int* host_ids,
@@ -342,10 +353,8 @@ extern "C" int nfk_embedding(void* out, const void* table, const int* host_ids,
     return NF_ERR_BAD_ARG;
   if (host_ids == nullptr && (feedback_src == nullptr || prev_tokens == nullptr))
     return NF_ERR_BAD_ARG;
-  embedding_kernel<<<grid_for(n_tokens), 128, 0, stream>>>((bf16*)out, (const bf16*)table, host_ids,
-                                                           feedback_src, prev_tokens, ids_out,
-                                                           n_tokens, hidden, vocab, status);
-  return ok_or_cuda();
+  return started(launch_early(embedding_kernel, grid_for(n_tokens), 128, 0, stream, 1, (bf16*)out, (const bf16*)table,
+                              host_ids, feedback_src, prev_tokens, ids_out, n_tokens, hidden, vocab, status));
 }
 
 extern "C" int nfk_gather_rows(void* out, const void* in, const int* rows_idx, int n, int cols,
@@ -355,9 +364,8 @@ extern "C" int nfk_gather_rows(void* out, const void* in, const int* rows_idx, i
   if (!out || !in || !rows_idx || n < 0 || cols % 8 != 0 || ld_in % 8 != 0 || !al16(out) ||
       !al16(in) || in_rows <= 0)
     return NF_ERR_BAD_ARG;
-  gather_rows_kernel<<<grid_for(n), 128, 0, stream>>>((bf16*)out, (const bf16*)in, rows_idx, n, cols,
-                                                      ld_in, in_rows, status);
-  return ok_or_cuda();
+  return started(launch_early(gather_rows_kernel, grid_for(n), 128, 0, stream, 1, (bf16*)out, (const bf16*)in, rows_idx, n,
+                              cols, ld_in, in_rows, status));
 }
 
 extern "C" int nfk_silu_mul(void* out, const void* gate, const void* up, long long n,
@@ -397,18 +405,16 @@ extern "C" int nfk_argmax(int* idx_out, float* val_out, const void* logits, int 
   if (rows == 0) return NF_OK;
   if (!idx_out || !logits || rows < 0 || cols <= 0 || ld % 8 != 0 || !al16(logits))
     return NF_ERR_BAD_ARG;
-  argmax_kernel<bf16><<<grid_for(rows), kArgmaxThreads, 0, stream>>>(idx_out, val_out, (const bf16*)logits,
-                                                                     rows, cols, ld, col_offset);
-  return ok_or_cuda();
+  return started(launch_early(argmax_kernel<bf16>, grid_for(rows), kArgmaxThreads, 0, stream, 1, idx_out, val_out,
+                              (const bf16*)logits, rows, cols, ld, col_offset));
 }
 
 extern "C" int nfk_argmax_f32(int* idx_out, float* val_out, const float* logits, int rows, int cols,
                               long long ld, int col_offset, cudaStream_t stream) {
   if (rows == 0) return NF_OK;
   if (!idx_out || !logits || rows < 0 || cols <= 0 || ld % 4 != 0 || !al16(logits)) return NF_ERR_BAD_ARG;
-  argmax_kernel<float><<<grid_for(rows), kArgmaxThreads, 0, stream>>>(idx_out, val_out, logits, rows, cols, ld,
-                                                                      col_offset);
-  return ok_or_cuda();
+  return started(launch_early(argmax_kernel<float>, grid_for(rows), kArgmaxThreads, 0, stream, 1, idx_out, val_out, logits,
+                              rows, cols, ld, col_offset));
 }
 
 extern "C" int nfk_argmax_combine(int* idx_out, const float* cand_val, const int* cand_idx,

@@ -422,6 +422,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
+  await_previous();
 
   if (warp == 0) {
     // ---------------- TMA producer (the whole warp walks the tiles, an elected lane issues) ----------------
@@ -851,6 +853,8 @@ inline int sm_count() { return device_sm_count(); }
 // Split-K second pass: D = sum_s partial[s] (+ bias) (+ beta * C), fp32 -> bf16.
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(DevParams p) {
+  let_next_start();
+  await_previous();
   const long long total = static_cast<long long>(p.M) * (p.N >> 3);
   const long long slab = static_cast<long long>(p.M) * p.N;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += 256ll * gridDim.x) {
@@ -885,6 +889,8 @@ constexpr int kRowVec = 8;   // 8-column groups per thread: 8 * 8 * 256 threads 
 __global__ void __launch_bounds__(256)
 splitk_reduce_norm_kernel(DevParams p) {
   __shared__ float red[8];
+  let_next_start();
+  await_previous();
   const int nvec = p.N >> 3;
   const long long slab = static_cast<long long>(p.M) * p.N;
   for (int row = blockIdx.x; row < p.M; row += gridDim.x) {
@@ -966,6 +972,8 @@ struct FixupGeom {
 template <int EPI>
 __global__ void __launch_bounds__(256)
 sk_fixup_kernel(DevParams p, FixupGeom f) {
+  let_next_start();
+  await_previous();
   const int rows_cta = f.mt * BM;
   const int groups = f.out_bn / 8;
   const long long slot_floats = static_cast<long long>(rows_cta) * f.bn;
@@ -1190,34 +1198,20 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   p.acc_bufs = geo.acc_bufs;
   p.tmem_cols = geo.tmem_cols;
   p.rs_staged = rs_staged ? 1 : 0;
-  if (CG == 2) {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(ctas);
-    lc.blockDim = dim3(kGemmThreads);
-    lc.dynamicSmemBytes = geo.smem_bytes;
-    lc.stream = stream;
-    cudaLaunchAttribute la[1];
-    la[0].id = cudaLaunchAttributeClusterDimension;
-    la[0].val.clusterDim.x = 2;
-    la[0].val.clusterDim.y = 1;
-    la[0].val.clusterDim.z = 1;
-    lc.attrs = la;
-    lc.numAttrs = 1;
-    if (cudaLaunchKernelEx(&lc, gemm_tcgen05_kernel<MT, EPI, CG, WIDE>, tmA, tmB0, tmB1, p) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return NF_ERR_CUDA;
-    }
-  } else {
-    gemm_tcgen05_kernel<MT, EPI, CG, WIDE><<<ctas, kGemmThreads, geo.smem_bytes, stream>>>(tmA, tmB0, tmB1, p);
-    if (cudaGetLastError() != cudaSuccess) return NF_ERR_CUDA;
+  if (launch_early(gemm_tcgen05_kernel<MT, EPI, CG, WIDE>, ctas, kGemmThreads, geo.smem_bytes, stream, CG, tmA, tmB0, tmB1, p) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
   }
   if (sk.q > 0 && EPI != 2) {
     FixupGeom f{MT, CG, bn, geo.out_bn, m_groups, (g.K + BK - 1) / BK, sk.rest};
     const long long total = static_cast<long long>(sk.rest) * CG * MT * BM * (geo.out_bn / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    sk_fixup_kernel<gated_epi(EPI) ? 1 : 0><<<static_cast<int>(blocks), 256, 0, stream>>>(p, f);
-    if (cudaGetLastError() != cudaSuccess) return NF_ERR_CUDA;
+    if (launch_early(sk_fixup_kernel<gated_epi(EPI) ? 1 : 0>, static_cast<int>(blocks), 256, 0, stream, 1, p, f) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return NF_ERR_CUDA;
+    }
   }
   p.norm_w = reinterpret_cast<const __nv_bfloat16*>(g.norm_w);
   p.norm_out = reinterpret_cast<__nv_bfloat16*>(g.norm_out);
@@ -1226,15 +1220,18 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   const bool want_norm = EPI == 0 && g.norm_w != nullptr;
   if (split_k > 1 && want_norm && g.N <= kRowVec * 8 * 256) {
     const int blocks = g.M < 16 * sm_count() ? g.M : 16 * sm_count();
-    splitk_reduce_norm_kernel<<<blocks, 256, 0, stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA;
+    if (launch_early(splitk_reduce_norm_kernel, blocks, 256, 0, stream, 1, p) == cudaSuccess) return NF_OK;
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
   }
   if (split_k > 1) {
     const long long total = static_cast<long long>(g.M) * (g.N >> 3);
     long long blocks = (total + 255) / 256;
     if (blocks > 4ll * sm_count()) blocks = 4ll * sm_count();
-    splitk_reduce_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p);
-    if (cudaGetLastError() != cudaSuccess) return NF_ERR_CUDA;
+    if (launch_early(splitk_reduce_kernel, static_cast<int>(blocks), 256, 0, stream, 1, p) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return NF_ERR_CUDA;
+    }
   }
   if (want_norm) {
     // the result rows are complete in D (contiguous rows required): a plain norm launch follows
@@ -1297,19 +1294,9 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
   fp.split = f.split;
   fp.kb_per = f.kb_per;
   fp.round_tokens = f.round_tokens;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(f.n_tiles * f.tok_tiles * f.split * CG);
-  lc.blockDim = dim3(kFewThreads);
-  lc.dynamicSmemBytes = f.smem_bytes;
-  lc.stream = stream;
-  cudaLaunchAttribute la[1];
-  la[0].id = cudaLaunchAttributeClusterDimension;
-  la[0].val.clusterDim.x = f.split * CG;
-  la[0].val.clusterDim.y = 1;
-  la[0].val.clusterDim.z = 1;
-  lc.attrs = la;
-  lc.numAttrs = f.split * CG > 1 ? 1 : 0;
-  if (cudaLaunchKernelEx(&lc, gemm_few_rows_kernel<GATED, CG>, tmW0, tmW1, tmX, fp) != cudaSuccess) {
+  fp.early_weights = g.weights_ready;
+  if (launch_early(gemm_few_rows_kernel<GATED, CG>, f.n_tiles * f.tok_tiles * f.split * CG, kFewThreads, f.smem_bytes, stream,
+                   f.split * CG, tmW0, tmW1, tmX, fp) != cudaSuccess) {
     (void)cudaGetLastError();
     return NF_ERR_CUDA;
   }

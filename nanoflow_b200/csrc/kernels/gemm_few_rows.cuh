@@ -28,7 +28,7 @@ struct FewPlan {
 
 struct FewParams {
   DevParams d;
-  int nt, tok_tiles, split, kb_per, round_tokens;
+  int nt, tok_tiles, split, kb_per, round_tokens, early_weights;
 };
 
 template <bool GATED, int CG>
@@ -91,6 +91,8 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_cons
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
+  if (warp != 0) await_previous();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -100,6 +102,32 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_cons
     // Tiles start at different k-blocks: in step, all CTAs would read the same 128-byte columns of rows that lie a power
     // of two apart, and the same lines of the activations (14336 x 2 x 4096, 1 row: 44.6 -> 41.5 us).
     const int rot = (tile * 13) % nkb;
+    auto load = [&](int st, int i, bool weights, bool tokens) {      // by one lane
+      uint8_t* sw = ring + st * STAGE;
+      const int k0 = (kb0 + (i + rot < nkb ? i + rot : i + rot - nkb)) * BK;
+      if (CG == 2) {
+        const uint32_t fb = mapa_shared(smem_u32(&full_bar[st]), lead_rank);   // both CTAs' bytes count on the leader's barrier
+        if (weights) {
+          if (leader) mbar_expect_tx(&full_bar[st], 2 * STAGE);
+          tma_load_2d_pair(sw, &tmW0, fb, k0, nb.col0);
+          if (GATED) tma_load_2d_pair(sw + kFewWBytes / 2, &tmW1, fb, k0, nb.col0);
+        }
+        if (tokens) tma_load_2d_pair(sw + kFewWBytes, &tmX, fb, k0, tok0 + half * (NT / 2));
+      } else {
+        if (weights) {
+          mbar_expect_tx(&full_bar[st], STAGE);
+          tma_load_2d(sw, &tmW0, &full_bar[st], k0, nb.col0);
+          if (GATED) tma_load_2d(sw + kFewWBytes / 2, &tmW1, &full_bar[st], k0, nb.col0);
+        }
+        if (tokens) tma_load_2d(sw + kFewWBytes, &tmX, &full_bar[st], nb.a_k0 + k0, tok0);
+      }
+    };
+    // The ring is filled with weights while the kernel that computes the tokens may still run.
+    const int early = fp.early_weights ? min(STAGES, nkb) : 0;
+    if (elect_one())
+      for (int i = 0; i < early; ++i) load(i, i, true, false);
+    __syncwarp();
+    await_previous();
     for (; it < nkb; ++it, s = (s + 1 == STAGES) ? 0 : s + 1, ph ^= (s == 0)) {
       if (!__all_sync(0xffffffffu, wait_or_abort(&empty_bar[s], ph ^ 1, abort_flag))) {
         report_status(p.status, NF_ST_TIMEOUT_SMEM_EMPTY);
@@ -107,22 +135,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_cons
         ok = false;
         break;
       }
-      uint8_t* sw = ring + s * STAGE;
-      const int k0 = (kb0 + (it + rot < nkb ? it + rot : it + rot - nkb)) * BK;
-      if (elect_one()) {
-        if (CG == 2) {
-          const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), lead_rank);   // both CTAs' bytes count on the leader's barrier
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * STAGE);
-          tma_load_2d_pair(sw, &tmW0, fb, k0, nb.col0);
-          if (GATED) tma_load_2d_pair(sw + kFewWBytes / 2, &tmW1, fb, k0, nb.col0);
-          tma_load_2d_pair(sw + kFewWBytes, &tmX, fb, k0, tok0 + half * (NT / 2));
-        } else {
-          mbar_expect_tx(&full_bar[s], STAGE);
-          tma_load_2d(sw, &tmW0, &full_bar[s], k0, nb.col0);
-          if (GATED) tma_load_2d(sw + kFewWBytes / 2, &tmW1, &full_bar[s], k0, nb.col0);
-          tma_load_2d(sw + kFewWBytes, &tmX, &full_bar[s], nb.a_k0 + k0, tok0);
-        }
-      }
+      if (elect_one()) load(s, it, it >= early, true);
       __syncwarp();
     }
     if (ok && CG == 2) {

@@ -89,6 +89,8 @@ typedef struct nfk_gemm_params {
   const void* bias2;    // gated epilogue: [N] bf16 bias of the up half (`bias` is the gate half's), null = none
   int rows_kernel;      // the kernel for few rows (gemm_few_rows.cuh): 0 = by rule; 1 = it (`cta_group` 1 / 2 and `split_k`
                         // as given, 0 = choose); 2 = the tile kernel
+  int weights_ready;    // B and B2 were complete before the launch that precedes this one on the stream (weights of a model
+                        // that is loaded): they may be fetched while that one still runs
 } nfk_gemm_params;
 
 int nfk_gemm_bf16(const nfk_gemm_params* p, cudaStream_t stream);

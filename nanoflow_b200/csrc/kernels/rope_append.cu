@@ -94,6 +94,8 @@ rope_append_kernel(nfk_rope_append_params p) {
 // (token, head, 16-byte pair) units are spread flat over the grid and the kernel is a pure copy.
 __global__ void __launch_bounds__(256)
 rope_append_table_kernel(nfk_rope_append_params p) {
+  let_next_start();
+  await_previous();
   const int hd = p.head_dim;
   const int half = hd >> 1;
   const int lph = hd >> 4;
@@ -156,6 +158,8 @@ rope_append_table_kernel(nfk_rope_append_params p) {
 
 __global__ void __launch_bounds__(256)
 rope_table_kernel(nfk_rope_table_params p) {
+  let_next_start();
+  await_previous();
   const long long total = static_cast<long long>(p.T) * p.half;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += 256ll * gridDim.x) {
     const int t = static_cast<int>(i / p.half);
@@ -179,8 +183,9 @@ extern "C" int nfk_rope_table(const nfk_rope_table_params* p, cudaStream_t strea
   const long long total = static_cast<long long>(p->T) * p->half;
   long long blocks = (total + 255) / 256;
   if (blocks > device_sm_count() * 8) blocks = device_sm_count() * 8;
-  rope_table_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(*p);
-  return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA;
+  if (launch_early(rope_table_kernel, static_cast<int>(blocks), 256, 0, stream, 1, *p) == cudaSuccess) return NF_OK;
+  (void)cudaGetLastError();
+  return NF_ERR_CUDA;
 }
 
 extern "C" int nfk_rope_append(const nfk_rope_append_params* p, cudaStream_t stream) {
@@ -201,8 +206,9 @@ extern "C" int nfk_rope_append(const nfk_rope_append_params* p, cudaStream_t str
     const long long total = static_cast<long long>(p->T) * units;
     long long nb = (total + 255) / 256;
     if (nb > device_sm_count() * 16) nb = device_sm_count() * 16;
-    rope_append_table_kernel<<<static_cast<int>(nb), 256, 0, stream>>>(*p);
-    return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA;
+    if (launch_early(rope_append_table_kernel, static_cast<int>(nb), 256, 0, stream, 1, *p) == cudaSuccess) return NF_OK;
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
   }
   int threads = units < 64 ? 64 : (units < 128 ? 128 : 256);
   int blocks = p->T < device_sm_count() * 8 ? p->T : device_sm_count() * 8;

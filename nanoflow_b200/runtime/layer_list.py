@@ -509,7 +509,7 @@ class LayerListEngine(Engine):
         if d32 is not None:
             p.D32, p.ld32, p.f32_col0 = _ptr(d32), d32.stride(0), f32_col0
         p.groups, p.group_k = groups, group_k
-        p.status = _ptr(self.bufs.status)
+        p.status, p.weights_ready = _ptr(self.bufs.status), 1
         if self.gemm_ws is not None:
             p.workspace, p.workspace_bytes = _ptr(self.gemm_ws), self.gemm_ws.numel() * 4
         shape = self.eng.gemm_shapes.get(key)

@@ -246,7 +246,7 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
                 p.split_k, p.stream_k = 1, 2      # whole tiles in row order (the launcher enforces it as well)
         p.num_ctas = budget.get("gemm", 0)
         p.smem_budget_kb = gemm_smem_budget_kb(eng, tp)
-        p.status = _ptr(st)
+        p.status, p.weights_ready = _ptr(st), 1
         if bufs.gemm_ws is not None:
             p.workspace = _ptr(bufs.gemm_ws)
             p.workspace_bytes = bufs.gemm_ws.numel() * bufs.gemm_ws.element_size()
@@ -564,6 +564,7 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
     lp.lda, lp.ldb, lp.ldd, lp.ldc = bufs.sample_hn.stride(0), w.lm_head.stride(0), bufs.logits.stride(0), 0
     lp.beta, lp.M, lp.N, lp.K = 0.0, 0, w.lm_head.shape[0], hidden
     lp.epilogue, lp.tile_n, lp.num_ctas, lp.status = 0, eng.gemm_tile_n.get("lm_head", 0), 0, _ptr(st)
+    lp.weights_ready = 1
     if bufs.gemm_ws is not None:
         lp.workspace = _ptr(bufs.gemm_ws)
         lp.workspace_bytes = bufs.gemm_ws.numel() * bufs.gemm_ws.element_size()
