@@ -4,10 +4,10 @@
 // item's query rows r = token * group + head fill one 128-row MMA tile, and the item walks its keys in
 // tiles of 64 tokens. Three roles share a 192-thread CTA and meet only through mbarriers:
 //
-//   warp 4, one thread   loads: TMA copies (no multicast) of the Q rows and of whole K / V pages from the
+//   warp 4               loads: TMA copies (no multicast) of the Q rows and of whole K / V pages from the
 //                        paged pool into 128B-swizzled shared memory, two K and two V tiles in flight;
 //                        the page ids of the next tile are fetched while the current one is issued
-//   warp 5, one thread   tcgen05.mma: S(t+1) = Q K(t+1)^T is issued before P(t) is waited for, into the
+//   warp 5               tcgen05.mma: S(t+1) = Q K(t+1)^T is issued before P(t) is waited for, into the
 //                        other of two S accumulators in TMEM, so the tensor cores work on the next tile's
 //                        scores while the softmax warps are still busy with this tile; then
 //                        O += P(t) V(t) with P read from TMEM (A operand in tensor memory) and V read
@@ -144,9 +144,11 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BAR_OFF);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // uniform, so that the roles' counters and the operands of TMA and tcgen05 instructions stay in uniform registers
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if ((sb & 1023u) != 0u) {
     // the operand layouts assume a 1024-aligned base; report instead of computing garbage
+    await_previous();
     if (threadIdx.x == 0) report_status(p.status, NF_ST_BAD_INDEX);
     return;
   }
@@ -173,28 +175,31 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  let_next_start();
+  await_previous();
 
   const int group = p.q_heads / p.kv_heads;
   const long long total = static_cast<long long>(p.num_items) * p.kv_heads;
   const int rounds = static_cast<int>((total + gridDim.x - 1) / gridDim.x);
   auto fail = [&](unsigned int code) {
-    report_status(p.status, code);
+    if (lane == 0) report_status(p.status, code);
     *abort_flag = 1;
   };
+  // for a whole warp: the same answer in all lanes
+  auto passed = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
+  auto aborted = [&]() { return __any_sync(0xffffffffu, *abort_flag != 0) != 0; };
 
   if (warp == 4) {
-    // ------------------------------------------------------------------ loads
-    if (lane == 0) {
-      uint32_t g = 0, n_item = 0;          // tiles / items issued so far by this CTA
-      uint32_t issued[NUM_BARS];           // per "full" barrier: loads issued on it
-      for (int b = 0; b < NUM_BARS; ++b) issued[b] = 0;
-      bool ok = true;
-      for (int k = 0; k < rounds && ok; ++k) {
-        const long long w = work_index(k, total);
-        if (w < 0) continue;
-        const Item it = read_item<EXT>(p, w);
-        if (!it.valid) continue;
-        if (!mbar_wait(&bars[Q_EMPTY], (n_item & 1) ^ 1) || *abort_flag) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); break; }
+    // ------------------------------------------------------------------ loads (the warp walks, an elected lane issues)
+    uint32_t g = 0, n_item = 0, k_issued = 0, v_issued = 0;     // tiles / items issued so far by this CTA
+    bool ok = true;
+    for (int k = 0; k < rounds && ok; ++k) {
+      const long long w = work_index(k, total);
+      if (w < 0) continue;
+      const Item it = read_item<EXT>(p, w);
+      if (!it.valid) continue;
+      if (!passed(&bars[Q_EMPTY], (n_item & 1) ^ 1) || aborted()) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); break; }
+      if (elect_one()) {
         if (EXT && p.q_rows > 0) {
           // one head per query row tile: 128 rows in two boxes; rows past the item's tokens are other tokens' (or
           // zero past the buffer) and are never stored
@@ -203,139 +208,145 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           for (int h = 0; h < NH; ++h)
             tma_load_2d(smem + Q_OFF + h * 16384, &tmQ, &bars[Q_FULL], it.kvh * HD + h * 64, it.tok0);
         } else {
-        mbar_expect_tx(&bars[Q_FULL], static_cast<uint32_t>(it.ntok * group) * HD * 2);
-        for (int tl = 0; tl < it.ntok; ++tl) {
-          // row of the [T * heads per row][HD] view
-          const int grow = (it.tok0 + tl) * (EXT && p.ld_q > 0 ? p.ld_q / HD : p.q_heads) + it.kvh * group;
+          mbar_expect_tx(&bars[Q_FULL], static_cast<uint32_t>(it.ntok * group) * HD * 2);
+          for (int tl = 0; tl < it.ntok; ++tl) {
+            // row of the [T * heads per row][HD] view
+            const int grow = (it.tok0 + tl) * (EXT && p.ld_q > 0 ? p.ld_q / HD : p.q_heads) + it.kvh * group;
 #pragma unroll
-          for (int h = 0; h < NH; ++h)
-            tma_load_2d(smem + Q_OFF + h * 16384 + tl * group * 128, &tmQ, &bars[Q_FULL], h * 64, grow);
-        }
-        }
-        ++issued[Q_FULL];
-        ++n_item;
-        int pages[4];
-        auto fetch_pages = [&](int t) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            int pslot = (it.t_first + t) * (kTile / kPage) + j - it.pg_first;
-            // past the sequence, or given back since nobody sees it: a valid page, masked by position
-            if (pslot < 0 || pslot >= it.np) pslot = 0;
-            int page = p.kv_indices[it.pg0 + pslot];
-            if (page < 0 || page >= p.num_pages) {
-              report_status(p.status, NF_ST_BAD_INDEX);
-              page = 0;
-            }
-            pages[j] = page;
+            for (int h = 0; h < NH; ++h)
+              tma_load_2d(smem + Q_OFF + h * 16384 + tl * group * 128, &tmQ, &bars[Q_FULL], h * 64, grow);
           }
-        };
-        fetch_pages(0);
-        for (int t = 0; t < it.n_tiles; ++t, ++g) {
-          const int s = g & 1;
-          const uint32_t ph = ((g >> 1) & 1) ^ 1;
-          int cur[4] = {pages[0], pages[1], pages[2], pages[3]};
-          if (t + 1 < it.n_tiles) fetch_pages(t + 1);     // in flight while this tile's copies are issued
-          if (!mbar_wait(&bars[K_EMPTY0 + s], ph) || *abort_flag) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); ok = false; break; }
-          mbar_expect_tx(&bars[K_FULL0 + s], kStageBytes);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            // row of the [pages*2*kv_heads*16][128] view, or row and column of the plain [rows][kv_ld] one
-            const bool plain = EXT && p.kv_ld > 0;
-            const int row0 = plain ? cur[j] * kPage : ((cur[j] * 2) * p.kv_heads + it.kvh) * kPage;
-            const int col0 = plain ? p.k_col + it.kvh * HD : 0;
-            uint8_t* dst = smem + K_OFF + s * kStageBytes + j * 2048;
-#pragma unroll
-            for (int h = 0; h < NH; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &bars[K_FULL0 + s], col0 + h * 64, row0);
-          }
-          ++issued[K_FULL0 + s];
-          if (!mbar_wait(&bars[V_EMPTY0 + s], ph) || *abort_flag) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); ok = false; break; }
-          mbar_expect_tx(&bars[V_FULL0 + s], kStageBytes);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const bool plain = EXT && p.kv_ld > 0;
-            const int row0 = plain ? cur[j] * kPage : ((cur[j] * 2 + 1) * p.kv_heads + it.kvh) * kPage;
-            const int col0 = plain ? p.v_col + it.kvh * HD : 0;
-            uint8_t* dst = smem + V_OFF + s * kStageBytes + j * 2048;
-#pragma unroll
-            for (int h = 0; h < NH; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &bars[V_FULL0 + s], col0 + h * 64, row0);
-          }
-          ++issued[V_FULL0 + s];
         }
       }
-      // copies still in flight must have landed before the CTA gives its shared memory back
-      const int fulls[5] = {Q_FULL, K_FULL0, K_FULL1, V_FULL0, V_FULL1};
-      for (int i = 0; i < 5; ++i) {
-        const int b = fulls[i];
-        if (issued[b] > 0) (void)mbar_wait(&bars[b], (issued[b] - 1) & 1);
+      __syncwarp();
+      ++n_item;
+      int pages[4];
+      auto fetch_pages = [&](int t) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          int pslot = (it.t_first + t) * (kTile / kPage) + j - it.pg_first;
+          // past the sequence, or given back since nobody sees it: a valid page, masked by position
+          if (pslot < 0 || pslot >= it.np) pslot = 0;
+          int page = p.kv_indices[it.pg0 + pslot];
+          if (page < 0 || page >= p.num_pages) {
+            report_status(p.status, NF_ST_BAD_INDEX);
+            page = 0;
+          }
+          pages[j] = page;
+        }
+      };
+      fetch_pages(0);
+      const bool plain = EXT && p.kv_ld > 0;
+      // one tile of keys (part 0) or values (1): rows of the [pages*2*kv_heads*16][128] view, or of the plain [rows][kv_ld] one
+      auto load_tile = [&](const int (&cur)[4], int part, int off, uint64_t* full) {
+        if (elect_one()) {
+          mbar_expect_tx(full, kStageBytes);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int row0 = plain ? cur[j] * kPage : ((cur[j] * 2 + part) * p.kv_heads + it.kvh) * kPage;
+            const int col0 = plain ? (part != 0 ? p.v_col : p.k_col) + it.kvh * HD : 0;
+#pragma unroll
+            for (int h = 0; h < NH; ++h) tma_load_2d(smem + off + j * 2048 + h * kHalfBytes, &tmKV, full, col0 + h * 64, row0);
+          }
+        }
+        __syncwarp();
+      };
+      for (int t = 0; t < it.n_tiles; ++t, ++g) {
+        const int s = g & 1;
+        const uint32_t ph = ((g >> 1) & 1) ^ 1;
+        const int cur[4] = {pages[0], pages[1], pages[2], pages[3]};
+        if (t + 1 < it.n_tiles) fetch_pages(t + 1);     // in flight while this tile's copies are issued
+        if (!passed(&bars[K_EMPTY0 + s], ph) || aborted()) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); ok = false; break; }
+        load_tile(cur, 0, K_OFF + s * kStageBytes, &bars[K_FULL0 + s]);
+        ++k_issued;
+        if (!passed(&bars[V_EMPTY0 + s], ph) || aborted()) { fail(NF_ST_TIMEOUT_SMEM_EMPTY); ok = false; break; }
+        load_tile(cur, 1, V_OFF + s * kStageBytes, &bars[V_FULL0 + s]);
+        ++v_issued;
       }
     }
+    // copies still in flight must have landed before the CTA gives its shared memory back
+    if (n_item > 0) (void)mbar_wait(&bars[Q_FULL], (n_item - 1) & 1);
+#pragma unroll
+    for (uint32_t s = 0; s < 2; ++s) {                   // tiles alternate between two stages
+      if (k_issued > s) (void)mbar_wait(&bars[K_FULL0 + s], (((k_issued + 1 - s) >> 1) - 1) & 1);
+      if (v_issued > s) (void)mbar_wait(&bars[V_FULL0 + s], (((v_issued + 1 - s) >> 1) - 1) & 1);
+    }
   } else if (warp == 5) {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc_bf16(128, kTile);
-      const uint32_t idesc_o = umma_idesc_bf16(128, HD) | kIdescBMnMajor;
-      uint32_t g = 0, n_item = 0;
-      // `pv_issued`: PV products issued so far by this CTA. The S accumulator that S(gt) goes into held P(gt-2),
-      // the A operand of PV(gt-2); products with different accumulators are not ordered against each other's
-      // operand reads, so the latest PV issued (gt-2 inside an item, gt-1 at its start) must have completed.
-      auto issue_s = [&](uint32_t gt, uint32_t pv_issued) -> bool {
-        const int s = gt & 1;
-        const uint32_t ph = (gt >> 1) & 1;
-        if (pv_issued > 0 && !mbar_wait(&bars[PV_DONE0 + ((pv_issued - 1) & 1)], ((pv_issued - 1) >> 1) & 1)) return false;
-        if (!mbar_wait(&bars[K_FULL0 + s], ph)) return false;
-        tc_fence_after();
-        const uint32_t kb = sb + K_OFF + s * kStageBytes;
+    // ------------------------------------------------------------------ MMA issue (the warp walks, an elected lane issues)
+    // With one thread in each of the two roles (`lane == 0`) the issue of a tile's twelve MMAs, not the MMAs, set the pace: 4096
+    // queries behind 4096 tokens, 32 heads, 497 -> 350 us (830 -> 1180 TFLOP/s); 16384 tokens 2382 -> 1798; 2 x 1000, 64 heads,
+    // 63.5 -> 43; 333 tokens 14.9 -> 10.
+    const uint32_t idesc_s = umma_idesc_bf16(128, kTile);
+    const uint32_t idesc_o = umma_idesc_bf16(128, HD) | kIdescBMnMajor;
+    const uint64_t q_desc = umma_desc_k_sw128(sb + Q_OFF), k_desc = umma_desc_k_sw128(sb + K_OFF);
+    const uint64_t v_desc = umma_desc_mn_sw128(sb + V_OFF, kHalfBytes, 1024);
+    uint32_t g = 0, n_item = 0;
+    // `pv_issued`: PV products issued so far by this CTA. The S accumulator that S(gt) goes into held P(gt-2),
+    // the A operand of PV(gt-2); products with different accumulators are not ordered against each other's
+    // operand reads, so the latest PV issued (gt-2 inside an item, gt-1 at its start) must have completed.
+    auto issue_s = [&](uint32_t gt, uint32_t pv_issued) -> bool {
+      const int s = gt & 1;
+      const uint32_t ph = (gt >> 1) & 1;
+      if (pv_issued > 0 && !passed(&bars[PV_DONE0 + ((pv_issued - 1) & 1)], ((pv_issued - 1) >> 1) & 1)) return false;
+      if (!passed(&bars[K_FULL0 + s], ph)) return false;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t kd = k_desc + static_cast<uint64_t>(s * (kStageBytes >> 4));
 #pragma unroll
         for (int h = 0; h < NH; ++h)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem + s * kTile, umma_desc_k_sw128(sb + Q_OFF + h * 16384 + k * 32),
-                         umma_desc_k_sw128(kb + h * kHalfBytes + k * 32), idesc_s, (h | k) ? 1u : 0u);
+            umma_bf16_ss(tmem + s * kTile, q_desc + ((h * 16384 + k * 32) >> 4), kd + ((h * kHalfBytes + k * 32) >> 4), idesc_s,
+                         (h | k) ? 1u : 0u);
         umma_commit(&bars[K_EMPTY0 + s]);
         umma_commit(&bars[S_FULL0 + s]);
-        return true;
-      };
-      bool ok = true;
-      for (int k = 0; k < rounds && ok; ++k) {
-        const long long w = work_index(k, total);
-        if (w < 0) continue;
-        const Item it = read_item<EXT>(p, w);
-        if (!it.valid) continue;
-        if (!mbar_wait(&bars[Q_FULL], n_item & 1) || *abort_flag) { fail(NF_ST_TIMEOUT_SMEM_FULL); break; }
-        if (!issue_s(g, g)) { fail(NF_ST_TIMEOUT_SMEM_FULL); break; }
-        for (int t = 0; t < it.n_tiles; ++t) {
-          const uint32_t gt = g + t;
-          if (t + 1 < it.n_tiles) {
-            if (!issue_s(gt + 1, gt)) { fail(NF_ST_TIMEOUT_SMEM_FULL); ok = false; break; }
-          } else {
-            umma_commit(&bars[Q_EMPTY]);     // the last S product of the item has been issued
-          }
-          // the previous item's O must have been read out before this item's first PV overwrites it
-          if (t == 0 && !mbar_wait(&bars[O_FREE], (n_item & 1) ^ 1)) { fail(NF_ST_TIMEOUT_TMEM_EMPTY); ok = false; break; }
-          const int s = gt & 1;
-          if (!mbar_wait(&bars[P_FULL0 + s], (gt >> 1) & 1) || !mbar_wait(&bars[V_FULL0 + s], (gt >> 1) & 1) || *abort_flag) {
-            fail(NF_ST_TIMEOUT_SMEM_FULL);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t vb = sb + V_OFF + s * kStageBytes;
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = true;
+    for (int k = 0; k < rounds && ok; ++k) {
+      const long long w = work_index(k, total);
+      if (w < 0) continue;
+      const Item it = read_item<EXT>(p, w);
+      if (!it.valid) continue;
+      if (!passed(&bars[Q_FULL], n_item & 1) || aborted()) { fail(NF_ST_TIMEOUT_SMEM_FULL); break; }
+      if (!issue_s(g, g)) { fail(NF_ST_TIMEOUT_SMEM_FULL); break; }
+      for (int t = 0; t < it.n_tiles; ++t) {
+        const uint32_t gt = g + t;
+        if (t + 1 < it.n_tiles) {
+          if (!issue_s(gt + 1, gt)) { fail(NF_ST_TIMEOUT_SMEM_FULL); ok = false; break; }
+        } else {
+          if (elect_one()) umma_commit(&bars[Q_EMPTY]);     // the last S product of the item has been issued
+          __syncwarp();
+        }
+        // the previous item's O must have been read out before this item's first PV overwrites it
+        if (t == 0 && !passed(&bars[O_FREE], (n_item & 1) ^ 1)) { fail(NF_ST_TIMEOUT_TMEM_EMPTY); ok = false; break; }
+        const int s = gt & 1;
+        if (!passed(&bars[P_FULL0 + s], (gt >> 1) & 1) || !passed(&bars[V_FULL0 + s], (gt >> 1) & 1) || aborted()) {
+          fail(NF_ST_TIMEOUT_SMEM_FULL);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t vd = v_desc + static_cast<uint64_t>(s * (kStageBytes >> 4));
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             umma_bf16_ts(tmem + 2 * kTile, tmem + s * kTile + k * 8,      // P(t): 16 tokens = 8 columns per step
-                         umma_desc_mn_sw128(vb + k * 2048, kHalfBytes, 1024), idesc_o, (t | k) ? 1u : 0u);
+                         vd + (k * 2048 >> 4), idesc_o, (t | k) ? 1u : 0u);
           if (EXT) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)                                   // the low parts of P(t)
-              umma_bf16_ts(tmem + 2 * kTile, tmem + s * kTile + 32 + k * 8,
-                           umma_desc_mn_sw128(vb + k * 2048, kHalfBytes, 1024), idesc_o, 1u);
+              umma_bf16_ts(tmem + 2 * kTile, tmem + s * kTile + 32 + k * 8, vd + (k * 2048 >> 4), idesc_o, 1u);
           }
           umma_commit(&bars[V_EMPTY0 + s]);
           umma_commit(&bars[PV_DONE0 + s]);
         }
-        g += it.n_tiles;
-        ++n_item;
+        __syncwarp();
       }
+      g += it.n_tiles;
+      ++n_item;
     }
   } else {
     // ------------------------------------------------------------------ softmax (one thread per query row)
@@ -412,10 +423,10 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             if (cbase + 32 + j < chunk_lo) r1[j] = 0xff800000u;
           }
         }
-        float mxp = -INFINITY;
+        float mq[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};       // four chains
 #pragma unroll
-        for (int j = 0; j < 32; ++j) mxp = fmaxf(mxp, fmaxf(__uint_as_float(r0[j]), __uint_as_float(r1[j])));
-        const float mx = mxp * scale;
+        for (int j = 0; j < 32; ++j) mq[j & 3] = fmaxf(mq[j & 3], fmaxf(__uint_as_float(r0[j]), __uint_as_float(r1[j])));
+        const float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3])) * scale;
         const bool grow = mx > m_ref + kRescaleGap || (m_ref == -INFINITY && mx > -INFINITY);
         if (t == 0) {
           m_ref = mx;
@@ -529,8 +540,11 @@ int launch_ws(const nfk_attn_params& p, const CUtensorMap& tmQ, const CUtensorMa
   const long long total = static_cast<long long>(p.num_items) * p.kv_heads;
   long long ctas = p.num_ctas > 0 ? p.num_ctas : 2LL * device_sm_count();   // two resident CTAs per SM
   if (ctas > total) ctas = total;
-  attn_prefill_ws_kernel<HD, EXT, CAP, DIST><<<static_cast<int>(ctas), kThreads, bytes, stream>>>(tmQ, tmKV, p);
-  return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA;
+  if (launch_early(attn_prefill_ws_kernel<HD, EXT, CAP, DIST>, static_cast<int>(ctas), kThreads, bytes, stream, 1, tmQ, tmKV, p) ==
+      cudaSuccess)
+    return NF_OK;
+  (void)cudaGetLastError();
+  return NF_ERR_CUDA;
 }
 
 }  // namespace
