@@ -184,6 +184,8 @@ template <class T, int NV, bool CONV, bool DEEP>
 __global__ void __launch_bounds__(kRnThreads)
 residual_norm_kernel(nfk_residual_norm_params p) {
   __shared__ float red[kRnThreads / 32];
+  let_next_start();
+  await_previous();
   const int nvec = (p.cols + 3) >> 2;
   for (int row = blockIdx.x; row < p.rows; row += gridDim.x) {
     int src_row = row;
@@ -324,22 +326,118 @@ residual_norm_kernel(nfk_residual_norm_params p) {
   }
 }
 
+// The plain step of most layers, x <- x + norm_in(y); h = norm_out(x), both norms of one kind and rows that the CTA's threads
+// cover exactly: the general kernel spends some 9400 instructions of a warp on a row of 4096 (choices, bounds, addresses of
+// the forms that it also knows), and issuing those is what bounds it. The same sums in the same order. x is requested with y,
+// weights ahead of the sums they follow. 1840 x 4096 bf16, layer norms: 30.9 -> 20.6 us (4.4 TB/s); RMS: 28.7 -> 18.4; 96
+// rows: 7.9 -> 4.5.
+template <int NV, bool LAYER>
+__device__ __forceinline__ void plain_norm(float4 (&v)[NV], const float4 (&w)[NV], const float* b, float inv_n, float eps, float* red) {
+  if (LAYER) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    const float mean = cta_sum(s, red) * inv_n;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) { v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean; }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    ss += v[i].x * v[i].x; ss += v[i].y * v[i].y; ss += v[i].z * v[i].z; ss += v[i].w * v[i].w;
+  }
+  const float inv = rsqrtf(cta_sum(ss, red) * inv_n + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const float4 bb = b != nullptr ? load4(b + (threadIdx.x + i * kRnThreads) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i].x = v[i].x * inv * w[i].x + bb.x;
+    v[i].y = v[i].y * inv * w[i].y + bb.y;
+    v[i].z = v[i].z * inv * w[i].z + bb.z;
+    v[i].w = v[i].w * inv * w[i].w + bb.w;
+  }
+}
+
+template <class T, int NV, bool LAYER>
+__global__ void __launch_bounds__(kRnThreads, NV <= 4 ? 3 : 1)
+residual_norm_plain_kernel(nfk_residual_norm_params p) {
+  __shared__ float red[kRnThreads / 32];
+  let_next_start();
+  await_previous();
+  const float inv_n = 1.f / static_cast<float>(p.cols);
+  const int c0 = threadIdx.x * 4;
+  constexpr int kStep = kRnThreads * 4;
+  for (int row = blockIdx.x; row < p.rows; row += gridDim.x) {
+    const T* src = reinterpret_cast<const T*>(p.y) + static_cast<long long>(row) * p.ld_y + c0;
+    float* xr = p.x + static_cast<long long>(row) * p.ld_x + c0;
+    T* hr = reinterpret_cast<T*>(p.h) + static_cast<long long>(row) * p.ld_h + c0;
+    float4 v[NV], x[NV], w[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = load4(src + i * kStep);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) x[i] = load4(xr + i * kStep);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) w[i] = load4(p.in_w + c0 + i * kStep);
+    plain_norm<NV, LAYER>(v, w, p.in_b, inv_n, p.eps, red);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) w[i] = load4(p.out_w + c0 + i * kStep);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      v[i].x += x[i].x; v[i].y += x[i].y; v[i].z += x[i].z; v[i].w += x[i].w;
+      store4(xr + i * kStep, v[i]);
+    }
+    plain_norm<NV, LAYER>(v, w, p.out_b, inv_n, p.eps, red);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) store4(hr + i * kStep, v[i]);
+  }
+}
+
+inline int started(cudaError_t e) {
+  if (e == cudaSuccess) return NF_OK;
+  (void)cudaGetLastError();
+  return NF_ERR_CUDA;
+}
+
+// Whether a call is the plain step (see residual_norm_plain_kernel).
+inline bool plain_step(const nfk_residual_norm_params& p) {
+  return p.y && p.h && !p.table && !p.rows_idx && !p.y2 && !p.pair_w && !p.e_out && !p.add && !p.norm_sum &&
+         (p.src_scale == 0.f || p.src_scale == 1.f) && !p.conv_w && !p.pos_freq && !p.hist_w && !p.hist_out &&
+         p.in_kind == p.out_kind && (p.in_kind == NFK_NORM_RMS || p.in_kind == NFK_NORM_LAYER) &&
+         (p.cols == 4 * kRnThreads || p.cols == 8 * kRnThreads || p.cols == 16 * kRnThreads || p.cols == 32 * kRnThreads);
+}
+
+template <class T, int NV>
+int launch_plain(const nfk_residual_norm_params& p, cudaStream_t stream) {
+  const int cap = device_sm_count() * 16;
+  const int grid = p.rows < cap ? p.rows : cap;
+  auto* kernel = p.in_kind == NFK_NORM_LAYER ? residual_norm_plain_kernel<T, NV, true> : residual_norm_plain_kernel<T, NV, false>;
+  return started(launch_early(kernel, grid, kRnThreads, 0, stream, 1, p));
+}
+
 template <class T, bool CONV, bool DEEP>
 int launch_rn(const nfk_residual_norm_params& p, cudaStream_t stream) {
   const int nvec = (p.cols + 3) / 4, per = (nvec + kRnThreads - 1) / kRnThreads;
   const int cap = device_sm_count() * 16;
   const int grid = p.rows < cap ? p.rows : cap;
-  if (per <= 1) residual_norm_kernel<T, 1, CONV, DEEP><<<grid, kRnThreads, 0, stream>>>(p);
-  else if (per <= 2) residual_norm_kernel<T, 2, CONV, DEEP><<<grid, kRnThreads, 0, stream>>>(p);
-  else if (per <= 4) residual_norm_kernel<T, 4, CONV, DEEP><<<grid, kRnThreads, 0, stream>>>(p);
-  else if (per <= 8) residual_norm_kernel<T, 8, CONV, DEEP><<<grid, kRnThreads, 0, stream>>>(p);
-  else if (per <= 16) residual_norm_kernel<T, 16, CONV, DEEP><<<grid, kRnThreads, 0, stream>>>(p);
+  cudaError_t e;
+  if (per <= 1) e = launch_early(residual_norm_kernel<T, 1, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 2) e = launch_early(residual_norm_kernel<T, 2, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 4) e = launch_early(residual_norm_kernel<T, 4, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 8) e = launch_early(residual_norm_kernel<T, 8, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 16) e = launch_early(residual_norm_kernel<T, 16, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
   else return NF_ERR_UNSUPPORTED;
-  return cudaGetLastError() == cudaSuccess ? NF_OK : NF_ERR_CUDA;
+  return started(e);
 }
 
 template <class T>
 int launch_rn_form(const nfk_residual_norm_params& p, cudaStream_t stream) {
+  if (plain_step(p)) {
+    switch (p.cols / (4 * kRnThreads)) {
+      case 1: return launch_plain<T, 1>(p, stream);
+      case 2: return launch_plain<T, 2>(p, stream);
+      case 4: return launch_plain<T, 4>(p, stream);
+      default: return launch_plain<T, 8>(p, stream);
+    }
+  }
   const bool deep = p.pos_freq != nullptr || p.hist_w != nullptr || p.hist_out != nullptr;
   if (p.conv_w != nullptr && p.conv_rows > 0) return deep ? launch_rn<T, true, true>(p, stream) : launch_rn<T, true, false>(p, stream);
   return deep ? launch_rn<T, false, true>(p, stream) : launch_rn<T, false, false>(p, stream);
