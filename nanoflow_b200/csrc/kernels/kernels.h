@@ -91,6 +91,8 @@ typedef struct nfk_gemm_params {
                         // as given, 0 = choose); 2 = the tile kernel
   int weights_ready;    // B and B2 were complete before the launch that precedes this one on the stream (weights of a model
                         // that is loaded): they may be fetched while that one still runs
+  int tuned_rows;       // rows that the pinned shape was measured at: a call with another number of 256-row groups leaves
+                        // the shape to the cost model (0 = the shape holds for every M)
 } nfk_gemm_params;
 
 int nfk_gemm_bf16(const nfk_gemm_params* p, cudaStream_t stream);

@@ -45,7 +45,7 @@ class GemmParams(Structure):
                 ("D32", c_void_p), ("ld32", c_longlong), ("f32_col0", c_int), ("act", c_int),
                 ("groups", c_int), ("group_k", c_int), ("lin_act", c_int),
                 ("act_limit", c_float), ("act_alpha", c_float), ("act_shift", c_float), ("bias2", c_void_p),
-                ("rows_kernel", c_int), ("weights_ready", c_int)]
+                ("rows_kernel", c_int), ("weights_ready", c_int), ("tuned_rows", c_int)]
 
 
 class RopeAppendParams(Structure):

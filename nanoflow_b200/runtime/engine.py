@@ -230,7 +230,7 @@ class Engine:
                         bias=bias, num_ctas=budget, workspace=b.gemm_ws,
                         smem_budget_kb=gemm_smem_budget_kb(e, w.tp))
                 r = done[(key, M)]
-                e.gemm_shapes[name] = dict(r["best"])
+                e.gemm_shapes[name] = dict(r["best"], rows=M)
                 self.gemm_tuning[name] = dict(M=M, best=r["best"], us=r["us"], auto_us=r["auto_us"])
         torch.cuda.synchronize(self.device)
         for t in (b.h, b.attn_out, b.act, b.qkv, b.x[0], b.x[1], b.attn_full):

@@ -242,6 +242,7 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
             # measured at start-up (ops/autotune.py)
             p.tile_m, p.tile_n, p.cta_group = shape["tile_m"], shape["tile_n"], shape["cta_group"]
             p.split_k, p.stream_k = shape["split_k"], shape["stream_k"]
+            p.tuned_rows = shape.get("rows", 0)
             if gate is not None:
                 p.split_k, p.stream_k = 1, 2      # whole tiles in row order (the launcher enforces it as well)
         p.num_ctas = budget.get("gemm", 0)

@@ -1,0 +1,32 @@
+"""Which shape a GEMM call takes when the caller pins one that was measured at another number of rows."""
+from ctypes import byref, c_void_p
+
+import pytest
+
+from nanoflow_b200 import ops
+
+
+def _plan(M, N, K, **f):
+    p, out = ops.GemmParams(), ops.GemmPlan()
+    p.M, p.N, p.K, p.workspace, p.workspace_bytes = M, N, K, c_void_p(256), 160 << 20
+    for k, v in f.items():
+        setattr(p, k, v)
+    assert ops.lib().nfk_gemm_describe(byref(p), byref(out)) == 0
+    return {n: getattr(out, n) for n, _ in ops.GemmPlan._fields_}
+
+
+@pytest.mark.parametrize("tuned,M,holds", [(0, 48, True), (2048, 2048, True), (2048, 1793, True), (2048, 1792, False), (2048, 48, False),
+                                           (256, 256, True), (256, 1, True), (256, 257, False), (100, 129, True)])
+def test_a_tuned_shape_holds_for_its_own_number_of_row_groups(tuned, M, holds):
+    pin = dict(tile_m=1, tile_n=192, cta_group=1, split_k=1, stream_k=2)
+    got = _plan(M, 10240, 8192, tuned_rows=tuned, **pin)
+    assert got == (_plan(M, 10240, 8192, **pin) if holds else _plan(M, 10240, 8192))
+
+
+@pytest.mark.parametrize("swiglu", [0, 1])
+@pytest.mark.parametrize("M", [1, 64, 128, 129, 255, 256, 257, 333, 512, 513, 700, 1024, 2048, 4096, 16384])
+@pytest.mark.parametrize("N,K", [(8, 64), (640, 512), (4096, 4096), (14336, 4096), (8192, 28672), (128256, 4096)])
+def test_the_model_chooses_what_is_built(M, N, K, swiglu):
+    pl = _plan(M, N, K, epilogue=swiglu)
+    assert pl["stages"] >= 2 and pl["tile_m"] * pl["tile_n"] <= 512 and pl["smem_bytes"] <= 227 * 1024
+    assert not (pl["cta_group"] == 2 and (M <= 128 or pl["tile_m"] != 1)) and not (swiglu and pl["split_k"] != 1)
