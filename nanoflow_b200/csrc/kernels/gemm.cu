@@ -1308,7 +1308,7 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
 // shared-memory budget, gated input, reduce-scatter) stay with it, and so do a norm of rows that are not contiguous and a
 // caller without a workspace, who gets one sum in the order of k.
 bool few_rows_takes(const nfk_gemm_params& g) {
-  if (g.rows_kernel == 2 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
+  if (g.rows_kernel == 2 || g.keep_order != 0 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
   if (g.num_ctas > 0 || g.smem_budget_kb > 0 || g.stream_k != 0) return false;
   if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
   if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
@@ -1341,21 +1341,35 @@ int few_rows(const nfk_gemm_params& g, cudaStream_t stream) {
 // K 4096 to 28672, two of them gated) at 15 numbers of rows from 100 to 2000: the shape it takes is 1.2 % slower than the
 // fastest one on average; with the constants before, 6 % and up to 80 % (333 x 32000 x 8192: 284 -> 158 us,
 // 512 x 14336 x 2 x 4096: 179 -> 119, 192 x 10240 x 8192: 57 -> 40).
+//
+// The earlier constants stay for calls with keep_order: a recurrent layer carries every change of rounding into its state
+// and on to the next tokens, so models with one keep the order of sums that these shapes give (where K is cut).
 struct Shape {
   int bn, mt, split_k, cg;
   bool stream_k;
 };
+struct ShapeModel {
+  double mma, fill, least_single, least_pair;                 // TFLOP/s, GB/s of an SM; us per k-block at least
+  double uneven, single;                                      // factors: gated tiles of uneven width, single CTAs
+  double unit, per_col_single, per_col;                       // us per unit, and per accumulator column
+  double reduce, reduce_rate, fix, fix_rate, copy_rate;       // us and TB/s of the second passes; GB/s of a CTA's partial copies
+  double weight_rate;                                         // TB/s at which the weight arrives, 0 = no bound
+  double tail_gain;                                           // a stream-K tail has to be below this share of the best without
+};
+constexpr ShapeModel kModel{10.2, 115.0, 0.296, 0.273, 1.08, 1.05, 0.847, 0.0119, 0.00119, 5.15, 3.27, 2.52, 1.27, 218.0, 5.79, 1.0};
+constexpr ShapeModel kEarlierModel{11.0, 100.0, 0.0, 0.36, 1.0, 1.0, 2.0, 0.012, 0.003, 3.0, 4.0, 3.0, 3.0, 150.0, 0.0, 0.88};
 Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
+  const ShapeModel& m = g.keep_order != 0 ? kEarlierModel : kModel;
   const int ctas = g.num_ctas > 0 ? g.num_ctas : sm_count();
   const int m_tiles = (g.M + BM - 1) / BM;
   const int num_kb = (g.K + BK - 1) / BK;
-  const double weight_us = static_cast<double>(g.N) * g.K * (swiglu ? 4.0 : 2.0) / 5.79e6;
+  const double weight_us = m.weight_rate > 0.0 ? static_cast<double>(g.N) * g.K * (swiglu ? 4.0 : 2.0) / (m.weight_rate * 1e6) : 0.0;
   Shape best{256, 1, 1, 1, false}, best_tail{256, 1, 1, 1, true};
   double best_cost = 1e30, best_tail_cost = 1e30;
   const int cg_lo = g.cta_group == 2 ? 2 : 1, cg_hi = g.cta_group == 1 ? 1 : 2;
   auto bounded = [&](double c) {
     const double w = weight_us + 0.25 * c;
-    return c > w ? c : w;
+    return m.weight_rate > 0.0 && w > c ? w : c;
   };
   for (int cg = cg_lo; cg <= cg_hi; ++cg) {
     for (int mt = 1; mt <= (cg == 2 ? 1 : 4); mt *= 2) {
@@ -1372,17 +1386,17 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
         const int tiles = m_groups * n_blocks;
         const int mt_eff = m_tiles < mt ? m_tiles : mt;
         // per k-block and SM (a CTA of a pair stages only half of the weight tile)
-        const double t_mma = 2.0 * BM * mt_eff * bn * BK / 10.2e6;
-        const double t_fill = (mt_eff * 16384.0 + bn * 128.0 / cg) / 115.0e3;
+        const double t_mma = 2.0 * BM * mt_eff * bn * BK / (m.mma * 1e6);
+        const double t_fill = (mt_eff * 16384.0 + bn * 128.0 / cg) / (m.fill * 1e3);
         double t_kb = t_mma > t_fill ? t_mma : t_fill;
-        const double t_least = cg == 2 ? 0.273 : 0.296;
+        const double t_least = cg == 2 ? m.least_pair : m.least_single;
         if (t_kb < t_least) t_kb = t_least;
-        if (swiglu && bn % 64 != 0) t_kb *= 1.08;
-        if (cg == 1) t_kb *= 1.05;
+        if (swiglu && bn % 64 != 0) t_kb *= m.uneven;
+        if (cg == 1) t_kb *= m.single;
         // per unit: prologue + epilogue; the epilogue hides under the next main loop only when TMEM
         // holds two accumulator sets
         const bool single_acc = mt * bn * 2 > 512;
-        const double unit_fixed = 0.847 + (single_acc ? 0.0119 : 0.00119) * mt_eff * bn;
+        const double unit_fixed = m.unit + (single_acc ? m.per_col_single : m.per_col) * mt_eff * bn;
         const int workers = ctas / cg > 0 ? ctas / cg : 1;
         const int max_sk = (swiglu || g.workspace == nullptr || g.epilogue == NFK_EPI_REDUCE_SCATTER) ? 1 : 8;
         for (int sk = 1; sk <= max_sk; ++sk) {
@@ -1391,7 +1405,7 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
           const int waves = (units + workers - 1) / workers;
           const int kb_per = (num_kb + sk - 1) / sk;
           double cost = waves * (kb_per * t_kb + unit_fixed);
-          if (sk > 1) cost += 5.15 + (sk + 1.0) * g.M * static_cast<double>(g.N) * 4.0 / 3.27e6;  // partial write + reduce
+          if (sk > 1) cost += m.reduce + (sk + 1.0) * g.M * static_cast<double>(g.N) * 4.0 / (m.reduce_rate * 1e6);  // partial write + reduce
           cost = bounded(cost);
           if (cost < best_cost) {
             best_cost = cost;
@@ -1406,8 +1420,8 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
               const double tile_bytes = mt_eff * BM * bn * 4.0;          // one fp32 copy of a CTA's tile rows
               const double pieces = static_cast<double>(num_kb) / pl.q + 1.0;
               // a worker's range may straddle two tiles
-              const double fix_us = 2.52 + pl.rest * cg * pieces * tile_bytes / 1.27e6;
-              const double tail = pl.q * t_kb + 2.0 * unit_fixed + tile_bytes / 218.0e3 + fix_us;
+              const double fix_us = m.fix + pl.rest * cg * pieces * tile_bytes / (m.fix_rate * 1e6);
+              const double tail = pl.q * t_kb + 2.0 * unit_fixed + tile_bytes / (m.copy_rate * 1e3) + fix_us;
               const double c2 = bounded((tiles / workers) * (kb_per * t_kb + unit_fixed) + tail);
               if (c2 < best_tail_cost) {
                 best_tail_cost = c2;
@@ -1420,7 +1434,7 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
     }
   }
   if (g.stream_k == 1 && best_tail_cost < 1e30) return best_tail;
-  return best_tail_cost < best_cost ? best_tail : best;
+  return best_tail_cost < m.tail_gain * best_cost ? best_tail : best;
 }
 
 // A shape measured at another number of rows (tuned_rows) says little about this call: it holds for calls with as many

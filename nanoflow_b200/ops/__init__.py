@@ -45,7 +45,8 @@ class GemmParams(Structure):
                 ("D32", c_void_p), ("ld32", c_longlong), ("f32_col0", c_int), ("act", c_int),
                 ("groups", c_int), ("group_k", c_int), ("lin_act", c_int),
                 ("act_limit", c_float), ("act_alpha", c_float), ("act_shift", c_float), ("bias2", c_void_p),
-                ("rows_kernel", c_int), ("weights_ready", c_int), ("tuned_rows", c_int)]
+                ("rows_kernel", c_int), ("weights_ready", c_int), ("tuned_rows", c_int),
+                ("keep_order", c_int)]
 
 
 class RopeAppendParams(Structure):
@@ -308,7 +309,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
          cta_group: int = 0, stream_k: int = 0, norm_w: Optional[torch.Tensor] = None,
          norm_out: Optional[torch.Tensor] = None, norm_eps: float = 1e-5,
          gate_flags: Optional[torch.Tensor] = None, gate_epoch: int = 0, gate_nranks: int = 1,
-         rows_kernel: int = 0) -> torch.Tensor:
+         rows_kernel: int = 0, keep_order: bool = False) -> torch.Tensor:
     """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) (+ beta * residual). Rows may be strided.
 
     With ``norm_w`` / ``norm_out`` the call also leaves ``norm_out = RMSNorm(out) * norm_w`` (from the
@@ -320,7 +321,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     ``gate_flags`` (int32 [ceil(M/128), 8]): rows of ``a`` are still arriving; the kernel waits, per
     128-row block, until words [block, 0:gate_nranks] have reached ``gate_epoch``.
 
-    ``rows_kernel`` 1 / 2 asks for / rules out the kernel for few rows (0 = the launcher's rule)."""
+    ``rows_kernel`` 1 / 2 asks for / rules out the kernel for few rows (0 = the launcher's rule).
+    ``keep_order``: shapes by the earlier rules (see kernels.h)."""
     _bf16(a, "a"); _bf16(w, "w")
     M, K = a.shape
     N, K2 = w.shape
@@ -352,7 +354,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     p.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     p.smem_budget_kb = smem_budget_kb
     p.cta_group = cta_group
-    p.rows_kernel = rows_kernel
+    p.rows_kernel, p.keep_order = rows_kernel, int(keep_order)
     p.stream_k = stream_k
     if norm_w is not None:
         _bf16(norm_w, "norm_w"); _bf16(norm_out, "norm_out")
@@ -400,7 +402,8 @@ def gemm_swiglu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *,
                 status: Optional[torch.Tensor] = None, tile_m: int = 0, split_k: int = 0,
                 workspace: Optional[torch.Tensor] = None, cta_group: int = 0,
                 stream_k: int = 0, smem_budget_kb: int = 0, gate_flags: Optional[torch.Tensor] = None,
-                gate_epoch: int = 0, gate_nranks: int = 1, rows_kernel: int = 0) -> torch.Tensor:
+                gate_epoch: int = 0, gate_nranks: int = 1, rows_kernel: int = 0,
+                keep_order: bool = False) -> torch.Tensor:
     """out[M,F] = silu(a @ w_gate^T) * (a @ w_up^T), gate and up products fused in one kernel.
     ``gate_flags``: as in :func:`gemm`."""
     _bf16(a, "a"); _bf16(w_gate, "w_gate"); _bf16(w_up, "w_up")
@@ -423,7 +426,7 @@ def gemm_swiglu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *,
     p.workspace = _p(workspace)
     p.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     p.cta_group = cta_group
-    p.rows_kernel = rows_kernel
+    p.rows_kernel, p.keep_order = rows_kernel, int(keep_order)
     p.stream_k = stream_k
     p.smem_budget_kb = smem_budget_kb
     _set_gate(p, gate_flags, gate_epoch, gate_nranks, M)

@@ -70,7 +70,7 @@ def candidates(M: int, N: int, K: int, swiglu: bool) -> List[Dict[str, int]]:
 def tune_gemm(a: torch.Tensor, weights: Sequence[torch.Tensor], out: torch.Tensor, *,
               weights_up: Optional[Sequence[torch.Tensor]] = None, residual: Optional[torch.Tensor] = None,
               bias: Optional[torch.Tensor] = None, num_ctas: int = 0, workspace: Optional[torch.Tensor] = None,
-              smem_budget_kb: int = 0, iters: int = 4, passes: int = 2) -> Dict[str, object]:
+              smem_budget_kb: int = 0, iters: int = 4, passes: int = 2, keep_order: bool = False) -> Dict[str, object]:
     """Time every candidate on ``a @ weights[i]^T`` (cycling through ``weights``) and return
     ``{"best": kwargs, "us": best time, "auto_us": time of the cost model's own choice, "table": [...]}``.
     Candidates the launcher rejects (shape not built, workspace too small) are skipped."""
@@ -86,10 +86,10 @@ def tune_gemm(a: torch.Tensor, weights: Sequence[torch.Tensor], out: torch.Tenso
         if swiglu:
             gemm_swiglu(a, w, weights_up[i % len(weights)], out=out, num_ctas=num_ctas, workspace=workspace,
                         smem_budget_kb=smem_budget_kb, tile_m=c["tile_m"], tile_n=c["tile_n"],
-                        cta_group=c["cta_group"], stream_k=c["stream_k"])
+                        cta_group=c["cta_group"], stream_k=c["stream_k"], keep_order=keep_order)
         else:
             gemm(a, w, out=out, residual=residual, bias=bias, num_ctas=num_ctas, workspace=workspace,
-                 smem_budget_kb=smem_budget_kb, **c)
+                 smem_budget_kb=smem_budget_kb, keep_order=keep_order, **c)
 
     for _ in range(passes):
         for ci, c in enumerate(cands):

@@ -509,14 +509,13 @@ class LayerListEngine(Engine):
         if d32 is not None:
             p.D32, p.ld32, p.f32_col0 = _ptr(d32), d32.stride(0), f32_col0
         p.groups, p.group_k = groups, group_k
-        p.status, p.weights_ready = _ptr(self.bufs.status), 1
+        p.status, p.weights_ready, p.keep_order = _ptr(self.bufs.status), 1, 1
         if self.gemm_ws is not None:
             p.workspace, p.workspace_bytes = _ptr(self.gemm_ws), self.gemm_ws.numel() * 4
         shape = self.eng.gemm_shapes.get(key)
         if shape is not None:
             p.tile_m, p.tile_n, p.cta_group = shape["tile_m"], shape["tile_n"], shape["cta_group"]
             p.split_k, p.stream_k = shape["split_k"], shape["stream_k"]
-            p.tuned_rows = shape.get("rows", 0)
         self._op(name, p, dyn=[("M", rows)], kernel=self.gemm_kernel, layer=layer)
 
     # ---- mixers: read self.h, leave their output projection in self.y ---------------------------------
@@ -866,9 +865,10 @@ class LayerListEngine(Engine):
                 dst = self.y if out is None else out[:T * n].view(T, n)
                 sig = (key, n, wt.shape[1], up is not None)
                 if sig not in done:
-                    done[sig] = autotune.tune_gemm(a, [wt], dst, weights_up=None if up is None else [up], workspace=self.gemm_ws)
+                    done[sig] = autotune.tune_gemm(a, [wt], dst, weights_up=None if up is None else [up], workspace=self.gemm_ws,
+                                                    keep_order=True)
                 res = done[sig]
-                self.eng.gemm_shapes[name] = dict(res["best"], rows=T)
+                self.eng.gemm_shapes[name] = dict(res["best"])
                 self.gemm_tuning[name] = dict(M=T, best=res["best"], us=res["us"], auto_us=res["auto_us"])
         torch.cuda.synchronize(self.device)
         for t in (self.h, self.y, *self.flat.values()):
