@@ -15,8 +15,8 @@
 // share a 256-row tile (tcgen05.mma.cta_group::2) and each stages half of the weight tile. A cost
 // model picks the shape; engines time the candidates on their own shapes (ops/autotune.py).
 //
-// Roles inside one 192-thread CTA: warp 0 lane 0 = TMA producer, warp 1 = TMEM owner and (lane 0)
-// MMA issuer, warps 2..5 = epilogue (TMEM -> registers -> global). Two TMEM accumulators are
+// Roles inside one 192-thread CTA: warp 0 = TMA producer, warp 1 = TMEM owner and MMA issuer (an elected
+// lane of each issues), warps 2..5 = epilogue (TMEM -> registers -> global). Two TMEM accumulators are
 // ping-ponged so the epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Takes the place of the reference's CUTLASS Sm80 device::Gemm wrapper
