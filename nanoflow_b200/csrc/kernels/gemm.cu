@@ -1442,10 +1442,19 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
 // 48 x 10240 x 8192, where the weight takes 26.
 nfk_gemm_params with_own_shape(const nfk_gemm_params& g) {
   nfk_gemm_params p = g;
-  if (g.tuned_rows > 0 && (g.M + 255) / 256 != (g.tuned_rows + 255) / 256)
-    p.tile_m = p.tile_n = p.cta_group = p.split_k = p.stream_k = 0;
-  return p;
+  if (g.tuned_rows <= 0) return p;
+  p.tile_m = p.tile_n = p.cta_group = p.split_k = p.stream_k = 0;
+  if ((g.M + 255) / 256 != (g.tuned_rows + 255) / 256) return p;
+  if (g.keep_order != 0) {
+    const Shape own = choose_shape(p, g.epilogue == NFK_EPI_SWIGLU);
+    if (own.split_k > 1 || own.stream_k || g.split_k > 1 || g.stream_k == 1) return p;
+  }
+  return g;
 }
+//
+// With keep_order a stopwatch must not decide where K is cut: a pick changes with the clock of the day, and the order of sums
+// with it. Shapes that leave K whole all add up in the order of k, so a tuned one of them takes the place of a whole-K shape of
+// the cost model; where the model cuts K for this M, or the tuned shape does, the model's shape stands.
 
 // Shape of this call: the cost model's, or the caller's pinned one, checked against what is built.
 int resolve_shape(const nfk_gemm_params& gp, bool swiglu, bool rs, Shape& s) {

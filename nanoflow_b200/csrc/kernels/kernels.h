@@ -93,8 +93,9 @@ typedef struct nfk_gemm_params {
                         // that is loaded): they may be fetched while that one still runs
   int tuned_rows;       // rows that the pinned shape was measured at: a call with another number of 256-row groups leaves
                         // the shape to the cost model (0 = the shape holds for every M)
-  int keep_order;       // 1 = shapes and kernel by the earlier rules, which keeps the order of sums (models whose recurrent
-                        // state carries a change of rounding on)
+  int keep_order;       // 1 = the order of sums follows from M, N and K alone, by the earlier rules: shapes and kernel by these,
+                        // a tuned shape (tuned_rows > 0) only where it and the rules' shape leave K whole (layer-list models:
+                        // a recurrent state carries a change of rounding on)
 } nfk_gemm_params;
 
 int nfk_gemm_bf16(const nfk_gemm_params* p, cudaStream_t stream);

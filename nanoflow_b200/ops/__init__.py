@@ -382,16 +382,17 @@ class GemmPlan(Structure):
 
 def gemm_plan(M: int, N: int, K: int, *, swiglu: bool = False, tile_n: int = 0, tile_m: int = 0, cta_group: int = 0,
               split_k: int = 0, stream_k: int = 0, num_ctas: int = 0, workspace_bytes: int = 0,
-              smem_budget_kb: int = 0) -> dict:
+              smem_budget_kb: int = 0, keep_order: bool = False, tuned_rows: int = 0) -> dict:
     """What ``gemm`` / ``gemm_swiglu`` would launch for these sizes (tile shape, tiles, workers, stream-K
     tail) without launching anything; works without a GPU. ``workspace_bytes`` > 0 stands for a caller
-    that passes a workspace of that size."""
+    that passes a workspace of that size, ``tuned_rows`` > 0 for a shape that was measured at that many rows."""
     p = GemmParams()
     p.M, p.N, p.K = M, N, K
     p.epilogue, p.tile_n, p.tile_m, p.cta_group = (1 if swiglu else 0), tile_n, tile_m, cta_group
     p.split_k, p.stream_k, p.num_ctas, p.smem_budget_kb = split_k, stream_k, num_ctas, smem_budget_kb
     if workspace_bytes > 0:
         p.workspace, p.workspace_bytes = c_void_p(256), workspace_bytes    # never dereferenced by the planner
+    p.keep_order, p.tuned_rows = int(keep_order), tuned_rows
     out = GemmPlan()
     _check(lib().nfk_gemm_describe(byref(p), byref(out)), "nfk_gemm_describe")
     return {f: getattr(out, f) for f, _ in GemmPlan._fields_}

@@ -19,7 +19,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
-from . import gemm, gemm_swiglu
+from . import gemm, gemm_plan, gemm_swiglu
 
 KEYS = ("tile_m", "tile_n", "cta_group", "split_k", "stream_k")
 AUTO: Dict[str, int] = dict(tile_m=0, tile_n=0, cta_group=0, split_k=0, stream_k=0)
@@ -67,17 +67,28 @@ def candidates(M: int, N: int, K: int, swiglu: bool) -> List[Dict[str, int]]:
     return out
 
 
+def same_order(cands: List[Dict[str, int]], M: int, N: int, K: int, swiglu: bool, workspace_bytes: int) -> List[Dict[str, int]]:
+    """Those of ``cands`` that add up in the order of the cost model's own shape: all that leave K whole if it does so, else
+    that shape alone (another tile shape cuts K elsewhere)."""
+    own = gemm_plan(M, N, K, swiglu=swiglu, workspace_bytes=workspace_bytes, keep_order=True)
+    whole = own["split_k"] == 1 and not own["stream_k"]
+    return [c for c in cands if c == AUTO or (whole and c["split_k"] == 1 and c["stream_k"] != 1)]
+
+
 def tune_gemm(a: torch.Tensor, weights: Sequence[torch.Tensor], out: torch.Tensor, *,
               weights_up: Optional[Sequence[torch.Tensor]] = None, residual: Optional[torch.Tensor] = None,
               bias: Optional[torch.Tensor] = None, num_ctas: int = 0, workspace: Optional[torch.Tensor] = None,
               smem_budget_kb: int = 0, iters: int = 4, passes: int = 2, keep_order: bool = False) -> Dict[str, object]:
     """Time every candidate on ``a @ weights[i]^T`` (cycling through ``weights``) and return
     ``{"best": kwargs, "us": best time, "auto_us": time of the cost model's own choice, "table": [...]}``.
-    Candidates the launcher rejects (shape not built, workspace too small) are skipped."""
+    Candidates the launcher rejects (shape not built, workspace too small) are skipped, and with ``keep_order`` those that
+    would add up in another order than the cost model's choice."""
     M, K = a.shape
     N = weights[0].shape[0]
     swiglu = weights_up is not None
     cands = candidates(M, N, K, swiglu)
+    if keep_order:
+        cands = same_order(cands, M, N, K, swiglu, 0 if workspace is None else workspace.numel() * workspace.element_size())
     best_us = [float("inf")] * len(cands)
     layer = 0
 

@@ -516,6 +516,7 @@ class LayerListEngine(Engine):
         if shape is not None:
             p.tile_m, p.tile_n, p.cta_group = shape["tile_m"], shape["tile_n"], shape["cta_group"]
             p.split_k, p.stream_k = shape["split_k"], shape["stream_k"]
+            p.tuned_rows = shape.get("rows", 0)
         self._op(name, p, dyn=[("M", rows)], kernel=self.gemm_kernel, layer=layer)
 
     # ---- mixers: read self.h, leave their output projection in self.y ---------------------------------
@@ -823,7 +824,9 @@ class LayerListEngine(Engine):
 
     # ---- GEMM shapes ----------------------------------------------------------------------------------
     def _autotune(self) -> None:
-        """Measured shapes for the dense products of every distinct layer at the full batch size."""
+        """Measured shapes for the dense products of every distinct layer at the full batch size. The picks may differ from one
+        start to the next and the results may not: only shapes that leave K whole are offered, and the launcher takes them only
+        where its own shape does so too (``keep_order``)."""
         from ..ops import autotune
         m, T, done = self.model, self.T, {}
         self.h.normal_()
@@ -868,7 +871,7 @@ class LayerListEngine(Engine):
                     done[sig] = autotune.tune_gemm(a, [wt], dst, weights_up=None if up is None else [up], workspace=self.gemm_ws,
                                                     keep_order=True)
                 res = done[sig]
-                self.eng.gemm_shapes[name] = dict(res["best"])
+                self.eng.gemm_shapes[name] = dict(res["best"], rows=T)
                 self.gemm_tuning[name] = dict(M=T, best=res["best"], us=res["us"], auto_us=res["auto_us"])
         torch.cuda.synchronize(self.device)
         for t in (self.h, self.y, *self.flat.values()):

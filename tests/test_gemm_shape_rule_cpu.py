@@ -4,6 +4,7 @@ from ctypes import byref, c_void_p
 import pytest
 
 from nanoflow_b200 import ops
+from nanoflow_b200.ops import autotune
 
 
 def _plan(M, N, K, **f):
@@ -30,3 +31,30 @@ def test_the_model_chooses_what_is_built(M, N, K, swiglu):
     pl = _plan(M, N, K, epilogue=swiglu)
     assert pl["stages"] >= 2 and pl["tile_m"] * pl["tile_n"] <= 512 and pl["smem_bytes"] <= 227 * 1024
     assert not (pl["cta_group"] == 2 and (M <= 128 or pl["tile_m"] != 1)) and not (swiglu and pl["split_k"] != 1)
+
+
+def _cut(plan):
+    """Where K is cut: tiles of the tail and their ranges, or the number of equal parts."""
+    if plan["stream_k"]:
+        return tuple(plan[k] for k in ("tile_m", "tile_n", "cta_group", "tail_first_tile", "tail_range_kb"))
+    return plan["split_k"]
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("N,K", [(4608, 4096), (4096, 4096), (12288, 4096), (4096, 14336), (14336, 4096), (64, 128)])
+def test_no_pick_moves_the_cut_of_k_where_the_order_is_kept(N, K, swiglu):
+    """Whatever the tuner offers at the dense batch, and whatever shape it would pin, K is cut as it is without a pick."""
+    T, ws = 2048, 160 << 20
+    every = autotune.candidates(T, N, K, swiglu)
+    offered = autotune.same_order(every, T, N, K, swiglu, ws)
+    assert autotune.AUTO in offered
+    for M in (1, 96, 128, 700, 1793, 1840, 2000, 2048, 4096):
+        want = _cut(ops.gemm_plan(M, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True))
+        for c in every:
+            if c["split_k"] > 1 and swiglu:
+                continue
+            got = ops.gemm_plan(M, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True, tuned_rows=T, **c)
+            assert _cut(got) == want, (M, c, got)
+    own = _cut(ops.gemm_plan(T, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True))
+    for c in offered:
+        assert c == autotune.AUTO or (own == 1 and _cut(ops.gemm_plan(T, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True, **c)) == 1)
