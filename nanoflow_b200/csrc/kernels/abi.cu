@@ -6,27 +6,6 @@
 
 using namespace nf;
 
-extern "C" int nfk_norm_p(const nfk_norm_params* p, cudaStream_t s) {
-  if (!p) return NF_ERR_BAD_ARG;
-  return p->resid ? nfk_add_rmsnorm(p->out, p->resid, p->x, p->w, p->rows, p->cols, p->eps, s)
-                  : nfk_rmsnorm(p->out, p->x, p->w, p->rows, p->cols, p->eps, s);
-}
-extern "C" int nfk_embedding_p(const nfk_embedding_params* p, cudaStream_t s) {
-  if (!p) return NF_ERR_BAD_ARG;
-  return nfk_embedding(p->out, p->table, p->host_ids, p->feedback_src, p->prev_tokens, p->ids_out,
-                       p->n_tokens, p->hidden, p->vocab, p->status, s);
-}
-extern "C" int nfk_gather_p(const nfk_gather_params* p, cudaStream_t s) {
-  if (!p) return NF_ERR_BAD_ARG;
-  return nfk_gather_rows(p->out, p->in, p->rows_idx, p->n, p->cols, p->ld_in, p->status, p->in_rows, s);
-}
-extern "C" int nfk_argmax_p(const nfk_argmax_params* p, cudaStream_t s) {
-  if (!p) return NF_ERR_BAD_ARG;
-  if (p->dtype == NFK_F32)
-    return nfk_argmax_f32(p->idx_out, p->val_out, reinterpret_cast<const float*>(p->logits), p->rows, p->cols, p->ld,
-                          p->col_offset, s);
-  return nfk_argmax(p->idx_out, p->val_out, p->logits, p->rows, p->cols, p->ld, p->col_offset, s);
-}
 extern "C" int nfk_argmax_combine_p(const nfk_argmax_combine_params* p, cudaStream_t s) {
   if (!p) return NF_ERR_BAD_ARG;
   return nfk_argmax_combine(p->idx_out, p->cand_val, p->cand_idx, p->shards, p->rows, s);

@@ -661,10 +661,11 @@ int launch_decode_st(const nfk_attn_params* p, cudaStream_t stream) {
   if (ctas > total) ctas = total;
   static std::atomic<unsigned int> launch_seq{0};
   const int slot = static_cast<int>(launch_seq.fetch_add(1u) % kDecodeCounterSlots);
-  cudaError_t e = launch_early(attn_decode_kernel<HD, ST, EXT>, static_cast<int>(ctas), kDecThreads, Cfg::SMEM_BYTES, stream, 1,
-                               *p, slot);
+  cudaError_t e = launch_kernel(early_first(p->early_start), attn_decode_kernel<HD, ST, EXT>, static_cast<int>(ctas), kDecThreads,
+                                Cfg::SMEM_BYTES, stream, 1, *p, slot);
   if (e == cudaSuccess && p->chunk_pages > 0 && max_chunks > 1)
-    e = launch_early(attn_decode_merge_kernel<HD>, p->req_count * p->q_heads, HD, 0, stream, 1, *p);
+    e = launch_kernel(early_further(p->early_start), attn_decode_merge_kernel<HD>, p->req_count * p->q_heads, HD, 0, stream, 1,
+                      *p);
   if (e == cudaSuccess) return NF_OK;
   (void)cudaGetLastError();
   return NF_ERR_CUDA;

@@ -540,8 +540,8 @@ int launch_ws(const nfk_attn_params& p, const CUtensorMap& tmQ, const CUtensorMa
   const long long total = static_cast<long long>(p.num_items) * p.kv_heads;
   long long ctas = p.num_ctas > 0 ? p.num_ctas : 2LL * device_sm_count();   // two resident CTAs per SM
   if (ctas > total) ctas = total;
-  if (launch_early(attn_prefill_ws_kernel<HD, EXT, CAP, DIST>, static_cast<int>(ctas), kThreads, bytes, stream, 1, tmQ, tmKV, p) ==
-      cudaSuccess)
+  if (launch_kernel(early_first(p.early_start), attn_prefill_ws_kernel<HD, EXT, CAP, DIST>, static_cast<int>(ctas), kThreads, bytes,
+                    stream, 1, tmQ, tmKV, p) == cudaSuccess)
     return NF_OK;
   (void)cudaGetLastError();
   return NF_ERR_CUDA;

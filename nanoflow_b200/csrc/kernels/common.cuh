@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
+
 namespace nf {
 
 // ---- host-visible error codes (returned by every extern "C" launcher) -------------------------
@@ -331,11 +333,16 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
 }
 
 // ---- launches that overlap the end of the kernel before them ------------------------------------------
-// A kernel launched by launch_early may start while the kernel before it on the stream still runs, as soon as every CTA
-// of that one has called let_next_start() (or has ended). await_previous() returns when all earlier work is complete and
+// A kernel launched early (launch_kernel) may start while the kernel before it on the stream still runs, as soon as every
+// CTA of that one has called let_next_start() (or has ended). await_previous() returns when all earlier work is complete and
 // visible; every CTA calls it before its first access to memory that earlier work writes or reads, and no CTA ends
 // without having called it, so that completion stays transitive along a stream. A kernel that allocates tensor memory
 // calls let_next_start() after that: the next kernel cannot then take columns that it still needs.
+//
+// Who launches early is the graph's choice (early_start of an op's parameters): CTAs that have started early hold threads,
+// registers and shared memory of their SM while they wait, and where another stream's kernel is to run beside the one that
+// they wait for, those are its places (a GEMM of 192 threads with four waiting CTAs of the rotary kernel, 256 threads each,
+// leaves no registers for a collective's CTA).
 NF_DEVICE void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 NF_DEVICE void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -357,24 +364,32 @@ NF_DEVICE float2 unpack_bf16x2(uint32_t u) {
 #endif  // __CUDACC__
 
 #ifdef __CUDACC__
-// kernel<<<grid, block, smem, stream>>>(args...), allowed to start early (see let_next_start), in clusters of `cluster` CTAs.
+inline bool early_first(int early_start) { return (early_start & NFK_EARLY_FIRST) != 0; }
+inline bool early_further(int early_start) { return (early_start & NFK_EARLY_FURTHER) != 0; }
+// kernel<<<grid, block, smem, stream>>>(args...) in clusters of `cluster` CTAs; `early`: see let_next_start.
 template <class... P, class... A>
-inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, int cluster,
-                                A... args) {
+inline cudaError_t launch_kernel(bool early, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, int cluster,
+                                 A... args) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(grid);
   lc.blockDim = dim3(block);
   lc.dynamicSmemBytes = smem;
   lc.stream = stream;
   cudaLaunchAttribute la[2];
-  la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  la[0].val.programmaticStreamSerializationAllowed = 1;
-  la[1].id = cudaLaunchAttributeClusterDimension;
-  la[1].val.clusterDim.x = cluster;
-  la[1].val.clusterDim.y = 1;
-  la[1].val.clusterDim.z = 1;
   lc.attrs = la;
-  lc.numAttrs = cluster > 1 ? 2 : 1;
+  lc.numAttrs = 0;
+  if (early) {
+    cudaLaunchAttribute& a = la[lc.numAttrs++];
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    cudaLaunchAttribute& a = la[lc.numAttrs++];
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = cluster;
+    a.val.clusterDim.y = 1;
+    a.val.clusterDim.z = 1;
+  }
   return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
 }
 #endif

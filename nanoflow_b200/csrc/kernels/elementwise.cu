@@ -342,21 +342,22 @@ inline int started(cudaError_t e) {
   return NF_ERR_CUDA;
 }
 template <class T>
-int launch_argmax(int* idx_out, float* val_out, const T* logits, int rows, int cols, long long ld, int col_offset,
-                  cudaStream_t stream) {
+int launch_argmax(const nfk_argmax_params& p, cudaStream_t stream) {
   // a thread of a part has two loads at least; with a split every cluster has one row
   int split = 1;
-  while (split < 8 && rows * split * 2 <= 2 * device_sm_count() && cols >= split * 2 * kArgmaxThreads * 8 * 2) split *= 2;
-  return started(launch_early(argmax_kernel<T>, split > 1 ? rows * split : grid_for(rows), kArgmaxThreads, 0, stream, split,
-                              idx_out, val_out, logits, rows, cols, ld, col_offset, split));
+  while (split < 8 && p.rows * split * 2 <= 2 * device_sm_count() && p.cols >= split * 2 * kArgmaxThreads * 8 * 2) split *= 2;
+  return started(launch_kernel(early_first(p.early_start), argmax_kernel<T>, split > 1 ? p.rows * split : grid_for(p.rows),
+                               kArgmaxThreads, 0, stream, split, p.idx_out, p.val_out, (const T*)p.logits, p.rows, p.cols, p.ld,
+                               p.col_offset, split));
 }
 template <bool ADD>
-int launch_norm(__nv_bfloat16* out, __nv_bfloat16* resid, const __nv_bfloat16* x, const __nv_bfloat16* w, int rows, int cols,
-                float eps, cudaStream_t stream) {
-  const int per = ((cols >> 3) + kNormThreads - 1) / kNormThreads;
+int launch_norm(const nfk_norm_params& p, cudaStream_t stream) {
+  const int per = ((p.cols >> 3) + kNormThreads - 1) / kNormThreads;
   auto* kernel = per <= 1 ? rmsnorm_kernel<ADD, 1> : per <= 2 ? rmsnorm_kernel<ADD, 2> : per <= 4 ? rmsnorm_kernel<ADD, 4>
                                                                                          : rmsnorm_kernel<ADD, kNormMaxVec>;
-  return started(launch_early(kernel, grid_for(rows), kNormThreads, 0, stream, 1, out, resid, x, w, rows, cols, eps));
+  return started(launch_kernel(early_first(p.early_start), kernel, grid_for(p.rows), kNormThreads, 0, stream, 1,
+                               (__nv_bfloat16*)p.out, (__nv_bfloat16*)p.resid, (const __nv_bfloat16*)p.x, (const __nv_bfloat16*)p.w,
+                               p.rows, p.cols, p.eps));
 }
 inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -366,46 +367,63 @@ inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) =
 using namespace nf;
 typedef __nv_bfloat16 bf16;
 
+extern "C" int nfk_norm_p(const nfk_norm_params* p, cudaStream_t stream) {
+  if (p == nullptr) return NF_ERR_BAD_ARG;
+  if (p->rows == 0) return NF_OK;
+  if (!p->out || !p->x || !p->w || p->rows < 0 || p->cols <= 0 || p->cols % 8 != 0 || p->cols > kNormMaxVec * 8 * kNormThreads ||
+      !al16(p->out) || !al16(p->x) || !al16(p->w) || !al16(p->resid))
+    return NF_ERR_BAD_ARG;
+  return p->resid != nullptr ? launch_norm<true>(*p, stream) : launch_norm<false>(*p, stream);
+}
+
 extern "C" int nfk_rmsnorm(void* out, const void* x, const void* w, int rows, int cols, float eps,
                            cudaStream_t stream) {
-  if (rows == 0) return NF_OK;
-  if (!out || !x || !w || rows < 0 || cols <= 0 || cols % 8 != 0 ||
-      cols > kNormMaxVec * 8 * kNormThreads || !al16(out) || !al16(x) || !al16(w))
-    return NF_ERR_BAD_ARG;
-  return launch_norm<false>((bf16*)out, nullptr, (const bf16*)x, (const bf16*)w, rows, cols, eps, stream);
+  const nfk_norm_params p{out, x, w, nullptr, rows, cols, eps, 0};
+  return nfk_norm_p(&p, stream);
 }
 
 extern "C" int nfk_add_rmsnorm(void* out, void* resid, const void* x, const void* w, int rows,
                                int cols, float eps, cudaStream_t stream) {
-  if (rows == 0) return NF_OK;
-  if (!out || !x || !w || !resid || rows < 0 || cols <= 0 || cols % 8 != 0 ||
-      cols > kNormMaxVec * 8 * kNormThreads || !al16(out) || !al16(x) || !al16(w) || !al16(resid))
+  if (rows != 0 && resid == nullptr) return NF_ERR_BAD_ARG;
+  const nfk_norm_params p{out, x, w, resid, rows, cols, eps, 0};
+  return nfk_norm_p(&p, stream);
+}
+
+extern "C" int nfk_embedding_p(const nfk_embedding_params* p, cudaStream_t stream) {
+  if (p == nullptr) return NF_ERR_BAD_ARG;
+  if (p->n_tokens == 0) return NF_OK;
+  if (!p->out || !p->table || p->n_tokens < 0 || p->hidden % 8 != 0 || p->vocab <= 0 || !al16(p->out) || !al16(p->table))
     return NF_ERR_BAD_ARG;
-  return launch_norm<true>((bf16*)out, (bf16*)resid, (const bf16*)x, (const bf16*)w, rows, cols, eps, stream);
+  if (p->host_ids == nullptr && (p->feedback_src == nullptr || p->prev_tokens == nullptr))
+    return NF_ERR_BAD_ARG;
+  return started(launch_kernel(early_first(p->early_start), embedding_kernel, grid_for(p->n_tokens), 128, 0, stream, 1, (bf16*)p->out,
+                               (const bf16*)p->table, p->host_ids, p->feedback_src, p->prev_tokens, p->ids_out, p->n_tokens,
+                               p->hidden, p->vocab, p->status));
 }
 
 extern "C" int nfk_embedding(void* out, const void* table, const int* host_ids,
                              const int* feedback_src, const int* prev_tokens, int* ids_out,
                              int n_tokens, int hidden, int vocab, unsigned int* status,
                              cudaStream_t stream) {
-  if (n_tokens == 0) return NF_OK;
-  if (!out || !table || n_tokens < 0 || hidden % 8 != 0 || vocab <= 0 || !al16(out) || !al16(table))
+  const nfk_embedding_params p{out, table, host_ids, feedback_src, prev_tokens, ids_out, n_tokens, hidden, vocab, status, 0};
+  return nfk_embedding_p(&p, stream);
+}
+
+extern "C" int nfk_gather_p(const nfk_gather_params* p, cudaStream_t stream) {
+  if (p == nullptr) return NF_ERR_BAD_ARG;
+  if (p->n == 0) return NF_OK;
+  if (!p->out || !p->in || !p->rows_idx || p->n < 0 || p->cols % 8 != 0 || p->ld_in % 8 != 0 || !al16(p->out) ||
+      !al16(p->in) || p->in_rows <= 0)
     return NF_ERR_BAD_ARG;
-  if (host_ids == nullptr && (feedback_src == nullptr || prev_tokens == nullptr))
-    return NF_ERR_BAD_ARG;
-  return started(launch_early(embedding_kernel, grid_for(n_tokens), 128, 0, stream, 1, (bf16*)out, (const bf16*)table,
-                              host_ids, feedback_src, prev_tokens, ids_out, n_tokens, hidden, vocab, status));
+  return started(launch_kernel(early_first(p->early_start), gather_rows_kernel, grid_for(p->n), 128, 0, stream, 1, (bf16*)p->out,
+                               (const bf16*)p->in, p->rows_idx, p->n, p->cols, p->ld_in, p->in_rows, p->status));
 }
 
 extern "C" int nfk_gather_rows(void* out, const void* in, const int* rows_idx, int n, int cols,
                                long long ld_in, unsigned int* status, int in_rows,
                                cudaStream_t stream) {
-  if (n == 0) return NF_OK;
-  if (!out || !in || !rows_idx || n < 0 || cols % 8 != 0 || ld_in % 8 != 0 || !al16(out) ||
-      !al16(in) || in_rows <= 0)
-    return NF_ERR_BAD_ARG;
-  return started(launch_early(gather_rows_kernel, grid_for(n), 128, 0, stream, 1, (bf16*)out, (const bf16*)in, rows_idx, n,
-                              cols, ld_in, in_rows, status));
+  const nfk_gather_params p{out, in, rows_idx, n, cols, ld_in, in_rows, status, 0};
+  return nfk_gather_p(&p, stream);
 }
 
 extern "C" int nfk_silu_mul(void* out, const void* gate, const void* up, long long n,
@@ -440,19 +458,25 @@ extern "C" int nfk_transpose(void* out, const void* in, int rows, int cols, cuda
   return ok_or_cuda();
 }
 
+extern "C" int nfk_argmax_p(const nfk_argmax_params* p, cudaStream_t stream) {
+  if (p == nullptr) return NF_ERR_BAD_ARG;
+  if (p->rows == 0) return NF_OK;
+  const bool f32 = p->dtype == NFK_F32;
+  if (!p->idx_out || !p->logits || p->rows < 0 || p->cols <= 0 || p->ld % (f32 ? 4 : 8) != 0 || !al16(p->logits))
+    return NF_ERR_BAD_ARG;
+  return f32 ? launch_argmax<float>(*p, stream) : launch_argmax<__nv_bfloat16>(*p, stream);
+}
+
 extern "C" int nfk_argmax(int* idx_out, float* val_out, const void* logits, int rows, int cols,
                           long long ld, int col_offset, cudaStream_t stream) {
-  if (rows == 0) return NF_OK;
-  if (!idx_out || !logits || rows < 0 || cols <= 0 || ld % 8 != 0 || !al16(logits))
-    return NF_ERR_BAD_ARG;
-  return launch_argmax<__nv_bfloat16>(idx_out, val_out, (const bf16*)logits, rows, cols, ld, col_offset, stream);
+  const nfk_argmax_params p{idx_out, val_out, logits, rows, cols, ld, col_offset, NFK_BF16, 0};
+  return nfk_argmax_p(&p, stream);
 }
 
 extern "C" int nfk_argmax_f32(int* idx_out, float* val_out, const float* logits, int rows, int cols,
                               long long ld, int col_offset, cudaStream_t stream) {
-  if (rows == 0) return NF_OK;
-  if (!idx_out || !logits || rows < 0 || cols <= 0 || ld % 4 != 0 || !al16(logits)) return NF_ERR_BAD_ARG;
-  return launch_argmax<float>(idx_out, val_out, logits, rows, cols, ld, col_offset, stream);
+  const nfk_argmax_params p{idx_out, val_out, logits, rows, cols, ld, col_offset, NFK_F32, 0};
+  return nfk_argmax_p(&p, stream);
 }
 
 extern "C" int nfk_argmax_combine(int* idx_out, const float* cand_val, const int* cand_idx,

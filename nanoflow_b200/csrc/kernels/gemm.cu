@@ -1077,6 +1077,13 @@ inline DevParams dev_params(const nfk_gemm_params& g, bool linear) {
   return p;
 }
 
+// The norm of finished rows as a launch of its own.
+inline int rmsnorm_rows(const nfk_gemm_params& g, cudaStream_t stream) {
+  const nfk_norm_params n{g.norm_out, g.D, g.norm_w, nullptr, g.M, g.N, g.norm_eps,
+                          early_further(g.early_start) ? NFK_EARLY_FIRST : 0};
+  return nfk_norm_p(&n, stream);
+}
+
 constexpr int kSmemMax = 227 * 1024;
 
 // Stream-K tail: with `tiles` tiles on `workers` workers, the tiles_dp tiles of the full waves are
@@ -1198,8 +1205,9 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   p.acc_bufs = geo.acc_bufs;
   p.tmem_cols = geo.tmem_cols;
   p.rs_staged = rs_staged ? 1 : 0;
-  if (launch_early(gemm_tcgen05_kernel<MT, EPI, CG, WIDE>, ctas, kGemmThreads, geo.smem_bytes, stream, CG, tmA, tmB0, tmB1, p) !=
-      cudaSuccess) {
+  const bool further = early_further(g.early_start);
+  if (launch_kernel(early_first(g.early_start), gemm_tcgen05_kernel<MT, EPI, CG, WIDE>, ctas, kGemmThreads, geo.smem_bytes, stream, CG,
+                    tmA, tmB0, tmB1, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NF_ERR_CUDA;
   }
@@ -1208,7 +1216,8 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
     const long long total = static_cast<long long>(sk.rest) * CG * MT * BM * (geo.out_bn / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    if (launch_early(sk_fixup_kernel<gated_epi(EPI) ? 1 : 0>, static_cast<int>(blocks), 256, 0, stream, 1, p, f) != cudaSuccess) {
+    if (launch_kernel(further, sk_fixup_kernel<gated_epi(EPI) ? 1 : 0>, static_cast<int>(blocks), 256, 0, stream, 1, p, f) !=
+        cudaSuccess) {
       (void)cudaGetLastError();
       return NF_ERR_CUDA;
     }
@@ -1220,7 +1229,7 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   const bool want_norm = EPI == 0 && g.norm_w != nullptr;
   if (split_k > 1 && want_norm && g.N <= kRowVec * 8 * 256) {
     const int blocks = g.M < 16 * sm_count() ? g.M : 16 * sm_count();
-    if (launch_early(splitk_reduce_norm_kernel, blocks, 256, 0, stream, 1, p) == cudaSuccess) return NF_OK;
+    if (launch_kernel(further, splitk_reduce_norm_kernel, blocks, 256, 0, stream, 1, p) == cudaSuccess) return NF_OK;
     (void)cudaGetLastError();
     return NF_ERR_CUDA;
   }
@@ -1228,7 +1237,7 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
     const long long total = static_cast<long long>(g.M) * (g.N >> 3);
     long long blocks = (total + 255) / 256;
     if (blocks > 4ll * sm_count()) blocks = 4ll * sm_count();
-    if (launch_early(splitk_reduce_kernel, static_cast<int>(blocks), 256, 0, stream, 1, p) != cudaSuccess) {
+    if (launch_kernel(further, splitk_reduce_kernel, static_cast<int>(blocks), 256, 0, stream, 1, p) != cudaSuccess) {
       (void)cudaGetLastError();
       return NF_ERR_CUDA;
     }
@@ -1236,7 +1245,7 @@ int launch_impl(const nfk_gemm_params& g, int bn, int split_k, bool stream_k, cu
   if (want_norm) {
     // the result rows are complete in D (contiguous rows required): a plain norm launch follows
     if (g.ldd != g.N || g.norm_ld != g.N) return NF_ERR_UNSUPPORTED;
-    return nfk_rmsnorm(g.norm_out, g.D, g.norm_w, g.M, g.N, g.norm_eps, stream);
+    return rmsnorm_rows(g, stream);
   }
   return NF_OK;
 }
@@ -1295,12 +1304,12 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
   fp.kb_per = f.kb_per;
   fp.round_tokens = f.round_tokens;
   fp.early_weights = g.weights_ready;
-  if (launch_early(gemm_few_rows_kernel<GATED, CG>, f.n_tiles * f.tok_tiles * f.split * CG, kFewThreads, f.smem_bytes, stream,
-                   f.split * CG, tmW0, tmW1, tmX, fp) != cudaSuccess) {
+  if (launch_kernel(early_first(g.early_start), gemm_few_rows_kernel<GATED, CG>, f.n_tiles * f.tok_tiles * f.split * CG, kFewThreads,
+                    f.smem_bytes, stream, f.split * CG, tmW0, tmW1, tmX, fp) != cudaSuccess) {
     (void)cudaGetLastError();
     return NF_ERR_CUDA;
   }
-  if (!GATED && g.norm_w != nullptr) return nfk_rmsnorm(g.norm_out, g.D, g.norm_w, g.M, g.N, g.norm_eps, stream);
+  if (!GATED && g.norm_w != nullptr) return rmsnorm_rows(g, stream);
   return NF_OK;
 }
 
@@ -1440,6 +1449,10 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
 // A shape measured at another number of rows (tuned_rows) says little about this call: it holds for calls with as many
 // 256-row groups of tiles, and the cost model chooses for the others. A shape tuned at 1024 rows took 50 us for
 // 48 x 10240 x 8192, where the weight takes 26.
+//
+// With keep_order a stopwatch must not decide where K is cut: a pick changes with the clock of the day, and the order of sums
+// with it. Shapes that leave K whole all add up in the order of k, so a tuned one of them takes the place of a whole-K shape of
+// the cost model; where the model cuts K for this M, or the tuned shape does, the model's shape stands.
 nfk_gemm_params with_own_shape(const nfk_gemm_params& g) {
   nfk_gemm_params p = g;
   if (g.tuned_rows <= 0) return p;
@@ -1451,10 +1464,6 @@ nfk_gemm_params with_own_shape(const nfk_gemm_params& g) {
   }
   return g;
 }
-//
-// With keep_order a stopwatch must not decide where K is cut: a pick changes with the clock of the day, and the order of sums
-// with it. Shapes that leave K whole all add up in the order of k, so a tuned one of them takes the place of a whole-K shape of
-// the cost model; where the model cuts K for this M, or the tuned shape does, the model's shape stands.
 
 // Shape of this call: the cost model's, or the caller's pinned one, checked against what is built.
 int resolve_shape(const nfk_gemm_params& gp, bool swiglu, bool rs, Shape& s) {

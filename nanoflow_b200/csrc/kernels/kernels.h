@@ -19,6 +19,8 @@ enum { NFK_EPI_LINEAR = 0, NFK_EPI_SWIGLU = 1, NFK_EPI_REDUCE_SCATTER = 2 };
 enum { NFK_ACT_SILU = 0, NFK_ACT_RELU = 1, NFK_ACT_GELU_TANH = 2, NFK_ACT_CAPPED = 3 };
 // activation of the linear epilogue (GELU: by erf; RELU2: the square of relu)
 enum { NFK_LIN_NONE = 0, NFK_LIN_TANH = 1, NFK_LIN_GELU = 2, NFK_LIN_RELU2 = 3 };
+// early_start of a parameter block: the call's first kernel / its further kernels may start early
+enum { NFK_EARLY_FIRST = 1, NFK_EARLY_FURTHER = 2 };
 enum { NFK_BF16 = 0, NFK_F32 = 1 };                                    // storage type of activations and weights
 
 typedef struct nfk_gemm_params {
@@ -89,13 +91,16 @@ typedef struct nfk_gemm_params {
   const void* bias2;    // gated epilogue: [N] bf16 bias of the up half (`bias` is the gate half's), null = none
   int rows_kernel;      // the kernel for few rows (gemm_few_rows.cuh): 0 = by rule; 1 = it (`cta_group` 1 / 2 and `split_k`
                         // as given, 0 = choose); 2 = the tile kernel
-  int weights_ready;    // B and B2 were complete before the launch that precedes this one on the stream (weights of a model
-                        // that is loaded): they may be fetched while that one still runs
+  int weights_ready;    // B and B2 are complete (weights of a loaded model): with early_start they may be fetched while the
+                        // launches before this one, back to the last that was not early, still run
   int tuned_rows;       // rows that the pinned shape was measured at: a call with another number of 256-row groups leaves
                         // the shape to the cost model (0 = the shape holds for every M)
   int keep_order;       // 1 = the order of sums follows from M, N and K alone, by the earlier rules: shapes and kernel by these,
                         // a tuned shape (tuned_rows > 0) only where it and the rules' shape leave K whole (layer-list models:
                         // a recurrent state carries a change of rounding on)
+  int early_start;      // NFK_EARLY_*: kernels of this call that may start while the one before them on the stream ends (they
+                        // wait for it before they touch what it reads or writes). Not where a kernel of another stream is to
+                        // run beside that one: CTAs that have started and wait would hold its places on the SMs
 } nfk_gemm_params;
 
 int nfk_gemm_bf16(const nfk_gemm_params* p, cudaStream_t stream);
@@ -174,6 +179,7 @@ typedef struct nfk_rope_append_params {
   unsigned int* status;
   const float* cos_sin;  // optional [T][head_dim/2][2] (cos, sin) of every token's angles (nfk_rope_table);
                          // null: the kernel computes them itself
+  int early_start;       // see nfk_gemm_params (with cos_sin; the kernel that computes angles itself has no early form)
 } nfk_rope_append_params;
 int nfk_rope_append(const nfk_rope_append_params* p, cudaStream_t stream);
 
@@ -184,6 +190,7 @@ typedef struct nfk_rope_table_params {
   const float* inv_freq; // [half]
   const int* positions;  // [T]
   int T, half;
+  int early_start;       // see nfk_gemm_params
 } nfk_rope_table_params;
 int nfk_rope_table(const nfk_rope_table_params* p, cudaStream_t stream);
 
@@ -227,6 +234,7 @@ typedef struct nfk_attn_params {
   const int* kv_first;     // [B] page slot of the sequence that a request's page list starts with; null = 0
   const float* dist;       // [q_heads][2] (a, b): score <- score - a ln(1 + b (i - j)); null = none
   int chunk;               // > 0: position i sees j only if i / chunk = j / chunk
+  int early_start;         // nfk_attn_decode, nfk_attn_prefill_ws: see nfk_gemm_params
 } nfk_attn_params;
 int nfk_attn_decode(const nfk_attn_params* p, cudaStream_t stream);
 // The same with the pages copied by a TMA producer warp into a ring of decode_stages (2, 3 or 4) pages per
@@ -303,6 +311,7 @@ typedef struct nfk_residual_norm_params {
   float* hist_out;           // [*, ld_x], null: none
   long long hist_stride;
   int hist_n;
+  int early_start;           // see nfk_gemm_params
 } nfk_residual_norm_params;
 int nfk_residual_norm(const nfk_residual_norm_params* p, cudaStream_t stream);
 
@@ -840,18 +849,20 @@ int nfk_ipc_close_handle(void* p);
 typedef struct nfk_norm_params {
   void* out; const void* x; const void* w; void* resid;   // resid != NULL: resid += x, out = norm(resid)
   int rows, cols; float eps;
+  int early_start;   // see nfk_gemm_params; likewise below
 } nfk_norm_params;
 typedef struct nfk_embedding_params {
   void* out; const void* table; const int* host_ids; const int* feedback_src; const int* prev_tokens;
-  int* ids_out; int n_tokens, hidden, vocab; unsigned int* status;
+  int* ids_out; int n_tokens, hidden, vocab; unsigned int* status; int early_start;
 } nfk_embedding_params;
 typedef struct nfk_gather_params {
   void* out; const void* in; const int* rows_idx; int n, cols; long long ld_in; int in_rows;
-  unsigned int* status;
+  unsigned int* status; int early_start;
 } nfk_gather_params;
 typedef struct nfk_argmax_params {
   int* idx_out; float* val_out; const void* logits; int rows, cols; long long ld; int col_offset;
   int dtype;   // NFK_BF16 / NFK_F32
+  int early_start;
 } nfk_argmax_params;
 typedef struct nfk_argmax_combine_params {
   int* idx_out; const float* cand_val; const int* cand_idx; int shards, rows;

@@ -410,7 +410,7 @@ int launch_plain(const nfk_residual_norm_params& p, cudaStream_t stream) {
   const int cap = device_sm_count() * 16;
   const int grid = p.rows < cap ? p.rows : cap;
   auto* kernel = p.in_kind == NFK_NORM_LAYER ? residual_norm_plain_kernel<T, NV, true> : residual_norm_plain_kernel<T, NV, false>;
-  return started(launch_early(kernel, grid, kRnThreads, 0, stream, 1, p));
+  return started(launch_kernel(early_first(p.early_start), kernel, grid, kRnThreads, 0, stream, 1, p));
 }
 
 template <class T, bool CONV, bool DEEP>
@@ -418,12 +418,13 @@ int launch_rn(const nfk_residual_norm_params& p, cudaStream_t stream) {
   const int nvec = (p.cols + 3) / 4, per = (nvec + kRnThreads - 1) / kRnThreads;
   const int cap = device_sm_count() * 16;
   const int grid = p.rows < cap ? p.rows : cap;
+  const bool early = early_first(p.early_start);
   cudaError_t e;
-  if (per <= 1) e = launch_early(residual_norm_kernel<T, 1, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
-  else if (per <= 2) e = launch_early(residual_norm_kernel<T, 2, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
-  else if (per <= 4) e = launch_early(residual_norm_kernel<T, 4, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
-  else if (per <= 8) e = launch_early(residual_norm_kernel<T, 8, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
-  else if (per <= 16) e = launch_early(residual_norm_kernel<T, 16, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  if (per <= 1) e = launch_kernel(early, residual_norm_kernel<T, 1, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 2) e = launch_kernel(early, residual_norm_kernel<T, 2, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 4) e = launch_kernel(early, residual_norm_kernel<T, 4, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 8) e = launch_kernel(early, residual_norm_kernel<T, 8, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
+  else if (per <= 16) e = launch_kernel(early, residual_norm_kernel<T, 16, CONV, DEEP>, grid, kRnThreads, 0, stream, 1, p);
   else return NF_ERR_UNSUPPORTED;
   return started(e);
 }

@@ -183,7 +183,8 @@ extern "C" int nfk_rope_table(const nfk_rope_table_params* p, cudaStream_t strea
   const long long total = static_cast<long long>(p->T) * p->half;
   long long blocks = (total + 255) / 256;
   if (blocks > device_sm_count() * 8) blocks = device_sm_count() * 8;
-  if (launch_early(rope_table_kernel, static_cast<int>(blocks), 256, 0, stream, 1, *p) == cudaSuccess) return NF_OK;
+  if (launch_kernel(early_first(p->early_start), rope_table_kernel, static_cast<int>(blocks), 256, 0, stream, 1, *p) == cudaSuccess)
+    return NF_OK;
   (void)cudaGetLastError();
   return NF_ERR_CUDA;
 }
@@ -206,7 +207,8 @@ extern "C" int nfk_rope_append(const nfk_rope_append_params* p, cudaStream_t str
     const long long total = static_cast<long long>(p->T) * units;
     long long nb = (total + 255) / 256;
     if (nb > device_sm_count() * 16) nb = device_sm_count() * 16;
-    if (launch_early(rope_append_table_kernel, static_cast<int>(nb), 256, 0, stream, 1, *p) == cudaSuccess) return NF_OK;
+    if (launch_kernel(early_first(p->early_start), rope_append_table_kernel, static_cast<int>(nb), 256, 0, stream, 1, *p) == cudaSuccess)
+      return NF_OK;
     (void)cudaGetLastError();
     return NF_ERR_CUDA;
   }

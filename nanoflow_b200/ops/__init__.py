@@ -46,7 +46,10 @@ class GemmParams(Structure):
                 ("groups", c_int), ("group_k", c_int), ("lin_act", c_int),
                 ("act_limit", c_float), ("act_alpha", c_float), ("act_shift", c_float), ("bias2", c_void_p),
                 ("rows_kernel", c_int), ("weights_ready", c_int), ("tuned_rows", c_int),
-                ("keep_order", c_int)]
+                ("keep_order", c_int), ("early_start", c_int)]
+
+
+EARLY_FIRST, EARLY_FURTHER = 1, 2      # early_start of a parameter block (NFK_EARLY_* of kernels.h)
 
 
 class RopeAppendParams(Structure):
@@ -56,12 +59,13 @@ class RopeAppendParams(Structure):
                 ("positions", c_void_p), ("token_req", c_void_p), ("kv_indptr", c_void_p),
                 ("kv_indices", c_void_p),
                 ("T", c_int), ("q_heads", c_int), ("kv_heads", c_int), ("head_dim", c_int),
-                ("page_size", c_int), ("num_pages", c_int), ("status", c_void_p), ("cos_sin", c_void_p)]
+                ("page_size", c_int), ("num_pages", c_int), ("status", c_void_p), ("cos_sin", c_void_p),
+                ("early_start", c_int)]
 
 
 class RopeTableParams(Structure):
     _fields_ = [("cos_sin", c_void_p), ("inv_freq", c_void_p), ("positions", c_void_p), ("T", c_int),
-                ("half", c_int)]
+                ("half", c_int), ("early_start", c_int)]
 
 
 class AttnParams(Structure):
@@ -75,7 +79,7 @@ class AttnParams(Structure):
                 ("items", c_void_p), ("num_items", c_int), ("status", c_void_p), ("decode_stages", c_int),
                 ("window", c_int), ("sinks", c_void_p), ("kv_ld", c_int), ("k_col", c_int), ("v_col", c_int),
                 ("q_rows", c_int), ("ld_q", c_int), ("softcap", c_float), ("precise", c_int), ("kv_first", c_void_p),
-                ("dist", c_void_p), ("chunk", c_int)]
+                ("dist", c_void_p), ("chunk", c_int), ("early_start", c_int)]
 
 
 BF16, F32 = 0, 1                                        # storage type of a kernel's activations and weights
@@ -106,7 +110,8 @@ class ResidualNormParams(Structure):
                 ("pair_w", c_void_p), ("pair_w2", c_void_p), ("table_add", c_int), ("conv_w", c_void_p), ("conv_out", c_void_p),
                 ("conv_state", c_void_p), ("state_slot", c_void_p), ("positions", c_void_p), ("conv_taps", c_int),
                 ("conv_rows", c_int), ("conv_ld", c_int), ("num_slots", c_int), ("pos_freq", c_void_p), ("hist", c_void_p),
-                ("hist_w", c_void_p), ("hist_out", c_void_p), ("hist_stride", c_longlong), ("hist_n", c_int)]
+                ("hist_w", c_void_p), ("hist_out", c_void_p), ("hist_stride", c_longlong), ("hist_n", c_int),
+                ("early_start", c_int)]
 
 
 class LatentAppendParams(Structure):
@@ -390,9 +395,9 @@ def gemm_plan(M: int, N: int, K: int, *, swiglu: bool = False, tile_n: int = 0, 
     p.M, p.N, p.K = M, N, K
     p.epilogue, p.tile_n, p.tile_m, p.cta_group = (1 if swiglu else 0), tile_n, tile_m, cta_group
     p.split_k, p.stream_k, p.num_ctas, p.smem_budget_kb = split_k, stream_k, num_ctas, smem_budget_kb
+    p.keep_order, p.tuned_rows = int(keep_order), tuned_rows
     if workspace_bytes > 0:
         p.workspace, p.workspace_bytes = c_void_p(256), workspace_bytes    # never dereferenced by the planner
-    p.keep_order, p.tuned_rows = int(keep_order), tuned_rows
     out = GemmPlan()
     _check(lib().nfk_gemm_describe(byref(p), byref(out)), "nfk_gemm_describe")
     return {f: getattr(out, f) for f, _ in GemmPlan._fields_}

@@ -11,6 +11,9 @@ worker loop, pipeline/src/computeBound.cu:115-193):
 ``run(plan)``           the three above in sequence
 ``getPipelineOutput()`` tokens of the last waited iteration
 
+Weights may be rewritten between iterations, on the engine's stream or by work that is complete before ``run_async()``: the
+first kernel of an iteration waits for all that the stream holds, and no kernel of the iteration reads a weight before that.
+
 Input token ids of decode requests never visit the host: the embedding op reads them from the
 previous iteration's ``sampled`` array on the device through ``feedback_src`` indices
 (computeBound.cu:122-150 does this merge on the host in the reference).
@@ -255,6 +258,7 @@ class Engine:
     def _make_executor(self, kind: str) -> None:
         self.native = None
         single = not (self.eng.overlap or any(op.stream != "gemm" for op in self.graph.ops))
+        self.graph.allow_early_starts()
         if kind in ("auto", "native", "graph"):
             try:
                 from .native import NativeExecutor

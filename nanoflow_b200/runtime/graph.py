@@ -29,23 +29,23 @@ STREAM_CLASSES = ("gemm", "attn", "net", "other", "copy", "attn2", "net2")
 
 class NormParams(Structure):
     _fields_ = [("out", c_void_p), ("x", c_void_p), ("w", c_void_p), ("resid", c_void_p),
-                ("rows", c_int), ("cols", c_int), ("eps", c_float)]
+                ("rows", c_int), ("cols", c_int), ("eps", c_float), ("early_start", c_int)]
 
 
 class EmbeddingParams(Structure):
     _fields_ = [("out", c_void_p), ("table", c_void_p), ("host_ids", c_void_p), ("feedback_src", c_void_p),
                 ("prev_tokens", c_void_p), ("ids_out", c_void_p), ("n_tokens", c_int), ("hidden", c_int),
-                ("vocab", c_int), ("status", c_void_p)]
+                ("vocab", c_int), ("status", c_void_p), ("early_start", c_int)]
 
 
 class GatherParams(Structure):
     _fields_ = [("out", c_void_p), ("inp", c_void_p), ("rows_idx", c_void_p), ("n", c_int), ("cols", c_int),
-                ("ld_in", c_longlong), ("in_rows", c_int), ("status", c_void_p)]
+                ("ld_in", c_longlong), ("in_rows", c_int), ("status", c_void_p), ("early_start", c_int)]
 
 
 class ArgmaxParams(Structure):
     _fields_ = [("idx_out", c_void_p), ("val_out", c_void_p), ("logits", c_void_p), ("rows", c_int),
-                ("cols", c_int), ("ld", c_longlong), ("col_offset", c_int), ("dtype", c_int)]
+                ("cols", c_int), ("ld", c_longlong), ("col_offset", c_int), ("dtype", c_int), ("early_start", c_int)]
 
 
 class ArgmaxCombineParams(Structure):
@@ -160,6 +160,41 @@ class OpGraph:
                 raise ValueError(f"op {name}: dependency {d} is not an earlier op")
         self.ops.append(op)
         return len(self.ops) - 1
+
+    def allow_early_starts(self) -> None:
+        """Let kernels start while the one before them on their stream ends (``early_start`` of the parameter blocks).
+
+        A kernel that has started early waits on the SMs, and where another stream's kernel is to run beside the one that it
+        waits for, it would hold that kernel's places. So an op starts early only if every op of another stream that may run
+        beside its predecessor is complete before it starts (it waits for that op as well), and the further kernels of an op
+        only if nothing runs beside the op. An op that is launched when another one has *started* (gated input) never does.
+        The first kernel of a stream stays a full dependency, so that whatever the caller queued before the iteration, new
+        weights for instance, is complete before any kernel of the iteration reads it."""
+        n, last, pred, kernel_seen = len(self.ops), {}, [-1] * len(self.ops), set()
+        before, after, follows = [0] * n, [0] * n, [[] for _ in range(n)]    # ops ordered before / after, as bit masks
+        on = {s: sum(1 << i for i, op in enumerate(self.ops) if op.stream == s) for s in STREAM_CLASSES}
+        for i, op in enumerate(self.ops):
+            pred[i] = last.get(op.stream, -1)
+            for d in op.deps + ([pred[i]] if pred[i] >= 0 else []):
+                before[i] |= before[d] | 1 << d
+                follows[d].append(i)
+            last[op.stream] = i
+        for i in range(n - 1, -1, -1):
+            for j in follows[i]:
+                after[i] |= after[j] | 1 << j
+        beside = [((1 << n) - 1) & ~on[op.stream] & ~before[i] & ~after[i] for i, op in enumerate(self.ops)]
+        for i, op in enumerate(self.ops):
+            if isinstance(op.params, (MemcpyParams, Memcpy2DParams)):
+                continue
+            first = op.stream not in kernel_seen
+            kernel_seen.add(op.stream)
+            if not hasattr(op.params, "early_start"):
+                continue
+            behind = not first and any(after[pred[i]] >> d & 1 for d in op.deps)     # the predecessor has long ended
+            if not first and not behind and not op.after_start and not beside[pred[i]] & ~before[i]:
+                op.params.early_start |= _ops.EARLY_FIRST
+            if not beside[i]:
+                op.params.early_start |= _ops.EARLY_FURTHER
 
     # ---- static checks (the host-side dependency checker) -----------------------------------------
     def happens_before(self) -> List[set]:

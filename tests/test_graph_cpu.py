@@ -486,3 +486,64 @@ def test_collectives_beside_other_kernels_get_a_cta_budget_by_form_and_rank_coun
     g1, _, keep1 = _host_graph("NON_OVERLAP", 2, None)         # nothing runs beside: the collective's own default (all SMs)
     coll = keep1[2]
     assert all(op.params.num_ctas == coll.num_ctas for op in g1.ops if op.kernel == "nfk_allreduce" and op.layer >= 0)
+
+
+def _early(g):
+    g.allow_early_starts()
+    return {op.name: op.params.early_start for op in g.ops if hasattr(op.params, "early_start")}
+
+
+@pytest.mark.parametrize("pipeline_type,tp,nano", [("NON_OVERLAP_LOCAL", 1, None), ("NANOBATCH_LOCAL", 1, [16, 32]), ("NON_OVERLAP", 2, None)])
+def test_kernels_in_line_start_early(pipeline_type, tp, nano):
+    """All on one stream but the prefill attention: everything starts early but the first kernel, the prefill attention (it
+    waits for another stream) and the further kernels of the decode attention, beside which the prefill attention runs."""
+    g, _, _keep = _host_graph(pipeline_type, tp, nano)
+    assert not any(getattr(op.params, "early_start", 0) for op in g.ops)
+    early = _early(g)
+    assert early.pop("embedding") == 2
+    for name, bits in early.items():
+        if "attn_prefill" in name:
+            assert bits == 0
+        elif nano is None:
+            assert bits == (1 if "attn_decode" in name else 3), name
+        else:
+            assert bits & 1 or name.split(".")[-1] in ("ln_attn", "qkv", "rope_append", "attn_decode"), name
+
+
+@pytest.mark.parametrize("cross_layer", [False, True])
+@pytest.mark.parametrize("attn_overlap", [False, True])
+@pytest.mark.parametrize("tp,nano,pipeline_type", [(1, None, "NON_OVERLAP_LOCAL"), (1, [16, 32], "NANOBATCH_LOCAL"), (1, [16, 32], "LOCAL"),
+                                                   (2, [16, 32], "PLLM"), (2, [16, 16, 16], "PLLM")])
+def test_nothing_waits_in_the_places_of_another_streams_kernel(tp, nano, pipeline_type, attn_overlap, cross_layer):
+    """While an op that has started early waits for its predecessor, every op of another stream is complete or ordered behind
+    the predecessor; and beside an op whose further kernels start early, nothing runs at all."""
+    g, _, _keep = _host_graph(pipeline_type, tp, nano, attn_overlap=attn_overlap, cross_layer=cross_layer)
+    early, last, before, seen = _early(g), {}, [], 0
+    preds = []
+    for i, op in enumerate(g.ops):
+        preds.append(last.get(op.stream))
+        mine = set()
+        for d in list(op.deps) + ([preds[i]] if preds[i] is not None else []):
+            mine |= before[d] | {d}
+        before.append(mine)
+        last[op.stream] = i
+    for i, op in enumerate(g.ops):
+        bits, others = early.get(op.name, 0), [o for o in range(len(g.ops)) if g.ops[o].stream != op.stream]
+        if bits & 1:
+            seen += 1
+            assert not op.after_start and all(o in before[i] or preds[i] in before[o] for o in others), op.name
+        if bits & 2:
+            assert all(o in before[i] or i in before[o] for o in others), op.name
+    assert seen > 0
+    if tp > 1:      # a product beside which a collective runs has nobody waiting on its SMs
+        for i, op in enumerate(g.ops):
+            if op.name.endswith((".rope_append", ".down")) and any(
+                    o not in before[i] and preds[i] not in before[o] for o in range(len(g.ops)) if g.ops[o].stream == "net"):
+                assert not early[op.name] & 1
+
+
+def test_a_gated_product_never_starts_early():
+    g, _, _keep = _host_graph("NON_OVERLAP_LOCAL", 1, None)
+    qkv = next(op for op in g.ops if op.name == "L0.nb0.qkv")
+    qkv.after_start = [0]
+    assert not _early(g)["L0.nb0.qkv"] & 1
