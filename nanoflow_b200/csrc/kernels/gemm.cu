@@ -1447,8 +1447,9 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
 }
 
 // A shape measured at another number of rows (tuned_rows) says little about this call: it holds for calls with as many
-// 256-row groups of tiles, and the cost model chooses for the others. A shape tuned at 1024 rows took 50 us for
-// 48 x 10240 x 8192, where the weight takes 26.
+// 256-row groups of tiles, and the rules choose for the others. A shape tuned at 1024 rows took 50 us for 48 x 10240 x 8192,
+// where the weight takes 26. Up to 256 rows that is too coarse: a shape holds for as many tiles of 128 rows, and only where
+// the rules would not take the few-rows kernel, unless it was measured at exactly this number of rows.
 //
 // With keep_order a stopwatch must not decide where K is cut: a pick changes with the clock of the day, and the order of sums
 // with it. Shapes that leave K whole all add up in the order of k, so a tuned one of them takes the place of a whole-K shape of
@@ -1458,6 +1459,7 @@ nfk_gemm_params with_own_shape(const nfk_gemm_params& g) {
   if (g.tuned_rows <= 0) return p;
   p.tile_m = p.tile_n = p.cta_group = p.split_k = p.stream_k = 0;
   if ((g.M + 255) / 256 != (g.tuned_rows + 255) / 256) return p;
+  if (g.M <= 256 && g.M != g.tuned_rows && ((g.M + BM - 1) / BM != (g.tuned_rows + BM - 1) / BM || few_rows_takes(p))) return p;
   if (g.keep_order != 0) {
     const Shape own = choose_shape(p, g.epilogue == NFK_EPI_SWIGLU);
     if (own.split_k > 1 || own.stream_k || g.split_k > 1 || g.stream_k == 1) return p;
@@ -1546,6 +1548,7 @@ extern "C" int nfk_gemm_describe(const nfk_gemm_params* given, nfk_gemm_plan* ou
   out->tail_max_pieces = sk.max_pieces;
   out->stages = geo.stages;
   out->smem_bytes = geo.smem_bytes;
+  out->few_rows = few_rows_takes(*g) ? 1 : 0;
   return NF_OK;
 }
 

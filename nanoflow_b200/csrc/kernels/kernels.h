@@ -93,8 +93,8 @@ typedef struct nfk_gemm_params {
                         // as given, 0 = choose); 2 = the tile kernel
   int weights_ready;    // B and B2 are complete (weights of a loaded model): with early_start they may be fetched while the
                         // launches before this one, back to the last that was not early, still run
-  int tuned_rows;       // rows that the pinned shape was measured at: a call with another number of 256-row groups leaves
-                        // the shape to the cost model (0 = the shape holds for every M)
+  int tuned_rows;       // rows that the pinned shape was measured at: calls of other sizes leave the shape to the rules (another
+                        // number of 256-row groups, up to 256 rows of 128-row tiles; 0 = the shape holds for every M)
   int keep_order;       // 1 = the order of sums follows from M, N and K alone, by the earlier rules: shapes and kernel by these,
                         // a tuned shape (tuned_rows > 0) only where it and the rules' shape leave K whole (layer-list models:
                         // a recurrent state carries a change of rounding on)
@@ -113,6 +113,7 @@ typedef struct nfk_gemm_plan {
   int tiles, workers, num_kb;          // output tiles, CTAs (or CTA pairs), 64-wide k-blocks
   int tail_first_tile, tail_range_kb, tail_max_pieces;   // stream-K tail (tail_range_kb 0 = none)
   int stages, smem_bytes;
+  int few_rows;                        // 1 = the call goes to the few-rows kernel, and the rest is what the tile kernel would do
 } nfk_gemm_plan;
 int nfk_gemm_describe(const nfk_gemm_params* p, nfk_gemm_plan* out);
 

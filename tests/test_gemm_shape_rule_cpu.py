@@ -17,11 +17,23 @@ def _plan(M, N, K, **f):
 
 
 @pytest.mark.parametrize("tuned,M,holds", [(0, 48, True), (2048, 2048, True), (2048, 1793, True), (2048, 1792, False), (2048, 48, False),
-                                           (256, 256, True), (256, 1, True), (256, 257, False), (100, 129, True)])
+                                           (256, 256, True), (256, 1, False), (256, 128, False), (256, 129, True), (256, 257, False),
+                                           (100, 129, False), (128, 100, True), (128, 90, False), (90, 90, True)])
 def test_a_tuned_shape_holds_for_its_own_number_of_row_groups(tuned, M, holds):
+    """Up to 256 rows, where a tile of 128 rows is much: for its own number of such tiles, and not where the few-rows kernel
+    takes the call unless the shape was measured at this very number of rows."""
     pin = dict(tile_m=1, tile_n=192, cta_group=1, split_k=1, stream_k=2)
     got = _plan(M, 10240, 8192, tuned_rows=tuned, **pin)
     assert got == (_plan(M, 10240, 8192, **pin) if holds else _plan(M, 10240, 8192))
+    assert got["few_rows"] == (not holds and M <= 96)
+
+
+@pytest.mark.parametrize("M", [1, 24, 96])
+@pytest.mark.parametrize("swiglu", [0, 1])
+def test_a_small_batch_takes_the_few_rows_kernel_whatever_the_dense_batch(M, swiglu):
+    pin = dict(tile_m=1, tile_n=256, cta_group=2, split_k=1, stream_k=1)
+    for tuned in (256, 1024, 2048):
+        assert _plan(M, 28672, 8192, epilogue=swiglu, tuned_rows=tuned, **pin)["few_rows"]
 
 
 @pytest.mark.parametrize("swiglu", [0, 1])
