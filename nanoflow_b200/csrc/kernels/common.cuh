@@ -337,7 +337,8 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
 // CTA of that one has called let_next_start() (or has ended). await_previous() returns when all earlier work is complete and
 // visible; every CTA calls it before its first access to memory that earlier work writes or reads, and no CTA ends
 // without having called it, so that completion stays transitive along a stream. A kernel that allocates tensor memory
-// calls let_next_start() after that: the next kernel cannot then take columns that it still needs.
+// calls let_next_start() after that: the next kernel cannot then take columns that it still needs. A kernel that waits for
+// flags which another stream's or another GPU's kernel raises never calls it.
 //
 // Who launches early is the graph's choice (early_start of an op's parameters): CTAs that have started early hold threads,
 // registers and shared memory of their SM while they wait, and where another stream's kernel is to run beside the one that

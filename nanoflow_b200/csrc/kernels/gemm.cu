@@ -422,7 +422,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  let_next_start();
+  // With gated input this kernel waits for another stream's collective, whose CTAs still need their places on the SMs: the
+  // next kernel starts when this one has ended.
+  if (p.gate_flags == nullptr) let_next_start();
   await_previous();
 
   if (warp == 0) {

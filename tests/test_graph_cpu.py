@@ -11,13 +11,14 @@ from nanoflow_b200.utils import depcheck
 
 
 def _host_graph(pipeline_type, tp, nano, gbs=48, fuse_rs=False, net_streams=1, fake_wire=0.0, attn_overlap=False,
-                cross_layer=False, o_allgather=(), by_copy=False):
+                cross_layer=False, o_allgather=(), by_copy=False, gate=False):
     cfg = builtin_config("tiny", gpu_num=tp, global_batch_size=gbs, pipeline_type=pipeline_type, nanobatch_sizes=nano)
     m, e = cfg.model, cfg.engine
     e.fuse_gemm_rs = fuse_rs
     e.net_streams = net_streams
     e.attn_overlap = attn_overlap
     e.cross_layer_pipeline = cross_layer
+    e.gate_gemm = gate
     e.o_allgather_nanos = list(o_allgather)
     e.max_batch_size = gbs
     fw = random_full_weights(m, seed=0)
@@ -542,8 +543,15 @@ def test_nothing_waits_in_the_places_of_another_streams_kernel(tp, nano, pipelin
                 assert not early[op.name] & 1
 
 
-def test_a_gated_product_never_starts_early():
-    g, _, _keep = _host_graph("NON_OVERLAP_LOCAL", 1, None)
-    qkv = next(op for op in g.ops if op.name == "L0.nb0.qkv")
-    qkv.after_start = [0]
-    assert not _early(g)["L0.nb0.qkv"] & 1
+@pytest.mark.parametrize("nano", [[16, 32], [16, 16, 16]])
+def test_a_gated_product_neither_starts_early_nor_lets_its_successor(nano):
+    """It waits for a collective that may not have found its places on the SMs yet."""
+    g, _, _keep = _host_graph("PLLM", 2, nano, gate=True)
+    early, gated, last = _early(g), {i for i, op in enumerate(g.ops) if op.gated}, {}
+    assert len(gated) >= 4
+    for i, op in enumerate(g.ops):
+        if i in gated or last.get(op.stream) in gated:
+            assert not early.get(op.name, 0) & 1, op.name
+        if i in gated:
+            assert not early[op.name], op.name
+        last[op.stream] = i
