@@ -314,7 +314,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
          cta_group: int = 0, stream_k: int = 0, norm_w: Optional[torch.Tensor] = None,
          norm_out: Optional[torch.Tensor] = None, norm_eps: float = 1e-5,
          gate_flags: Optional[torch.Tensor] = None, gate_epoch: int = 0, gate_nranks: int = 1,
-         rows_kernel: int = 0, keep_order: bool = False) -> torch.Tensor:
+         rows_kernel: int = 0, keep_order: bool = False, weights_ready: bool = False,
+         early_start: int = 0) -> torch.Tensor:
     """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) (+ beta * residual). Rows may be strided.
 
     With ``norm_w`` / ``norm_out`` the call also leaves ``norm_out = RMSNorm(out) * norm_w`` (from the
@@ -327,7 +328,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     128-row block, until words [block, 0:gate_nranks] have reached ``gate_epoch``.
 
     ``rows_kernel`` 1 / 2 asks for / rules out the kernel for few rows (0 = the launcher's rule).
-    ``keep_order``: shapes by the earlier rules (see kernels.h)."""
+    ``keep_order``: shapes by the earlier rules (see kernels.h). ``early_start`` (EARLY_*): the kernels may start while the one
+    before them on the stream ends; with ``weights_ready`` the caller states that ``w`` was complete long before."""
     _bf16(a, "a"); _bf16(w, "w")
     M, K = a.shape
     N, K2 = w.shape
@@ -360,6 +362,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     p.smem_budget_kb = smem_budget_kb
     p.cta_group = cta_group
     p.rows_kernel, p.keep_order = rows_kernel, int(keep_order)
+    p.weights_ready, p.early_start = int(weights_ready), early_start
     p.stream_k = stream_k
     if norm_w is not None:
         _bf16(norm_w, "norm_w"); _bf16(norm_out, "norm_out")
@@ -409,7 +412,7 @@ def gemm_swiglu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *,
                 workspace: Optional[torch.Tensor] = None, cta_group: int = 0,
                 stream_k: int = 0, smem_budget_kb: int = 0, gate_flags: Optional[torch.Tensor] = None,
                 gate_epoch: int = 0, gate_nranks: int = 1, rows_kernel: int = 0,
-                keep_order: bool = False) -> torch.Tensor:
+                keep_order: bool = False, weights_ready: bool = False, early_start: int = 0) -> torch.Tensor:
     """out[M,F] = silu(a @ w_gate^T) * (a @ w_up^T), gate and up products fused in one kernel.
     ``gate_flags``: as in :func:`gemm`."""
     _bf16(a, "a"); _bf16(w_gate, "w_gate"); _bf16(w_up, "w_up")
@@ -433,6 +436,7 @@ def gemm_swiglu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *,
     p.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     p.cta_group = cta_group
     p.rows_kernel, p.keep_order = rows_kernel, int(keep_order)
+    p.weights_ready, p.early_start = int(weights_ready), early_start
     p.stream_k = stream_k
     p.smem_budget_kb = smem_budget_kb
     _set_gate(p, gate_flags, gate_epoch, gate_nranks, M)

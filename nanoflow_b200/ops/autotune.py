@@ -19,7 +19,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
-from . import gemm, gemm_plan, gemm_swiglu
+from . import EARLY_FIRST, EARLY_FURTHER, gemm, gemm_plan, gemm_swiglu
 
 KEYS = ("tile_m", "tile_n", "cta_group", "split_k", "stream_k")
 AUTO: Dict[str, int] = dict(tile_m=0, tile_n=0, cta_group=0, split_k=0, stream_k=0)
@@ -78,9 +78,10 @@ def same_order(cands: List[Dict[str, int]], M: int, N: int, K: int, swiglu: bool
 def tune_gemm(a: torch.Tensor, weights: Sequence[torch.Tensor], out: torch.Tensor, *,
               weights_up: Optional[Sequence[torch.Tensor]] = None, residual: Optional[torch.Tensor] = None,
               bias: Optional[torch.Tensor] = None, num_ctas: int = 0, workspace: Optional[torch.Tensor] = None,
-              smem_budget_kb: int = 0, iters: int = 4, passes: int = 2, keep_order: bool = False) -> Dict[str, object]:
+              smem_budget_kb: int = 0, iters: int = 4, passes: int = 2, keep_order: bool = False, early: bool = False) -> Dict[str, object]:
     """Time every candidate on ``a @ weights[i]^T`` (cycling through ``weights``) and return
     ``{"best": kwargs, "us": best time, "auto_us": time of the cost model's own choice, "table": [...]}``.
+    ``early``: launched as in a pipeline whose kernels start while the one before them ends (with the weights there).
     Candidates the launcher rejects (shape not built, workspace too small) are skipped, and with ``keep_order`` those that
     would add up in another order than the cost model's choice."""
     M, K = a.shape
@@ -92,15 +93,17 @@ def tune_gemm(a: torch.Tensor, weights: Sequence[torch.Tensor], out: torch.Tenso
     best_us = [float("inf")] * len(cands)
     layer = 0
 
+    how = dict(keep_order=keep_order, weights_ready=early, early_start=EARLY_FIRST | EARLY_FURTHER if early else 0)
+
     def run(c, i):
         w = weights[i % len(weights)]
         if swiglu:
             gemm_swiglu(a, w, weights_up[i % len(weights)], out=out, num_ctas=num_ctas, workspace=workspace,
                         smem_budget_kb=smem_budget_kb, tile_m=c["tile_m"], tile_n=c["tile_n"],
-                        cta_group=c["cta_group"], stream_k=c["stream_k"], keep_order=keep_order)
+                        cta_group=c["cta_group"], stream_k=c["stream_k"], **how)
         else:
             gemm(a, w, out=out, residual=residual, bias=bias, num_ctas=num_ctas, workspace=workspace,
-                 smem_budget_kb=smem_budget_kb, keep_order=keep_order, **c)
+                 smem_budget_kb=smem_budget_kb, **how, **c)
 
     for _ in range(passes):
         for ci, c in enumerate(cands):

@@ -231,7 +231,7 @@ class Engine:
                     done[(key, M)] = autotune.tune_gemm(
                         a[:M], ws, out[:M], weights_up=ups, residual=None if resid is None else resid[:M],
                         bias=bias, num_ctas=budget, workspace=b.gemm_ws,
-                        smem_budget_kb=gemm_smem_budget_kb(e, w.tp))
+                        smem_budget_kb=gemm_smem_budget_kb(e, w.tp), early=not e.overlap)
                 r = done[(key, M)]
                 e.gemm_shapes[name] = dict(r["best"], rows=M)
                 self.gemm_tuning[name] = dict(M=M, best=r["best"], us=r["us"], auto_us=r["auto_us"])

@@ -509,7 +509,7 @@ class LayerListEngine(Engine):
         if d32 is not None:
             p.D32, p.ld32, p.f32_col0 = _ptr(d32), d32.stride(0), f32_col0
         p.groups, p.group_k = groups, group_k
-        p.status, p.weights_ready, p.keep_order = _ptr(self.bufs.status), 1, 1
+        p.status, p.keep_order = _ptr(self.bufs.status), 1
         if self.gemm_ws is not None:
             p.workspace, p.workspace_bytes = _ptr(self.gemm_ws), self.gemm_ws.numel() * 4
         shape = self.eng.gemm_shapes.get(key)
@@ -869,7 +869,7 @@ class LayerListEngine(Engine):
                 sig = (key, n, wt.shape[1], up is not None)
                 if sig not in done:
                     done[sig] = autotune.tune_gemm(a, [wt], dst, weights_up=None if up is None else [up], workspace=self.gemm_ws,
-                                                    keep_order=True)
+                                                    keep_order=True, early=not self.eng.overlap)
                 res = done[sig]
                 self.eng.gemm_shapes[name] = dict(res["best"], rows=T)
                 self.gemm_tuning[name] = dict(M=T, best=res["best"], us=res["us"], auto_us=res["auto_us"])

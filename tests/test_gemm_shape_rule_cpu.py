@@ -2,6 +2,7 @@
 from ctypes import byref, c_void_p
 
 import pytest
+import torch
 
 from nanoflow_b200 import ops
 from nanoflow_b200.ops import autotune
@@ -70,3 +71,22 @@ def test_no_pick_moves_the_cut_of_k_where_the_order_is_kept(N, K, swiglu):
     own = _cut(ops.gemm_plan(T, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True))
     for c in offered:
         assert c == autotune.AUTO or (own == 1 and _cut(ops.gemm_plan(T, N, K, swiglu=swiglu, workspace_bytes=ws, keep_order=True, **c)) == 1)
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_the_tuner_times_what_the_pipeline_launches(monkeypatch, swiglu, early):
+    """Engines state that their weights are there, and kernels in line start early: so do the timed ones."""
+    calls = []
+
+    class Event:
+        def __init__(self, enable_timing=True): pass
+        record = synchronize = lambda self: None
+        elapsed_time = lambda self, other: 1.0
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(autotune, "gemm_swiglu" if swiglu else "gemm", lambda *a, **kw: calls.append(kw))
+    a, w, out = torch.zeros(300, 128), torch.zeros(256, 128), torch.zeros(300, 256)
+    r = autotune.tune_gemm(a, [w], out, weights_up=[w] if swiglu else None, early=early)
+    assert r["best"] == autotune.AUTO and calls
+    assert all(kw["weights_ready"] == early and kw["early_start"] == (3 if early else 0) for kw in calls)
