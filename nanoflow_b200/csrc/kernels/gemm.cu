@@ -1324,12 +1324,22 @@ bool few_rows_takes(const nfk_gemm_params& g) {
   if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
   if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
   if (g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0 || g.workspace == nullptr) return false;
-  // Measured (4096 to 28672 columns of K, us, tile kernel with its best shape -> this one). Gated: 48 rows 54 -> 46 and
-  // 170 -> 150, 192 rows 75 -> 68 and 212 -> 208, 333 rows 109 -> 110. Linear: 48 rows 17 -> 16, 81 -> 77; 96 rows 42 -> 39,
-  // 34 -> 31, 128 rows 16 -> 19, 93 -> 88. Very many tiles (an output head, 1002): 1 row 179 -> 156, 48 rows 170 -> 170,
-  // 96 rows 174 -> 199: the tokens that each tile stages beside its weights.
-  if (g.epilogue == NFK_EPI_SWIGLU) return g.M <= 256;
-  return g.M <= (g.N <= 65536 ? 96 : 48);
+  // Measured in a chain with a small kernel between products, cold weights, this kernel fetching weights early (us, tile kernel
+  // with its own rule -> this one). What it loses by is the tokens that each CTA stages beside its weights.
+  //   Linear: 4096 x 4096 at 48 rows 14.1 -> 12.8, 96 16.2 -> 17.0; 8192 x 8192 at 96 35.1 -> 31.9; 32000 x 8192 at 96
+  //   89.5 -> 91.0; 128256 x 4096 at 48 173 -> 167, at 96 174 -> 199. With fewer CTAs than SMs (1280 x 8192: 80) 64 rows
+  //   16.7 -> 16.4, 96 rows 17.5 -> 19.8.
+  //   Gated, all tiles at once (two CTAs on an SM): 14336 x 4096 at 112 rows 75 -> 54, 192 93 -> 66, 240 99 -> 73; at 256, where
+  //   the tile kernel's rows are full, 73.5 -> 75.2, 18944 x 3584 72 -> 77, 2048 x 4096 28 -> 35. Very few tiles (1024 x 4096,
+  //   64 CTAs): 160 rows 21.8 -> 21.8, 192 21.9 -> 27.1.
+  //   Gated, more than one round: 28672 x 8192 at 112 rows 187 -> 177, 144 214 -> 197, 192 216 -> 222, 256 211 -> 247; 22016 x 8192
+  //   at 112 168 -> 166, 128 159 -> 172, 144 168 -> 172, 192 171 -> 204.
+  const int groups = g.groups > 1 ? g.groups : 1;
+  const bool gated = g.epilogue == NFK_EPI_SWIGLU;
+  const int ctas = n_block_count(groups, g.N / groups, gated ? 64 : 128);    // before K is cut
+  if (!gated) return g.M <= (g.N > 65536 ? 48 : 8 * ctas < sm_count() ? 64 : 96);
+  if (ctas > 2 * sm_count()) return g.M <= 144 && g.M != 128;
+  return g.M <= (8 * ctas < sm_count() ? 160 : 255);
 }
 
 int few_rows(const nfk_gemm_params& g, cudaStream_t stream) {

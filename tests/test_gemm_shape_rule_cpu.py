@@ -90,3 +90,13 @@ def test_the_tuner_times_what_the_pipeline_launches(monkeypatch, swiglu, early):
     r = autotune.tune_gemm(a, [w], out, weights_up=[w] if swiglu else None, early=early)
     assert r["best"] == autotune.AUTO and calls
     assert all(kw["weights_ready"] == early and kw["early_start"] == (3 if early else 0) for kw in calls)
+
+
+@pytest.mark.parametrize("N,K,swiglu,last,not_at", [
+    (4096, 4096, 0, 96, ()), (1280, 8192, 0, 64, ()), (32000, 8192, 0, 96, ()), (128256, 4096, 0, 48, ()),
+    (14336, 4096, 1, 255, ()), (18944, 3584, 1, 255, ()), (2048, 4096, 1, 255, ()), (1024, 4096, 1, 160, ()),
+    (22016, 8192, 1, 144, (128,)), (28672, 8192, 1, 144, (128,))])
+def test_the_few_rows_kernel_gets_the_sizes_at_which_it_is_faster(N, K, swiglu, last, not_at):
+    """The lines that the measurements beside the rule give (148 SMs)."""
+    for M in (1, 16, 48, 64, 80, 96, 112, 127, 128, 129, 144, 145, 160, 192, 255, 256, 257, 300):
+        assert _plan(M, N, K, epilogue=swiglu)["few_rows"] == (M <= last and M not in not_at), M
