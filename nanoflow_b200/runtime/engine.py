@@ -42,6 +42,27 @@ GEMM_WS_BYTES = 160 << 20      # fp32 partial sums of split-K / stream-K-tail GE
 DECODE_SPLIT_ROWS = 8192       # workspace rows (request x q head) reserved for split-KV decode
 
 
+def decode_split(pages: np.ndarray, q_heads: int, kv_heads: int, ctas: int, fixed: int = 0):
+    """Pages per work item (0 = a request's whole context) and most items per request of one decode-attention launch, for
+    requests of ``pages`` pages on ``ctas`` CTAs; ``fixed`` > 0: pages per item as configured.
+
+    A launch deals (request, KV head, chunk) items to its CTAs. Contexts are cut where the longest is more than a CTA's share
+    of the launch's pages, so that it would still run when the other CTAs are done: into chunks of two thirds of a share, but
+    of several pages per warp, since an item costs some 4 us besides its pages. 24 contexts of 100 to 4800 tokens, 8 KV heads,
+    two CTAs per SM: whole 64 us, a quarter of the longest (what filled the SMs at equal lengths) 55, this 35; 48 of 200 to
+    3000: 90, 64, 58; 256 of 200 to 2000: whole 152, any cut more."""
+    if not len(pages) or len(pages) * q_heads > DECODE_SPLIT_ROWS:
+        return 0, 1
+    longest, cp = int(pages.max()), fixed
+    if cp <= 0:
+        share = math.ceil(int(pages.sum()) * kv_heads / ctas)
+        if longest <= max(16, share):
+            return 0, 1
+        cp = max(8 if share <= 8 else 16, math.ceil(share * 2 / 3), math.ceil(longest / DECODE_MAX_CHUNKS))
+    mc = max(1, math.ceil(longest / cp))
+    return (cp, mc) if mc <= DECODE_MAX_CHUNKS else (0, 1)
+
+
 class MetaLayout:
     """Offsets (int32 words) of every per-iteration array inside one contiguous metadata block."""
 
@@ -193,6 +214,9 @@ class Engine:
         if e.autotune_gemm:
             self._autotune_gemms()
         self.graph: OpGraph = build_graph(m, e, weights, self.bufs, self.coll, io)
+        # CTAs that a nano-batch's decode attention is launched with (0 in the op = two per SM)
+        budget = {op.nano: op.params.num_ctas for op in self.graph.ops if op.name.endswith(".attn_decode")}
+        self.decode_ctas = [budget[k] or 2 * ops.sm_count(self.device) for k in range(len(self.nano_sizes))]
 
     # ---- GEMM shapes --------------------------------------------------------------------------------
     def _autotune_gemms(self) -> None:
@@ -317,32 +341,10 @@ class Engine:
 
     def _stage_model(self, plan: BatchPlan, put, sym: Dict[str, int]) -> None:
         """Metadata arrays and symbols that only this family's ops use."""
-        cp, mc = self._decode_split(plan)
-        sym["decode_chunk_pages"], sym["decode_max_chunks"] = cp, mc
-
-    def _decode_split(self, plan: BatchPlan):
-        """Pages per work item of the decode attention (0 = a request's whole context) and most items per request.
-
-        A launch deals (request, KV head, chunk) items to two CTAs per SM. Contexts are cut where the longest is more than
-        a CTA's share of all pages, so that it would still run when the other CTAs are done: into chunks of two thirds of
-        a share, but of several pages per warp, since an item costs some 4 us besides its pages. 24 contexts of 100 to 4800
-        tokens, 8 KV heads: whole 64 us, a quarter of the longest (what filled the SMs at equal lengths) 55, this 35;
-        48 of 200 to 3000: 90, 64, 58; 256 of 200 to 2000: whole 152, any cut more."""
-        counts = [np.diff(plan.kv_indptr[nb.dec_begin:nb.dec_begin + nb.dec_count + 1]) for nb in plan.nano if nb.dec_count]
-        if not counts:
-            return 0, 1
-        longest, pages = max(int(c.max()) for c in counts), sum(int(c.sum()) for c in counts)
-        if self.eng.decode_chunk_pages > 0:
-            cp = self.eng.decode_chunk_pages
-        else:
-            share = math.ceil(pages * self.model.kv_heads_local / (2 * ops.sm_count(self.device)))
-            if longest <= max(16, share):
-                return 0, 1
-            cp = max(8 if share <= 8 else 16, math.ceil(share * 2 / 3), math.ceil(longest / DECODE_MAX_CHUNKS))
-        mc = max(1, math.ceil(longest / cp))
-        if mc > DECODE_MAX_CHUNKS or plan.num_decode * self.model.q_heads_local > DECODE_SPLIT_ROWS:
-            return 0, 1
-        return cp, mc
+        for k, nb in enumerate(plan.nano):
+            pages = np.diff(plan.kv_indptr[nb.dec_begin:nb.dec_begin + nb.dec_count + 1])
+            sym[f"nb{k}_chunk_pages"], sym[f"nb{k}_max_chunks"] = decode_split(
+                pages, self.model.q_heads_local, self.model.kv_heads_local, self.decode_ctas[k], self.eng.decode_chunk_pages)
 
     def run_async(self, timed: bool = False) -> None:
         st = self._staged

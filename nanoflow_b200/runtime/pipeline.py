@@ -174,8 +174,8 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
     nb_dec0 = [g.symbol(f"nb{k}_dec_begin") for k in range(nn)]
     nb_decn = [g.symbol(f"nb{k}_dec_count") for k in range(nn)]
     nb_items = [g.symbol(f"nb{k}_items") for k in range(nn)]
-    chunk_pages = g.symbol("decode_chunk_pages")
-    max_chunks = g.symbol("decode_max_chunks")
+    nb_chunk_pages = [g.symbol(f"nb{k}_chunk_pages") for k in range(nn)]
+    nb_max_chunks = [g.symbol(f"nb{k}_max_chunks") for k in range(nn)]
 
     m = bufs.meta
     # ---- prologue: ids (device feedback) + embedding into residual buffer 0 ------------------------
@@ -309,8 +309,8 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
         dp.workspace = _ptr(bufs.decode_ws)
         dec_kernel = "nfk_attn_decode_tma" if (eng.decode_impl == "tma" and hd == 128) else "nfk_attn_decode"
         dec = g.add(f"L{l}.nb{k}.attn_decode", dp, S("attn"), deps=[ro], kernel=dec_kernel,
-                    dyn=[("req_begin", nb_dec0[k]), ("req_count", nb_decn[k]), ("chunk_pages", chunk_pages),
-                         ("max_chunks", max_chunks)], layer=l, nano=k)
+                    dyn=[("req_begin", nb_dec0[k]), ("req_count", nb_decn[k]), ("chunk_pages", nb_chunk_pages[k]),
+                         ("max_chunks", nb_max_chunks[k])], layer=l, nano=k)
         pp = attn_params()
         pp.num_ctas = budget.get("attn_prefill", 0)
         pp.items = _ptr(bufs.nano_items[k])

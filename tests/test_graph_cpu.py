@@ -1,5 +1,6 @@
 """Static checks of the op graph on CPU: every pipeline variant builds, dependencies only point
 backwards, and no two ops that touch the same bytes (one of them writing) are left unordered."""
+import numpy as np
 import pytest
 import torch
 
@@ -555,3 +556,39 @@ def test_a_gated_product_neither_starts_early_nor_lets_its_successor(nano):
         if i in gated:
             assert not early[op.name], op.name
         last[op.stream] = i
+
+
+def test_decode_chunks_follow_each_launchs_own_share():
+    """Two nano-batches are two launches: half the pages each, and each cuts as if it were alone. Fewer CTAs have larger shares."""
+    from nanoflow_b200.runtime.engine import decode_split
+    pages = np.array([300] + [7 + 13 * (i % 20) for i in range(23)])
+    alone = decode_split(pages, 32, 8, 296)
+    share = -(-int(pages.sum()) * 8 // 296)
+    assert alone == (max(16, -(-share * 2 // 3)), -(-300 // max(16, -(-share * 2 // 3))))
+    cfg_graph, _, _keep = _host_graph("NANOBATCH_LOCAL", 1, [16, 32])
+    fields = {op.nano: dict(op.dyn) for op in cfg_graph.ops if op.name.endswith("attn_decode")}
+    assert [fields[k]["chunk_pages"] for k in (0, 1)] == ["nb0_chunk_pages", "nb1_chunk_pages"]
+    assert [fields[k]["max_chunks"] for k in (0, 1)] == ["nb0_max_chunks", "nb1_max_chunks"]
+    wide, narrow = decode_split(pages, 32, 8, 296), decode_split(pages, 32, 8, 148)
+    assert narrow[0] > wide[0] or narrow == (0, 1)
+    assert decode_split(pages, 32, 8, 8) == (0, 1) and decode_split(np.array([], dtype=int), 32, 8, 296) == (0, 1)
+    assert decode_split(pages, 32, 8, 296, fixed=100) == (100, 3) and decode_split(pages, 32, 8, 296, fixed=2) == (0, 1)
+    assert decode_split(np.full(300, 40), 32, 8, 296) == (0, 1)
+
+
+@pytest.mark.parametrize("budget", [0, 96])
+def test_an_engine_cuts_per_nano_batch(budget):
+    import types
+    from nanoflow_b200.runtime import engine as E
+    nano = [types.SimpleNamespace(dec_begin=0, dec_count=12), types.SimpleNamespace(dec_begin=12, dec_count=12),
+            types.SimpleNamespace(dec_begin=24, dec_count=0)]
+    per = np.array([40] * 11 + [400] + [60] * 12)
+    plan = types.SimpleNamespace(nano=nano, kv_indptr=np.concatenate([[0], np.cumsum(per)]))
+    ctas = budget or 296
+    eng = types.SimpleNamespace(model=types.SimpleNamespace(q_heads_local=32, kv_heads_local=8), eng=types.SimpleNamespace(decode_chunk_pages=0),
+                                decode_ctas=[ctas] * 3)
+    sym = {}
+    E.Engine._stage_model(eng, plan, None, sym)
+    for k, p in enumerate((per[:12], per[12:], per[:0])):
+        assert (sym[f"nb{k}_chunk_pages"], sym[f"nb{k}_max_chunks"]) == E.decode_split(p, 32, 8, ctas)
+    assert sym["nb0_max_chunks"] > 1 and sym["nb2_chunk_pages"] == 0
