@@ -128,9 +128,10 @@ __device__ __forceinline__ DecodeRange decode_range(const nfk_attn_params& p, in
 
 // Chunks before each request (first_chunk[0 .. req_count]) by a scan of the block; returns their number.
 constexpr int kDecListed = 512;
+constexpr int kDecListBytes = (kDecListed + 1 + kDecThreads / 32) * 4;
 static_assert(kDecListed == 4 * kDecThreads, "four requests per thread");
 __device__ __forceinline__ int list_chunks(const nfk_attn_params& p, int* first_chunk) {
-  __shared__ int warp_sum_of[kDecThreads / 32];
+  int* warp_sum_of = first_chunk + kDecListed + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = threadIdx.x * 4;
   int n[4], mine = 0;
 #pragma unroll
@@ -170,8 +171,11 @@ __device__ __forceinline__ int list_chunks(const nfk_attn_params& p, int* first_
 
 // EXT: sink in the denominator, capped scores, distance bias, chunks, page lists that start inside the sequence, queries in
 // wider rows, probabilities as a bf16 pair (in an instantiation of its own).
-template <int HD, int ST, bool EXT>
-__global__ void __launch_bounds__(kDecThreads, EXT ? 2 : 3)
+// LIST: work items are the chunks that hold pages, from a list in shared memory behind the pipeline buffers.
+// Registers: two CTAs of 96 KB are all that fit an SM, so three stages at head_dim 128 need no cap for a third (with one, the
+// loop spilled 28 bytes), and a listed launch has two CTAs per SM; with two stages the cap leaves room for other kernels.
+template <int HD, int ST, bool EXT, bool LIST>
+__global__ void __launch_bounds__(kDecThreads, EXT || LIST || (HD == 128 && ST == 3) ? 2 : 3)
 attn_decode_kernel(nfk_attn_params p, int slot) {
   using Cfg = DecCfg<HD, ST>;
   constexpr int kDecStages = ST;
@@ -179,14 +183,13 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.q_heads / p.kv_heads;
   const int max_chunks = p.chunk_pages > 0 ? p.max_chunks : 1;
-  // Work items: (request, kv head, chunk). With chunks, only those that hold pages are listed, if the requests fit the list:
-  // requests of very different length then leave no run of empty items to walk through.
-  __shared__ int first_chunk[kDecListed + 1];
+  // Work items: (request, kv head, chunk). With the list requests of very different length leave no run of empty items to walk
+  // through.
+  int* first_chunk = reinterpret_cast<int*>(smem + Cfg::SMEM_BYTES);
   let_next_start();
   await_previous();
-  const bool listed = max_chunks > 1 && p.req_count <= kDecListed;
   long long total = static_cast<long long>(p.req_count) * p.kv_heads * max_chunks;
-  if (listed) total = static_cast<long long>(list_chunks(p, first_chunk)) * p.kv_heads;
+  if (LIST) total = static_cast<long long>(list_chunks(p, first_chunk)) * p.kv_heads;
   const __nv_bfloat16* qbase = reinterpret_cast<const __nv_bfloat16*>(p.q);
   const __nv_bfloat16* pool = reinterpret_cast<const __nv_bfloat16*>(p.kv_pool);
   __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(p.out);
@@ -202,7 +205,7 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
     if (threadIdx.x == 0) fetched = static_cast<long long>(gridDim.x) + atomicAdd(&counters[0], 1u);
     do {
     int chunk, kvh, bl;
-    if (listed) {
+    if (LIST) {
       const int entry = static_cast<int>(item / p.kv_heads);
       kvh = static_cast<int>(item) - entry * p.kv_heads;
       bl = 0;                                                 // last request that starts at or before the entry
@@ -644,14 +647,14 @@ int check_common(const nfk_attn_params* p, bool decode = false) {
   return NF_OK;
 }
 
-template <int HD, int ST, bool EXT>
-int launch_decode_st(const nfk_attn_params* p, cudaStream_t stream) {
-  using Cfg = DecCfg<HD, ST>;
+template <int HD, int ST, bool EXT, bool LIST>
+int launch_decode_form(const nfk_attn_params* p, cudaStream_t stream) {
+  constexpr int bytes = DecCfg<HD, ST>::SMEM_BYTES + (LIST ? kDecListBytes : 0);
   static bool attr_dev[kMaxDevices] = {false};   // the attribute is per device
   bool& attr = attr_dev[device_slot()];
   if (!attr) {
-    if (cudaFuncSetAttribute(attn_decode_kernel<HD, ST, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Cfg::SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_decode_kernel<HD, ST, EXT, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+        cudaSuccess)
       return NF_ERR_CUDA;
     attr = true;
   }
@@ -661,14 +664,24 @@ int launch_decode_st(const nfk_attn_params* p, cudaStream_t stream) {
   if (ctas > total) ctas = total;
   static std::atomic<unsigned int> launch_seq{0};
   const int slot = static_cast<int>(launch_seq.fetch_add(1u) % kDecodeCounterSlots);
-  cudaError_t e = launch_kernel(early_first(p->early_start), attn_decode_kernel<HD, ST, EXT>, static_cast<int>(ctas), kDecThreads,
-                                Cfg::SMEM_BYTES, stream, 1, *p, slot);
+  cudaError_t e = launch_kernel(early_first(p->early_start), attn_decode_kernel<HD, ST, EXT, LIST>, static_cast<int>(ctas),
+                                kDecThreads, bytes, stream, 1, *p, slot);
   if (e == cudaSuccess && p->chunk_pages > 0 && max_chunks > 1)
     e = launch_kernel(early_further(p->early_start), attn_decode_merge_kernel<HD>, p->req_count * p->q_heads, HD, 0, stream, 1,
                       *p);
   if (e == cudaSuccess) return NF_OK;
   (void)cudaGetLastError();
   return NF_ERR_CUDA;
+}
+
+// The list takes another 2 KB of shared memory: not where a launch has a CTA budget, since it may then share its SMs with a
+// GEMM's CTAs, whose 130 KB leave 96 KB and not a byte more (1 KB reserved for each CTA). The launch then has no static
+// shared memory either.
+static_assert(DecCfg<128, 3>::SMEM_BYTES + 1024 + (130 + 1) * 1024 <= 228 * 1024, "a decode CTA beside a GEMM CTA");
+template <int HD, int ST, bool EXT>
+int launch_decode_st(const nfk_attn_params* p, cudaStream_t stream) {
+  const bool list = p->chunk_pages > 0 && p->max_chunks > 1 && p->req_count <= kDecListed && p->num_ctas <= 0;
+  return list ? launch_decode_form<HD, ST, EXT, true>(p, stream) : launch_decode_form<HD, ST, EXT, false>(p, stream);
 }
 
 template <int HD>

@@ -32,8 +32,11 @@ def test_every_chunk_is_taken_once(lens, chunk_pages, max_chunks):
     args = dict(q_heads=qh, req_begin=0, req_count=B, status=st)
     ops.attn_decode(q, whole, pool, qo, kvp, kvi, last, **args)
     ops.attn_decode(q, out, pool, qo, kvp, kvi, last, chunk_pages=chunk_pages, workspace=ws, max_chunks=max_chunks, **args)
+    # with a CTA budget the launch keeps to its pipeline buffers and walks every (request, head, chunk) instead of a list
+    walked = torch.zeros_like(q)
+    ops.attn_decode(q, walked, pool, qo, kvp, kvi, last, chunk_pages=chunk_pages, workspace=ws, max_chunks=max_chunks, num_ctas=48, **args)
     ops.check_status(st, "decode")
     live = torch.tensor(lens, device="cuda") > 0
-    assert torch.isfinite(out[live].float()).all()
+    assert torch.isfinite(out[live].float()).all() and torch.equal(out[live], walked[live])
     # weights of at most 1 and values of up to 4.5 standard deviations: 2^-8 of both, rounding at the end included
     assert ((out - whole)[live].float().abs() <= 4.5 * 2 ** -7).all()
