@@ -1,11 +1,16 @@
 """The GEMM kernel for few rows (csrc/kernels/gemm_few_rows.cuh) against the same product in fp32.
 
 Tolerance: inputs are bf16, sums are fp32 and the result is rounded to bf16 once, so an element is off by at most half a
-bf16 step of its own size (2^-9) plus the fp32 rounding of its sum, K * 2^-24 of the sum of absolute products at worst."""
+bf16 step (8 significant bits: up to 2^-8 of its size) plus the fp32 rounding of its sum, K * 2^-24 of the sum of absolute
+products at worst."""
+from ctypes import byref, c_void_p
+
 import pytest
 import torch
 
 from nanoflow_b200 import ops
+from nanoflow_b200.ops import layer_list as forms
+from nanoflow_b200.runtime.graph import NormParams
 
 pytestmark = pytest.mark.gpu
 F32 = torch.float32
@@ -71,16 +76,71 @@ def test_gated(M, F, K):
         assert ((out.double() - ref).abs() <= ref.abs() * 2 ** -8 + (g.abs() + u.abs() + 1) * 2 ** -14).all()
 
 
-def test_same_sum_every_time_and_rows_independent():
-    """The order of the sum depends on neither the run nor the rows beside it, and strided rows are read and written."""
-    a, w = _data(128, 4096, 4096)
+@pytest.mark.parametrize("few,most", [(40, 128), (1, 17), (150, 256)])
+def test_same_sum_every_time_whatever_the_other_rows(few, most):
+    """The order of the sum depends on neither the run nor, within 1 ... 128 and within 129 ... 256 rows (one CTA per tile and
+    pairs of CTAs cut K differently), the number of rows beside a row; strided rows are read and written."""
+    a, w = _data(most, 4096, 4096)
     one = ops.gemm(a, w, rows_kernel=1)
     for _ in range(5):
         assert torch.equal(one, ops.gemm(a, w, rows_kernel=1))
-    wide, outw = torch.zeros(40, 4096 + 64, device="cuda").bfloat16(), torch.zeros(40, 4096 + 8, device="cuda").bfloat16()
-    wide[:, :4096] = a[:40]
+    assert torch.equal(one[:few], ops.gemm(a[:few], w, rows_kernel=1))
+    wide, outw = torch.zeros(few, 4096 + 64, device="cuda").bfloat16(), torch.zeros(few, 4096 + 8, device="cuda").bfloat16()
+    wide[:, :4096] = a[:few]
     ops.gemm(wide[:, :4096], w, out=outw[:, :4096], rows_kernel=1)
-    assert torch.equal(outw[:, :4096], ops.gemm(a[:40].contiguous(), w, rows_kernel=1)) and not outw[:, 4096:].any()
+    assert torch.equal(outw[:, :4096], one[:few]) and not outw[:, 4096:].any()
+
+
+@pytest.mark.parametrize("cg", [1, 2])
+@pytest.mark.parametrize("N,K", [(136, 64), (384, 192), (1000, 1096), (4096, 4096)])
+@pytest.mark.parametrize("M", [1, 40, 130])
+def test_weights_fetched_before_the_rows_are_there(M, N, K, cg):
+    """A chain of early launches: a norm writes the rows, the product has fetched weights meanwhile (fewer k-blocks than stages,
+    and more), and the next norm writes the rows again. The same bits as one launch after the other."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    _, w = _data(1, N, K)
+    _, up = _data(1, N, K, 1)
+    ones = torch.ones(K, device="cuda").bfloat16()
+    xs = [torch.randn(M, K, device="cuda", generator=g).bfloat16() for _ in range(8)]
+    want = []
+    for x in xs:
+        a = ops.rmsnorm(x, ones, 1e-5)
+        want.append((ops.gemm(a, w, rows_kernel=1, cta_group=cg), ops.gemm_swiglu(a, w, up, rows_kernel=1, cta_group=cg)))
+    a = torch.empty_like(xs[0])
+    got = [(torch.empty(M, N, device="cuda").bfloat16(), torch.empty(M, N, device="cuda").bfloat16()) for _ in xs]
+    stream, early = c_void_p(torch.cuda.current_stream().cuda_stream), dict(rows_kernel=1, cta_group=cg, weights_ready=True, early_start=3)
+    for _ in range(3):
+        for x, (lin, gated) in zip(xs, got):
+            p = NormParams(out=c_void_p(a.data_ptr()), x=c_void_p(x.data_ptr()), w=c_void_p(ones.data_ptr()), resid=c_void_p(0), rows=M,
+                           cols=K, eps=1e-5, early_start=1)
+            assert ops.lib().nfk_norm_p(byref(p), stream) == 0
+            ops.gemm(a, w, out=lin, **early)
+            ops.gemm_swiglu(a, w, up, out=gated, **early)
+    torch.cuda.synchronize()
+    assert all(torch.equal(p, q) and torch.equal(r, t) for (p, r), (q, t) in zip(want, got))
+
+
+@pytest.mark.parametrize("M", [1, 33, 200])
+@pytest.mark.parametrize("groups,n,K", [(1, 1000, 1096), (3, 200, 136), (8, 128, 64), (32, 512, 128)])
+def test_other_forms_of_the_epilogue(M, groups, n, K):
+    """Block-diagonal products, columns that leave as fp32, activations of finished columns."""
+    g = torch.Generator(device="cuda").manual_seed(groups)
+    a = torch.randn(M, groups * K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(groups * n, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    ref = torch.einsum("mgk,gnk->mgn", a.double().view(M, groups, K), w.double().view(groups, n, K)).reshape(M, -1)
+    size = torch.einsum("mgk,gnk->mgn", a.double().abs().view(M, groups, K), w.double().abs().view(groups, n, K)).reshape(M, -1)
+    kw = dict(groups=groups, group_k=K, k=K, rows_kernel=1)
+    _close(forms.gemm(a, w, **kw), ref, size, K)
+    for col0 in (0, 8, groups * n // 2 // 8 * 8):
+        f32 = torch.zeros(M, groups * n - col0 + 4, device="cuda")
+        out = forms.gemm(a, w, out32=f32, f32_col0=col0, **kw)
+        assert ((f32[:, :groups * n - col0].double() - ref[:, col0:]).abs() <= size[:, col0:] * (K * 2.0 ** -24)).all()
+        assert not f32[:, groups * n - col0:].any()
+        if col0:
+            _close(out, ref[:, :col0], size[:, :col0], K)
+    relu2 = torch.relu(ref) ** 2            # the square doubles the sum's relative error
+    got = forms.gemm(a, w, lin_act="relu2", **kw).double()
+    assert ((got - relu2).abs() <= relu2 * 2 ** -8 + 2.1 * ref.abs() * size * (K * 2.0 ** -24) + (size * (K * 2.0 ** -24)) ** 2).all()
 
 
 def test_rule_gives_small_batches_to_it_and_keeps_other_forms():
