@@ -326,11 +326,11 @@ residual_norm_kernel(nfk_residual_norm_params p) {
   }
 }
 
-// The plain step of most layers, x <- x + norm_in(y); h = norm_out(x), both norms of one kind and rows that the CTA's threads
-// cover exactly: the general kernel spends some 9400 instructions of a warp on a row of 4096 (choices, bounds, addresses of
-// the forms that it also knows), and issuing those is what bounds it. The same sums in the same order. x is requested with y,
-// weights ahead of the sums they follow. 1840 x 4096 bf16, layer norms: 30.9 -> 20.6 us (4.4 TB/s); RMS: 28.7 -> 18.4; 96
-// rows: 7.9 -> 4.5.
+// The plain step of most layers, x <- x + norm_in(y); h = norm_out(x), both norms of one kind and rows of 1024, 2048, 4096 or
+// 8192 columns, which the CTA's threads cover exactly (other multiples of 1024 stay with the general kernel). That one spends
+// some 9400 instructions of a warp on a row of 4096 (choices, bounds, addresses of the forms that it also knows), and issuing
+// those is what bounds it. The same sums in the same order. x is requested with y, weights ahead of the sums they follow.
+// 1840 x 4096 bf16, layer norms: 30.9 -> 20.6 us (4.4 TB/s); RMS: 28.7 -> 18.4; 96 rows: 7.9 -> 4.5.
 template <int NV, bool LAYER>
 __device__ __forceinline__ void plain_norm(float4 (&v)[NV], const float4 (&w)[NV], const float* b, float inv_n, float eps, float* red) {
   if (LAYER) {

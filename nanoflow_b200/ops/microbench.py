@@ -440,6 +440,14 @@ def small_case(which: str):
         ws = torch.zeros(160 << 20, dtype=torch.uint8, device="cuda")
         for _ in range(4):
             ops.gemm(a, w, out=out, workspace=ws)
+    elif which == "gemm_few":
+        # a decode batch through gate / up: the few-rows kernel, 235 MB of weights per call
+        M, N, K = 48, 14336, 4096
+        a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+        w, up = (torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02 for _ in range(2))
+        ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
+        for _ in range(4):
+            ops.gemm_swiglu(a, w, up, workspace=ws)
     elif which == "gemm_shapes":
         # one launch per kernel shape: CTA pair 256 wide, CTA pair 128 wide, single CTA 256 wide
         M, N, K = 4096, 8192, 8192
