@@ -157,7 +157,7 @@ struct DevParams {
   float* D32;
   long long ld32;
   int f32_col0;
-  int d32_wide;                     // rows of D32 start on 32-byte boundaries
+  int d32_wide, d_wide, part_wide;  // rows of D32 / D / the fp32 partial copies start on 32-byte boundaries
   GatedAct act;                     // gated epilogue
   int lin_act;                      // linear epilogue: NFK_LIN_*
   int groups, group_n, group_k;     // block-diagonal product (groups 1: an ordinary one)
@@ -202,6 +202,26 @@ __device__ __forceinline__ void add_bias8(float* v, const __nv_bfloat16* bias) {
   add_bias8(v, *reinterpret_cast<const uint4*>(bias));
 }
 
+// A thread holds columns of one row of its own, so a store of 16 bytes touches half a sector in each of 32 rows; 32 bytes make
+// it whole.
+__device__ __forceinline__ void store_32_bytes(void* dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f,
+                                               uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e),
+               "r"(f), "r"(g), "r"(h)
+               : "memory");
+}
+
+// Eight fp32 partial sums of one row.
+__device__ __forceinline__ void store_part8(float* dst, const float* v, bool wide) {
+  if (wide) {
+    store_32_bytes(dst, __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]),
+                   __float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
+    return;
+  }
+  __stcg(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
+  __stcg(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
+}
+
 // Eight finished columns of one row: bf16 to D, or fp32 to D32 from f32_col0 on (a multiple of 8).
 __device__ __forceinline__ void store_cols8(const DevParams& p, int row, int col, float* v) {
   if (p.lin_act != NFK_LIN_NONE) {
@@ -227,6 +247,18 @@ __device__ __forceinline__ void store_cols8(const DevParams& p, int row, int col
   o.z = pack_bf16x2(v[4], v[5]);
   o.w = pack_bf16x2(v[6], v[7]);
   *reinterpret_cast<uint4*>(p.D + static_cast<long long>(row) * p.ldd + col) = o;
+}
+
+// Sixteen finished columns of one row, of which the first eight or all lie before `col_end`.
+__device__ __forceinline__ void store_cols16(const DevParams& p, int row, int col, int col_end, float* v) {
+  if (p.d_wide && p.D32 == nullptr && p.lin_act == NFK_LIN_NONE && (col & 15) == 0 && col + 8 < col_end) {
+    store_32_bytes(p.D + static_cast<long long>(row) * p.ldd + col, pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                   pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]), pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]),
+                   pack_bf16x2(v[12], v[13]), pack_bf16x2(v[14], v[15]));
+    return;
+  }
+  store_cols8(p, row, col, v);
+  if (col + 8 < col_end) store_cols8(p, row, col + 8, v + 8);
 }
 
 // Tile index -> (m group, n block). Normally m groups vary fastest, so CTAs that run together share
@@ -622,10 +654,70 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const int row = (m_first + mt) * BM + q * 32 + lane;
           const bool row_ok = row < p.M;
           const long long row_local = static_cast<long long>(mt * BM + q * 32 + lane) * BN;
-          const __nv_bfloat16* crow =
-              (EPI == 0 && p.C != nullptr) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
           const NBlock nb = n_block(p, n_blk, OUT_BN);
           const int tile_col_end = nb.col_end;   // columns past it belong to the next tile
+          if constexpr (gated_epi(EPI)) {
+            // 16 gate and 16 up columns at a time: more would take 80 registers more, which a kernel beside this one needs. With
+            // the activations' chains overlapped (gated_acts) a tile of 128 x 128 leaves in 4 us instead of 22, under the next
+            // tile's loop; 14336 x 2 x 4096: 256 rows 71 -> 52 us, 333 100 -> 81, 700 163 -> 122, 1000 228 -> 164.
+#pragma unroll 1
+            for (int c = 0; c < OUT_BN; c += 16) {
+              uint32_t r[16], uu[16];
+              tmem_ld_32x32b_x16n(t_lane + mt * BN + c, r);
+              tmem_ld_32x32b_x16n(t_lane + mt * BN + BN / 2 + c, uu);
+              const int col = nb.col0 + c;
+              uint4 bias_w[EPI == kGatedBias ? 2 : 1], bias2_w[EPI == kGatedBias ? 2 : 1];
+              if constexpr (EPI == kGatedBias) {       // requested while the accumulators are on their way
+#pragma unroll
+                for (int g8 = 0; g8 < 2; ++g8) {
+                  const bool in = col + g8 * 8 < tile_col_end;
+                  bias_w[g8] = in ? *reinterpret_cast<const uint4*>(p.bias + col + g8 * 8) : make_uint4(0, 0, 0, 0);
+                  bias2_w[g8] = in ? *reinterpret_cast<const uint4*>(p.bias2 + col + g8 * 8) : make_uint4(0, 0, 0, 0);
+                }
+              }
+              tmem_ld_wait();
+              float gsum[16], usum[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                gsum[j] = __uint_as_float(r[j]);
+                usum[j] = __uint_as_float(uu[j]);
+              }
+              if (mode == 1) {
+                if (row_ok) {
+                  float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
+#pragma unroll
+                  for (int g8 = 0; g8 < 2; ++g8) {
+                    store_part8(own + c + g8 * 8, gsum + g8 * 8, p.part_wide);
+                    store_part8(own + BN / 2 + c + g8 * 8, usum + g8 * 8, p.part_wide);
+                  }
+                }
+                continue;
+              }
+              if constexpr (EPI == kGatedBias) {
+#pragma unroll
+                for (int g8 = 0; g8 < 2; ++g8) {
+                  add_bias8(gsum + g8 * 8, bias_w[g8]);
+                  add_bias8(usum + g8 * 8, bias2_w[g8]);
+                }
+              }
+              gated_acts<16>(gsum, usum, p.act);
+              if (row_ok && col < tile_col_end) store_cols16(p, row, col, tile_col_end, gsum);
+            }
+            continue;
+          }
+          // What the residual adds to a chunk of 32 columns is requested a chunk ahead: D may be C itself, so the compiler
+          // cannot move these loads over the stores of the chunk before, and each eight columns would wait for HBM.
+          const __nv_bfloat16* crow =
+              (EPI == 0 && p.C != nullptr && p.partial == nullptr && mode == 0 && row_ok) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
+          uint4 c_next[4];
+          auto request_c = [&](int c) {
+#pragma unroll
+            for (int g8 = 0; g8 < 4; ++g8) {
+              const int col = nb.col0 + c * 32 + g8 * 8;
+              c_next[g8] = col < tile_col_end ? *reinterpret_cast<const uint4*>(crow + col) : make_uint4(0, 0, 0, 0);
+            }
+          };
+          if (EPI == 0 && crow != nullptr) request_c(0);
 #pragma unroll 1
           for (int c = 0; c * 32 < OUT_BN; ++c) {
             uint32_t r[32];
@@ -634,76 +726,32 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int nval = tail16 ? 16 : 32;
             if (tail16) tmem_ld_32x32b_x16(t_lane + mt * BN + c * 32, r);
             else tmem_ld_32x32b_x32(t_lane + mt * BN + c * 32, r);
-            // biases are requested while the accumulators are on their way
-            uint4 bias_w[EPI == kGatedBias ? 4 : 1], bias2_w[EPI == kGatedBias ? 4 : 1];
-            if constexpr (EPI == kGatedBias) {
+            uint4 c_now[4];
+            if (EPI == 0 && crow != nullptr) {
 #pragma unroll
-              for (int g8 = 0; g8 < 4; ++g8) {
-                const int col = nb.col0 + c * 32 + g8 * 8;
-                bias_w[g8] = col < tile_col_end ? *reinterpret_cast<const uint4*>(p.bias + col) : make_uint4(0, 0, 0, 0);
-                bias2_w[g8] = col < tile_col_end ? *reinterpret_cast<const uint4*>(p.bias2 + col) : make_uint4(0, 0, 0, 0);
-              }
+              for (int g8 = 0; g8 < 4; ++g8) c_now[g8] = c_next[g8];
+              if ((c + 1) * 32 < OUT_BN) request_c(c + 1);
             }
-            if (gated_epi(EPI)) {
-              uint32_t uu[32];
-              if (tail16) tmem_ld_32x32b_x16(t_lane + mt * BN + BN / 2 + c * 32, uu);
-              else tmem_ld_32x32b_x32(t_lane + mt * BN + BN / 2 + c * 32, uu);
-              tmem_ld_wait();
-              float gsum[32], usum[32];
+            tmem_ld_wait();
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                gsum[j] = __uint_as_float(r[j]);
-                usum[j] = __uint_as_float(uu[j]);
+            for (int j = 0; j < 32; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
+            if (EPI == 0 && mode == 1) {
+              if (row_ok) {
+                float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
+#pragma unroll
+                for (int g8 = 0; g8 < 4; ++g8)
+                  if (g8 * 8 < nval) store_part8(own + c * 32 + g8 * 8, v + g8 * 8, p.part_wide);
               }
-              if (mode == 1) {
-                if (row_ok) {
-                  float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
-#pragma unroll
-                  for (int g4 = 0; g4 < 8; ++g4)
-                    if (g4 * 4 < nval) {
-                      __stcg(reinterpret_cast<float4*>(own + c * 32) + g4,
-                             make_float4(gsum[g4 * 4], gsum[g4 * 4 + 1], gsum[g4 * 4 + 2], gsum[g4 * 4 + 3]));
-                      __stcg(reinterpret_cast<float4*>(own + BN / 2 + c * 32) + g4,
-                             make_float4(usum[g4 * 4], usum[g4 * 4 + 1], usum[g4 * 4 + 2], usum[g4 * 4 + 3]));
-                    }
-                }
-                continue;
-              }
-              if constexpr (EPI == kGatedBias) {
-#pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8) {
-                  add_bias8(gsum + g8 * 8, bias_w[g8]);
-                  add_bias8(usum + g8 * 8, bias2_w[g8]);
-                }
-              }
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = gated_act(gsum[j], usum[j], p.act);
-            } else {
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
-              if (EPI == 0 && mode == 1) {
-                if (row_ok) {
-                  float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
-#pragma unroll
-                  for (int g4 = 0; g4 < 8; ++g4)
-                    if (g4 * 4 < nval)
-                      __stcg(reinterpret_cast<float4*>(own + c * 32) + g4,
-                             make_float4(v[g4 * 4], v[g4 * 4 + 1], v[g4 * 4 + 2], v[g4 * 4 + 3]));
-                }
-                continue;
-              }
+              continue;
             }
             const int col0 = nb.col0 + c * 32;
             if (EPI == 0 && p.partial != nullptr) {
               if (row_ok && col0 < tile_col_end) {
                 float* prow = p.partial + (static_cast<long long>(sg.ks) * p.M + row) * p.N;
 #pragma unroll
-                for (int g4 = 0; g4 < 8; ++g4) {
-                  const int col = col0 + g4 * 4;
-                  if (col < tile_col_end)
-                    *reinterpret_cast<float4*>(prow + col) =
-                        make_float4(v[g4 * 4], v[g4 * 4 + 1], v[g4 * 4 + 2], v[g4 * 4 + 3]);
+                for (int g8 = 0; g8 < 4; ++g8) {
+                  const int col = col0 + g8 * 8;
+                  if (col < tile_col_end) store_part8(prow + col, v + g8 * 8, p.part_wide);
                 }
               }
               continue;
@@ -773,24 +821,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
               for (int g8 = 0; g8 < 4; ++g8) {
                 const int col = col0 + g8 * 8;
-                if (col < tile_col_end) {  // N is a multiple of 8
+                if (EPI == 0 && col < tile_col_end) {  // N is a multiple of 8
                   float* vv = v + g8 * 8;
-                  if (EPI == 0) {
-                    if (p.bias != nullptr) add_bias8(vv, p.bias + col);
-                    if (crow != nullptr) {
-                      const uint4 cv = *reinterpret_cast<const uint4*>(crow + col);
-                      const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
+                  if (p.bias != nullptr) add_bias8(vv, p.bias + col);
+                  if (crow != nullptr) {
+                    const uint32_t cw[4] = {c_now[g8].x, c_now[g8].y, c_now[g8].z, c_now[g8].w};
 #pragma unroll
-                      for (int j = 0; j < 4; ++j) {
-                        const float2 f = unpack_bf16x2(cw[j]);
-                        vv[2 * j] += p.beta * f.x;
-                        vv[2 * j + 1] += p.beta * f.y;
-                      }
+                    for (int j = 0; j < 4; ++j) {
+                      const float2 f = unpack_bf16x2(cw[j]);
+                      vv[2 * j] += p.beta * f.x;
+                      vv[2 * j + 1] += p.beta * f.y;
                     }
                   }
-                  store_cols8(p, row, col, vv);
                 }
               }
+#pragma unroll
+              for (int g16 = 0; g16 < 2; ++g16)
+                if (col0 + g16 * 16 < tile_col_end) store_cols16(p, row, col0 + g16 * 16, tile_col_end, v + g16 * 16);
             }
           }
         }
@@ -1022,8 +1069,7 @@ sk_fixup_kernel(DevParams p, FixupGeom f) {
         add_bias8(a, p.bias + col);
         add_bias8(u, p.bias2 + col);
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) a[j] = gated_act(a[j], u[j], p.act);
+      gated_acts<8>(a, u, p.act);
     } else {
       if (p.bias != nullptr) add_bias8(a, p.bias + col);
       if (p.C != nullptr) {
@@ -1071,6 +1117,8 @@ inline DevParams dev_params(const nfk_gemm_params& g, bool linear) {
   p.ld32 = g.ld32;
   p.f32_col0 = g.f32_col0;
   p.d32_wide = (reinterpret_cast<uintptr_t>(g.D32) & 31) == 0 && g.ld32 % 8 == 0;
+  p.d_wide = (reinterpret_cast<uintptr_t>(g.D) & 31) == 0 && g.ldd % 16 == 0;
+  p.part_wide = (reinterpret_cast<uintptr_t>(g.workspace) & 31) == 0;      // rows of N (a multiple of 8) or bn floats
   p.act = GatedAct{g.act, g.act_limit, g.act_alpha, g.act_shift};
   p.lin_act = linear ? g.lin_act : NFK_LIN_NONE;
   p.groups = g.groups > 1 ? g.groups : 1;

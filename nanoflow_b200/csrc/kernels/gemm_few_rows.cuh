@@ -251,8 +251,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_cons
       if (p.bias != nullptr) add_bias8(v, p.bias + col);
       if (GATED) {
         if (p.bias != nullptr) add_bias8(u, p.bias2 + col);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = gated_act(v[j], u[j], p.act);
+        gated_acts<8>(v, u, p.act);
       } else if (p.C != nullptr) {
         const uint4 cv = *reinterpret_cast<const uint4*>(p.C + static_cast<long long>(row) * p.ldc + col);
         const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};

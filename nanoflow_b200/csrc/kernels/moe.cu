@@ -376,8 +376,13 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            v[j] = GATED ? gated_act(__uint_as_float(r[j]), __uint_as_float(u[j]), act) : __uint_as_float(r[j]);
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          if constexpr (GATED) {
+            float up[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) up[j] = __uint_as_float(u[j]);
+            gated_acts<32>(v, up, act);
+          }
           if (!GATED && p.lin_act != NFK_LIN_NONE) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = lin_act_of(v[j], p.lin_act);
