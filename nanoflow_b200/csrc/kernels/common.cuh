@@ -274,6 +274,9 @@ NF_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
 NF_DEVICE void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
+NF_DEVICE void st_shared_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // TMA load into this CTA's shared memory whose byte count is reported to a barrier that may live in
 // the peer CTA (`bar_cluster_addr` from mapa_shared). No multicast: each CTA fetches its own tiles.
 NF_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tm, uint32_t bar_cluster_addr, int x, int y) {

@@ -1127,7 +1127,10 @@ sk_fixup_kernel(DevParams p, FixupGeom f) {
   }
 }
 
+constexpr int kSmemMax = 227 * 1024;
+
 #include "gemm_few_rows.cuh"
+#include "gemm_split_cluster.cuh"
 
 // The caller's parameters as the kernels take them; geometry and work distribution are filled in by the launchers.
 inline DevParams dev_params(const nfk_gemm_params& g, bool linear) {
@@ -1173,8 +1176,6 @@ inline int rmsnorm_rows(const nfk_gemm_params& g, cudaStream_t stream) {
                           early_further(g.early_start) ? NFK_EARLY_FIRST : 0};
   return nfk_norm_p(&n, stream);
 }
-
-constexpr int kSmemMax = 227 * 1024;
 
 // Stream-K tail: with `tiles` tiles on `workers` workers, the tiles_dp tiles of the full waves are
 // whole-tile units; the k-blocks of the rest are cut into ranges of q (>= 8, so a piece is worth its
@@ -1405,11 +1406,100 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
   return NF_OK;
 }
 
+struct Shape {
+  int bn, mt, split_k, cg;
+  bool stream_k;
+};
+
+// Clusters of `size` CTAs of `kernel`, with all the shared memory of an SM each, that can be resident at once; asked once per
+// device, for which it also sets the kernel's attributes. `known` is that device's answer.
+template <class Kernel>
+int resident_clusters(Kernel* kernel, int size, int& known) {
+  if (known == 0) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    (void)cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaLaunchConfig_t qc = {};
+    qc.gridDim = dim3(sm_count() / size * size);
+    qc.blockDim = dim3(kGemmThreads);
+    qc.dynamicSmemBytes = kSmemMax;
+    cudaLaunchAttribute qa[1];
+    qa[0].id = cudaLaunchAttributeClusterDimension;
+    qa[0].val.clusterDim.x = size;
+    qa[0].val.clusterDim.y = 1;
+    qa[0].val.clusterDim.z = 1;
+    qc.attrs = qa;
+    qc.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &qc) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    known = n;
+  }
+  return known;
+}
+
+// What a B200 answers, for planning without one.
+constexpr int kResidentClusters[kSplitMaxCluster + 1] = {0, 148, 74, 47, 35, 27, 22, 18, 14};
+
+template <int CG>
+int resident_split_clusters(int size) {
+  static int known_dev[kMaxDevices][kSplitMaxCluster + 1] = {};
+  const int n = resident_clusters(gemm_split_cluster_kernel<CG>, size, known_dev[device_slot()][size]);
+  return n > 0 ? n : kResidentClusters[size];
+}
+
+// Calls that may run as clusters which add their parts of K among themselves. Those with a CTA or shared-memory budget keep the
+// launches that leave places beside them, and so does a norm of rows that are not contiguous.
+bool cluster_forms(const nfk_gemm_params& g) {
+  return g.rows_kernel != 3 && g.epilogue != NFK_EPI_REDUCE_SCATTER && g.gate_flags == nullptr && g.num_ctas <= 0 && g.smem_budget_kb <= 0 &&
+         g.stream_k != 3 && (g.norm_w == nullptr || (g.ldd == g.N && g.norm_ld == g.N));
+}
+
+// The split that one launch can do, from the shape that was chosen (or pinned): all tiles at once, since a cluster that waits
+// for a place would make a second wave of a product that is one wave long.
+SplitPlan split_in_cluster(const nfk_gemm_params& g, const Shape& s) {
+  if (!cluster_forms(g) || g.epilogue != NFK_EPI_LINEAR || s.mt != 1 || s.split_k < 2) return SplitPlan{};
+  SplitPlan f = split_plan(g.M, g.N, g.K, g.groups > 1 ? g.groups : 1, s.bn, s.cg, s.split_k);
+  if (f.stages < 2) return SplitPlan{};
+  const int size = s.split_k * s.cg;
+  if (f.tiles > (s.cg == 2 ? resident_split_clusters<2>(size) : resident_split_clusters<1>(size))) f.stages = 0;
+  return f;
+}
+
+template <int CG>
+int launch_split(const nfk_gemm_params& g, const SplitPlan& f, cudaStream_t stream) {
+  const int groups = g.groups > 1 ? g.groups : 1;
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_bf16_2d(&tmA, g.A, g.M, g.K + static_cast<uint64_t>(groups - 1) * g.group_k, g.lda, BM, BK);
+  if (rc == NF_OK) rc = make_tmap_bf16_2d(&tmB, g.B, g.N, g.K, g.ldb, f.bn / CG, BK);
+  if (rc != NF_OK) return rc;
+  SplitParams sp;
+  sp.d = dev_params(g, true);
+  sp.d.split_k = f.split;
+  sp.d.bn = f.bn;
+  sp.d.stages = f.stages;
+  sp.d.tmem_cols = f.tmem_cols;
+  sp.m_groups = f.m_groups;
+  sp.kb_per = f.kb_per;
+  sp.slice = f.slice;
+  sp.early_weights = g.weights_ready;
+  if (launch_kernel(early_first(g.early_start), gemm_split_cluster_kernel<CG>, f.tiles * f.split * CG, kGemmThreads, f.smem_bytes, stream,
+                    f.split * CG, tmA, tmB, sp) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
+  }
+  return g.norm_w != nullptr ? rmsnorm_rows(g, stream) : NF_OK;
+}
+
 // Whether the few-rows kernel takes this call. Forms that fix how the tile kernel cuts its work (a pinned shape, a CTA or
 // shared-memory budget, gated input, reduce-scatter) stay with it, and so do a norm of rows that are not contiguous and a
 // caller without a workspace, who gets one sum in the order of k.
 bool few_rows_takes(const nfk_gemm_params& g) {
-  if (g.rows_kernel == 2 || g.keep_order != 0 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
+  if (g.rows_kernel >= 2 || g.keep_order != 0 || g.epilogue == NFK_EPI_REDUCE_SCATTER || g.gate_flags != nullptr) return false;
   if (g.num_ctas > 0 || g.smem_budget_kb > 0 || g.stream_k != 0) return false;
   if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
   if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
@@ -1456,10 +1546,6 @@ int few_rows(const nfk_gemm_params& g, cudaStream_t stream) {
 // The earlier constants stay for calls with keep_order, the layer-list models' products: a recurrent layer carries every change
 // of rounding into its state and on to the next tokens (logits of a second step moved by up to 0.9 of their size in an element,
 // while either order is equally far from 64 bits: 0.0074), so these models keep the order of sums that the earlier shapes give.
-struct Shape {
-  int bn, mt, split_k, cg;
-  bool stream_k;
-};
 struct ShapeModel {
   double mma, fill, least_single, least_pair;                 // TFLOP/s, GB/s of an SM; us per k-block at least
   double uneven, single;                                      // factors: gated tiles of uneven width, single CTAs
@@ -1714,5 +1800,7 @@ extern "C" int nfk_gemm_bf16(const nfk_gemm_params* given, cudaStream_t stream) 
     return launch_mt<1>(*g, s.bn, s.mt, s.cg, 1, s.stream_k, stream);
   }
   if (rs) return launch_mt<2>(*g, s.bn, s.mt, s.cg, 1, false, stream);
+  const SplitPlan f = split_in_cluster(*g, s);
+  if (f.stages >= 2) return s.cg == 2 ? launch_split<2>(*g, f, stream) : launch_split<1>(*g, f, stream);
   return launch_mt<0>(*g, s.bn, s.mt, s.cg, s.split_k, s.stream_k, stream);
 }

@@ -90,7 +90,7 @@ typedef struct nfk_gemm_params {
   float act_limit, act_alpha, act_shift;   // constants of NFK_ACT_CAPPED
   const void* bias2;    // gated epilogue: [N] bf16 bias of the up half (`bias` is the gate half's), null = none
   int rows_kernel;      // the kernel for few rows (gemm_few_rows.cuh): 0 = by rule; 1 = it (`cta_group` 1 / 2 and `split_k`
-                        // as given, 0 = choose); 2 = the tile kernel
+                        // as given, 0 = choose); 2 = the tile kernel; 3 = the tile kernel, a split of K in two launches
   int weights_ready;    // B and B2 are complete (weights of a loaded model): with early_start they may be fetched while the
                         // launches before this one, back to the last that was not early, still run
   int tuned_rows;       // rows that the pinned shape was measured at: calls of other sizes leave the shape to the rules (another

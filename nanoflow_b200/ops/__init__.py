@@ -327,7 +327,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     ``gate_flags`` (int32 [ceil(M/128), 8]): rows of ``a`` are still arriving; the kernel waits, per
     128-row block, until words [block, 0:gate_nranks] have reached ``gate_epoch``.
 
-    ``rows_kernel`` 1 / 2 asks for / rules out the kernel for few rows (0 = the launcher's rule).
+    ``rows_kernel`` 1 / 2 asks for / rules out the kernel for few rows (0 = the launcher's rule); see kernels.h for others.
     ``keep_order``: shapes by the earlier rules (see kernels.h). ``early_start`` (EARLY_*): the kernels may start while the one
     before them on the stream ends; with ``weights_ready`` the caller states that ``w`` was complete long before."""
     _bf16(a, "a"); _bf16(w, "w")
