@@ -874,6 +874,12 @@ typedef struct nfk_copy_cols_params {
 typedef struct nfk_memcpy_params {   // plain async copy (any direction); elem_bytes * count bytes
   void* dst; const void* src; long long elem_bytes; int count;
 } nfk_memcpy_params;
+// Up to two copies of 32-bit words by one kernel, for a few kilobytes between pinned host memory and the device at the two ends
+// of an iteration: a kernel starts within a microsecond of its neighbours on the stream, a copy engine within five. Both sides
+// have to be memory that the device can address. `early`: NFK_EARLY_FIRST or 0.
+typedef struct nfk_word_copy_params {
+  int* dst; const int* src; int count; int* dst2; const int* src2; int count2; int early;
+} nfk_word_copy_params;
 typedef struct nfk_memcpy2d_params {  // strided async copy: `height` rows of `width` bytes, row pitches in bytes
   void* dst; const void* src; long long dpitch, spitch, width; int height;
 } nfk_memcpy2d_params;
@@ -889,6 +895,7 @@ int nfk_argmax_p(const nfk_argmax_params* p, cudaStream_t s);
 int nfk_argmax_combine_p(const nfk_argmax_combine_params* p, cudaStream_t s);
 int nfk_copy_cols_p(const nfk_copy_cols_params* p, cudaStream_t s);
 int nfk_memcpy_p(const nfk_memcpy_params* p, cudaStream_t s);
+int nfk_word_copy_p(const nfk_word_copy_params* p, cudaStream_t s);
 typedef struct nfk_sleep_params { int micros; } nfk_sleep_params;   // nfk_sleep as an op of the graph
 int nfk_sleep_p(const nfk_sleep_params* p, cudaStream_t s);
 int nfk_kv_move_p(const nfk_kv_move_params* p, cudaStream_t s);

@@ -62,6 +62,11 @@ class MemcpyParams(Structure):
     _fields_ = [("dst", c_void_p), ("src", c_void_p), ("elem_bytes", c_longlong), ("count", c_int)]
 
 
+class WordCopyParams(Structure):
+    _fields_ = [("dst", c_void_p), ("src", c_void_p), ("count", c_int), ("dst2", c_void_p), ("src2", c_void_p), ("count2", c_int),
+                ("early", c_int)]
+
+
 class Memcpy2DParams(Structure):
     _fields_ = [("dst", c_void_p), ("src", c_void_p), ("dpitch", c_longlong), ("spitch", c_longlong),
                 ("width", c_longlong), ("height", c_int)]
@@ -109,7 +114,7 @@ KERNEL_OF = {
     GqaAppendParams: "nfk_gqa_append", GqaAttnParams: "nfk_gqa_attn", MoeRouteParams: "nfk_moe_route",
     MoePermuteParams: "nfk_moe_permute", MoeGemmParams: "nfk_moe_gemm", TokenShiftParams: "nfk_token_shift",
     TalkAttnParams: "nfk_talk_attn", ShortConvParams: "nfk_short_conv",
-    MemcpyParams: "nfk_memcpy_p", Memcpy2DParams: "nfk_memcpy2d_p", KvMoveParams: "nfk_kv_move_p", SleepParams: "nfk_sleep_p",
+    MemcpyParams: "nfk_memcpy_p", WordCopyParams: "nfk_word_copy_p", Memcpy2DParams: "nfk_memcpy2d_p", KvMoveParams: "nfk_kv_move_p", SleepParams: "nfk_sleep_p",
 }
 
 
@@ -187,11 +192,15 @@ class OpGraph:
             if isinstance(op.params, (MemcpyParams, Memcpy2DParams)):
                 continue
             first = op.stream not in kernel_seen
+            behind = not first and any(after[pred[i]] >> d & 1 for d in op.deps)     # the predecessor has long ended
+            early = not first and not behind and not op.after_start and not beside[pred[i]] & ~before[i]
+            if isinstance(op.params, WordCopyParams):            # a copy: what follows one stays a first kernel
+                op.params.early = _ops.EARLY_FIRST if early else 0
+                continue
             kernel_seen.add(op.stream)
             if not hasattr(op.params, "early_start"):
                 continue
-            behind = not first and any(after[pred[i]] >> d & 1 for d in op.deps)     # the predecessor has long ended
-            if not first and not behind and not op.after_start and not beside[pred[i]] & ~before[i]:
+            if early:
                 op.params.early_start |= _ops.EARLY_FIRST
             if not beside[i]:
                 op.params.early_start |= _ops.EARLY_FURTHER

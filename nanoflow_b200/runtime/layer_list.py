@@ -53,7 +53,7 @@ from .engine import DECODE_MAX_CHUNKS, DECODE_SPLIT_ROWS, GEMM_WS_BYTES, Engine,
 from .graph import (ArgmaxParams, AttnParams, DeltaParams, GemmParams, GqaAppendParams, GqaAttnParams, HeadNormGateParams,
                     LatentAppendParams, LatentAttnParams, LatentGatherParams, MemcpyParams, MlstmParams, MoeGemmParams,
                     MoePermuteParams, MoeRouteParams, OpGraph, ResidualNormParams, RgLruParams, RopeTableParams,
-                    ShortConvParams, TalkAttnParams, TokenShiftParams, WkvParams)
+                    ShortConvParams, TalkAttnParams, TokenShiftParams, WkvParams, WordCopyParams)
 from .pipeline import _ptr
 
 QUERY_TILE = 128             # query tokens per work item of the prefill attention kernel
@@ -360,11 +360,10 @@ class LayerListEngine(Engine):
         for s in ("nb0_T", "nb0_items", "nb0_dec_begin", "nb0_dec_count", "n_sample", "n_dec", "n_pre"):
             g.symbol(s)
         lay = self.layout
-        self._op("meta_h2d", MemcpyParams(dst=_ptr(self.meta_dev), src=c_void_p(0), elem_bytes=4, count=lay.fixed_words),
-                 dyn=[("src", g.symbol("meta_src"))])
-        self._op("kv_indices_h2d", MemcpyParams(dst=c_void_p(self.meta_dev.data_ptr() + 4 * lay.off["kv_indices"]),
-                                                src=c_void_p(0), elem_bytes=4, count=0),
-                 dyn=[("src", g.symbol("kv_src")), ("count", g.symbol("kv_words"))])
+        self._op("meta_h2d", WordCopyParams(dst=_ptr(self.meta_dev), src=c_void_p(0), count=lay.fixed_words,
+                                            dst2=c_void_p(self.meta_dev.data_ptr() + 4 * lay.off["kv_indices"]), src2=c_void_p(0),
+                                            count2=0),
+                 dyn=[("src", g.symbol("meta_src")), ("src2", g.symbol("kv_src")), ("count2", g.symbol("kv_words"))])
         if m.run_moes():
             self._op("moe_counts", MemcpyParams(dst=_ptr(self.moe_counts), src=_ptr(self.moe_zeros), elem_bytes=4,
                                                 count=self.moe_counts.numel()))
@@ -411,10 +410,9 @@ class LayerListEngine(Engine):
         self._op("argmax", ArgmaxParams(idx_out=_ptr(self.bufs.sampled), val_out=c_void_p(0), logits=_ptr(self.logits),
                                         rows=0, cols=m.vocab_size, ld=self.logits.stride(0), col_offset=0, dtype=ops.F32),
                  dyn=[("rows", S)])
-        self._op("tokens_d2h", MemcpyParams(dst=c_void_p(0), src=_ptr(self.bufs.sampled), elem_bytes=4, count=0),
-                 dyn=[("dst", g.symbol("tokens_dst")), ("count", S)])
-        self._op("status_d2h", MemcpyParams(dst=c_void_p(0), src=_ptr(self.bufs.status), elem_bytes=4, count=1),
-                 dyn=[("dst", g.symbol("status_dst"))])
+        self._op("tokens_d2h", WordCopyParams(dst=c_void_p(0), src=_ptr(self.bufs.sampled), count=0, dst2=c_void_p(0),
+                                              src2=_ptr(self.bufs.status), count2=1),
+                 dyn=[("dst", g.symbol("tokens_dst")), ("count", S), ("dst2", g.symbol("status_dst"))])
         return g
 
     def _op(self, name, params, *, dyn=(), kernel=None, layer=-1) -> None:

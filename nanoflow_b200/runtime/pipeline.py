@@ -34,7 +34,7 @@ from .. import ops as _ops
 from ..config import EngineConfig, ModelConfig
 from ..models.llama import RankWeights
 from .graph import (ArgmaxCombineParams, ArgmaxParams, AttnParams, EmbeddingParams, GatherParams, GemmParams, RopeTableParams,
-                    KvMoveParams, MemcpyParams, NormParams, OpGraph, RopeAppendParams)
+                    KvMoveParams, MemcpyParams, NormParams, OpGraph, RopeAppendParams, WordCopyParams)
 
 
 def _ptr(t: Optional[torch.Tensor], row: int = 0) -> c_void_p:
@@ -184,13 +184,11 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
                          ids_out=c_void_p(0), n_tokens=0, hidden=hidden, vocab=model.vocab_size, status=_ptr(st))
     pre = []
     if io is not None:
-        # pinned host -> device metadata copies; the source slot rotates, so the pointers are symbols
-        c1 = MemcpyParams(dst=_ptr(io.meta_dev), src=c_void_p(0), elem_bytes=4, count=io.fixed_words)
-        pre.append(g.add("meta_h2d", c1, S("other"), dyn=[("src", g.symbol("meta_src"))]))
-        c2 = MemcpyParams(dst=c_void_p(io.meta_dev.data_ptr() + 4 * io.kv_off_words), src=c_void_p(0),
-                          elem_bytes=4, count=0)
-        pre.append(g.add("kv_indices_h2d", c2, S("other"),
-                         dyn=[("src", g.symbol("kv_src")), ("count", g.symbol("kv_words"))]))
+        # metadata from pinned host memory; the source slot rotates, so the pointers are symbols
+        c1 = WordCopyParams(dst=_ptr(io.meta_dev), src=c_void_p(0), count=io.fixed_words,
+                            dst2=c_void_p(io.meta_dev.data_ptr() + 4 * io.kv_off_words), src2=c_void_p(0), count2=0)
+        pre.append(g.add("meta_h2d", c1, S("other"), dyn=[("src", g.symbol("meta_src")), ("src2", g.symbol("kv_src")),
+                                                          ("count2", g.symbol("kv_words"))]))
     if bufs.rope_table is not None:
         # cos / sin of every token's rotary angles, once per iteration for all layers
         tp_ = RopeTableParams()
@@ -587,11 +585,9 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
                                  cand_idx=_ptr(bufs.cand_idx), shards=tp, rows=Bcap)
         last = g.add("argmax_combine", cp, S("net"), deps=[agc if agc is not None else am])
     if io is not None:
-        c3 = MemcpyParams(dst=c_void_p(0), src=_ptr(bufs.sampled), elem_bytes=4, count=0)
-        td = g.add("tokens_d2h", c3, g.ops[last].stream, deps=[last],
-                   dyn=[("dst", g.symbol("tokens_dst")), ("count", n_sample)])
         # the status word travels with the tokens, so the host sees a timeout or a bad index in the
         # iteration that had it, not at the end of serving
-        c4 = MemcpyParams(dst=c_void_p(0), src=_ptr(st), elem_bytes=4, count=1)
-        g.add("status_d2h", c4, g.ops[last].stream, deps=[td], dyn=[("dst", g.symbol("status_dst"))])
+        c3 = WordCopyParams(dst=c_void_p(0), src=_ptr(bufs.sampled), count=0, dst2=c_void_p(0), src2=_ptr(st), count2=1)
+        g.add("tokens_d2h", c3, g.ops[last].stream, deps=[last],
+              dyn=[("dst", g.symbol("tokens_dst")), ("count", n_sample), ("dst2", g.symbol("status_dst"))])
     return g
