@@ -113,6 +113,11 @@ struct DecCfg {
 constexpr int kDecodeCounterSlots = 64;
 __device__ unsigned int g_decode_counters[kDecodeCounterSlots][2];
 
+// Chunks of a (request, KV head) that have left their partial result, per launch slot: the last one to arrive merges them and
+// sets its count back to zero.
+constexpr int kDecArrivals = 8192;
+__device__ unsigned int g_decode_arrived[kDecodeCounterSlots][kDecArrivals];
+
 // What the token at the end of a request sees: its position, the page slot that the page list starts with, and how many
 // pages of the list lie before the token's chunk.
 struct DecodeRange {
@@ -169,15 +174,56 @@ __device__ __forceinline__ int list_chunks(const nfk_attn_params& p, int* first_
   return all;
 }
 
+// Final row of one head from its chunks' partial results, by one warp: lanes hold the chunks' weights, 32 at a time, and every
+// lane two columns of 64. The chunks are added in their order.
+template <int HD>
+__device__ __forceinline__ void merge_chunks(const nfk_attn_params& p, int bl, int head, int tok, int n_chunks) {
+  constexpr int V = HD / 64;                                   // pairs of columns per lane
+  const int lane = threadIdx.x & 31;
+  const float* ws = p.workspace + (static_cast<long long>(bl) * p.q_heads + head) * p.max_chunks * (HD + 2);
+  float mm = -INFINITY;
+  for (int c = lane; c < n_chunks; c += 32) mm = fmaxf(mm, __ldcg(ws + c * (HD + 2) + HD));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, off));
+  const float msafe = mm == -INFINITY ? 0.f : mm;
+  float W = p.sinks != nullptr ? fast_exp2(p.sinks[head] * kLog2e - msafe) : 0.f;
+  float2 acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = make_float2(0.f, 0.f);
+  for (int c0 = 0; c0 < n_chunks; c0 += 32) {
+    const float mine = c0 + lane < n_chunks ? exp2f(__ldcg(ws + (c0 + lane) * (HD + 2) + HD) - msafe) : 0.f;
+    const int here = min(32, n_chunks - c0);
+#pragma unroll 4
+    for (int c = 0; c < here; ++c) {
+      const float w = __shfl_sync(0xffffffffu, mine, c);
+      const float* row = ws + (c0 + c) * (HD + 2);
+      W += w;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const float2 x = __ldcg(reinterpret_cast<const float2*>(row + v * 64) + lane);
+        acc[v].x += w * x.x;
+        acc[v].y += w * x.y;
+      }
+    }
+  }
+  uint32_t* dst = reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (static_cast<long long>(tok) * p.q_heads + head) * HD);
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+    dst[v * 32 + lane] = W > 0.f ? pack_bf16x2(acc[v].x / W, acc[v].y / W) : 0u;
+}
+
 // EXT: sink in the denominator, capped scores, distance bias, chunks, page lists that start inside the sequence, queries in
 // wider rows, probabilities as a bf16 pair (in an instantiation of its own).
-// LIST: work items are the chunks that hold pages, from a list in shared memory behind the pipeline buffers.
+// LIST: work items are the chunks that hold pages, from a list in shared memory behind the pipeline buffers; with `merge` the
+// chunk that is the last of its request and KV head to finish merges them all (a launch of its own for that stood 5 to 7 us
+// behind this one: it reads what has just been written, and nothing else runs meanwhile; 24 requests of 100 to 6000 tokens, 4
+// layers with the shorter copies at both ends, 875 -> 858 us, one request 682 -> 653).
 // Registers: two CTAs of 96 KB are all that fit an SM, so three stages at head_dim 128 need no cap for a third (with one, the
 // loop spilled 28 bytes: 256 contexts of 200 to 2000 tokens, 8 KV heads, 148 -> 132 us; 24 of 100 to 6000 49 -> 45; 48 of 200
 // to 3000 56 -> 46), and a listed launch has two CTAs per SM; with two stages the cap leaves room for other kernels.
 template <int HD, int ST, bool EXT, bool LIST>
 __global__ void __launch_bounds__(kDecThreads, EXT || LIST || (HD == 128 && ST == 3) ? 2 : 3)
-attn_decode_kernel(nfk_attn_params p, int slot) {
+attn_decode_kernel(nfk_attn_params p, int slot, int merge) {
   using Cfg = DecCfg<HD, ST>;
   constexpr int kDecStages = ST;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -412,6 +458,21 @@ attn_decode_kernel(nfk_attn_params p, int slot) {
         *reinterpret_cast<float2*>(ws + c) = make_float2(x * inv, y * inv);
         if (c == 0) ws[HD] = L > 0.f ? mm + log2f(L) : -INFINITY;
       }
+    }
+    if (LIST && merge != 0 && n_chunks > 1) {
+      __syncthreads();                                        // this chunk's partial rows are written
+      int last = 0;
+      if (threadIdx.x == 0) {
+        unsigned int* arrived = &g_decode_arrived[slot][bl * p.kv_heads + kvh];
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == static_cast<unsigned int>(n_chunks - 1) ? 1 : 0;
+        if (last != 0) {
+          *arrived = 0u;
+          __threadfence();
+        }
+      }
+      if (__syncthreads_or(last) != 0)
+        for (int r = warp; r < group; r += kDecThreads / 32) merge_chunks<HD>(p, bl, kvh * group + r, tok, n_chunks);
     }
     } while (false);
     __syncthreads();  // every warp is done with the pipeline buffers and the merge area
@@ -665,9 +726,10 @@ int launch_decode_form(const nfk_attn_params* p, cudaStream_t stream) {
   if (ctas > total) ctas = total;
   static std::atomic<unsigned int> launch_seq{0};
   const int slot = static_cast<int>(launch_seq.fetch_add(1u) % kDecodeCounterSlots);
+  const bool merge = LIST && static_cast<long long>(p->req_count) * p->kv_heads <= kDecArrivals;
   cudaError_t e = launch_kernel(early_first(p->early_start), attn_decode_kernel<HD, ST, EXT, LIST>, static_cast<int>(ctas),
-                                kDecThreads, bytes, stream, 1, *p, slot);
-  if (e == cudaSuccess && p->chunk_pages > 0 && max_chunks > 1)
+                                kDecThreads, bytes, stream, 1, *p, slot, merge ? 1 : 0);
+  if (e == cudaSuccess && !merge && p->chunk_pages > 0 && max_chunks > 1)
     e = launch_kernel(early_further(p->early_start), attn_decode_merge_kernel<HD>, p->req_count * p->q_heads, HD, 0, stream, 1,
                       *p);
   if (e == cudaSuccess) return NF_OK;
