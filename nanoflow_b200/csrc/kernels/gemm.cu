@@ -1131,6 +1131,7 @@ constexpr int kSmemMax = 227 * 1024;
 
 #include "gemm_few_rows.cuh"
 #include "gemm_split_cluster.cuh"
+#include "gemm_mid_rows.cuh"
 
 // The caller's parameters as the kernels take them; geometry and work distribution are filled in by the launchers.
 inline DevParams dev_params(const nfk_gemm_params& g, bool linear) {
@@ -1409,6 +1410,7 @@ int launch_few_rows(const nfk_gemm_params& g, const FewPlan& f, cudaStream_t str
 struct Shape {
   int bn, mt, split_k, cg;
   bool stream_k;
+  double us = 0.0;      // of a chosen shape, by the model
 };
 
 // Clusters of `size` CTAs of `kernel`, with all the shared memory of an SM each, that can be resident at once; asked once per
@@ -1495,6 +1497,46 @@ int launch_split(const nfk_gemm_params& g, const SplitPlan& f, cudaStream_t stre
   return g.norm_w != nullptr ? rmsnorm_rows(g, stream) : NF_OK;
 }
 
+template <bool GATED, bool TWO>
+int resident_mid_clusters(int size) {
+  static int known_dev[kMaxDevices][kSplitMaxCluster + 1] = {};
+  const int n = resident_clusters(gemm_mid_rows_kernel<GATED, TWO>, size, known_dev[device_slot()][size]);
+  return n > 0 ? n : kResidentClusters[size];
+}
+
+template <bool GATED, bool TWO>
+int launch_mid_rows(const nfk_gemm_params& g, const MidPlan& f, cudaStream_t stream) {
+  CUtensorMap tmW0, tmW1, tmX, tmX2;
+  int rc = make_tmap_bf16_2d(&tmW0, g.B, g.N, g.K, g.ldb, GATED ? 64 : 128, BK);
+  if (rc != NF_OK) return rc;
+  tmW1 = tmW0;
+  if (GATED) rc = make_tmap_bf16_2d(&tmW1, g.B2, g.N, g.K, g.ldb, 64, BK);
+  if (rc == NF_OK) rc = make_tmap_bf16_2d(&tmX, g.A, g.M, g.K, g.lda, f.nb / 2, BK);
+  if (rc != NF_OK) return rc;
+  tmX2 = tmX;
+  if (TWO) rc = make_tmap_bf16_2d(&tmX2, g.A, g.M, g.K, g.lda, f.nb2 / 2, BK);
+  if (rc != NF_OK) return rc;
+  (void)resident_mid_clusters<GATED, TWO>(2 * f.split);      // sets the kernel's attributes
+  MidParams mp;
+  mp.d = dev_params(g, !GATED);
+  mp.d.stages = f.stages;
+  mp.d.tmem_cols = f.tmem_cols;
+  mp.nb = f.nb;
+  mp.nb2 = f.nb2;
+  mp.tok_tiles = f.tok_tiles;
+  mp.split = f.split;
+  mp.kb_per = f.kb_per;
+  mp.round_tokens = f.round_tokens;
+  mp.early_weights = g.weights_ready;
+  if (launch_kernel(early_first(g.early_start), gemm_mid_rows_kernel<GATED, TWO>, f.n_tiles * f.tok_tiles * f.split * 2, kGemmThreads,
+                    f.smem_bytes, stream, f.split * 2, tmW0, tmW1, tmX, tmX2, mp) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NF_ERR_CUDA;
+  }
+  if (!GATED && g.norm_w != nullptr) return rmsnorm_rows(g, stream);
+  return NF_OK;
+}
+
 // Whether the few-rows kernel takes this call. Forms that fix how the tile kernel cuts its work (a pinned shape, a CTA or
 // shared-memory budget, gated input, reduce-scatter) stay with it, and so do a norm of rows that are not contiguous and a
 // caller without a workspace, who gets one sum in the order of k.
@@ -1538,10 +1580,9 @@ int few_rows(const nfk_gemm_params& g, cudaStream_t stream) {
 // one CTA cover several M tiles with one weight tile (each weight byte enters shared memory once), which wins when M is
 // small and the GEMM is bound by streaming the weight.
 //
-// The constants (us, bytes, TFLOP/s of one SM) are fitted to all candidate shapes of ten products (4096 to 128256 columns,
-// K 4096 to 28672, two of them gated) at 15 numbers of rows from 100 to 2000: the shape it takes is 1.2 % slower than the
-// fastest one on average; with the constants before, 6 % and up to 80 % (333 x 32000 x 8192: 284 -> 158 us,
-// 512 x 14336 x 2 x 4096: 179 -> 119, 192 x 10240 x 8192: 57 -> 40).
+// The constants (us, bytes, TFLOP/s of one SM) are fitted, with the gated epilogue and the split in a cluster as they are, to
+// all candidate shapes of eleven products (4096 to 128256 columns, K 4096 to 28672, three of them gated) at 15 numbers of rows
+// from 100 to 1500, by the time of the shape that is taken. Tiles of 224 columns are the best of the gated ones at most sizes.
 //
 // The earlier constants stay for calls with keep_order, the layer-list models' products: a recurrent layer carries every change
 // of rounding into its state and on to the next tokens (logits of a second step moved by up to 0.9 of their size in an element,
@@ -1553,22 +1594,59 @@ struct ShapeModel {
   double reduce, reduce_rate, fix, fix_rate, copy_rate;       // us and TB/s of the second passes; GB/s of a CTA's partial copies
   double weight_rate;                                         // TB/s at which the weight arrives, 0 = no bound
   double tail_gain;                                           // a stream-K tail has to be below this share of the best without
+  double cluster, cluster_col;                                // us, and per column sent, where parts meet in a cluster; 0 = as two launches
 };
-constexpr ShapeModel kModel{10.2, 115.0, 0.296, 0.273, 1.08, 1.05, 0.847, 0.0119, 0.00119, 5.15, 3.27, 2.52, 1.27, 218.0, 5.79, 1.0};
-constexpr ShapeModel kEarlierModel{11.0, 100.0, 0.0, 0.36, 1.0, 1.0, 2.0, 0.012, 0.003, 3.0, 4.0, 3.0, 3.0, 150.0, 0.0, 0.88};
-Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
+constexpr ShapeModel kModel{9.883, 129.2, 0.331, 0.295, 0.966, 1.095, 0.868, 0.0117, 0.00119, 7.28, 2.70, 2.47, 1.325, 177.0, 6.38, 1.0, 4.04, 0.01045};
+constexpr ShapeModel kEarlierModel{11.0, 100.0, 0.0, 0.36, 1.0, 1.0, 2.0, 0.012, 0.003, 3.0, 4.0, 3.0, 3.0, 150.0, 0.0, 0.88, 0.0, 0.0};
+// What one shape costs by the model, without a stream-K tail.
+struct TileCost {
+  double t_kb, unit_fixed, us;      // per k-block, per unit, the whole product
+  int tiles, workers, mt_eff;
+};
+double weight_bound(const ShapeModel& m, const nfk_gemm_params& g, bool swiglu, double us) {
+  if (m.weight_rate <= 0.0) return us;
+  const double w = static_cast<double>(g.N) * g.K * (swiglu ? 4.0 : 2.0) / (m.weight_rate * 1e6) + 0.25 * us;
+  return w > us ? w : us;
+}
+TileCost tile_cost(const ShapeModel& m, const nfk_gemm_params& g, bool swiglu, int bn, int mt, int sk, int cg) {
+  TileCost c;
+  const int ctas = g.num_ctas > 0 ? g.num_ctas : sm_count(), groups = g.groups > 1 ? g.groups : 1;
+  const int m_tiles = (g.M + BM - 1) / BM, num_kb = (g.K + BK - 1) / BK;
+  const int m_groups = (m_tiles + mt * cg - 1) / (mt * cg);
+  c.tiles = m_groups * n_block_count(groups, g.N / groups, swiglu ? bn / 2 : bn);
+  c.mt_eff = m_tiles < mt ? m_tiles : mt;
+  // per k-block and SM (a CTA of a pair stages only half of the weight tile)
+  const double t_mma = 2.0 * BM * c.mt_eff * bn * BK / (m.mma * 1e6);
+  const double t_fill = (c.mt_eff * 16384.0 + bn * 128.0 / cg) / (m.fill * 1e3);
+  c.t_kb = t_mma > t_fill ? t_mma : t_fill;
+  const double t_least = cg == 2 ? m.least_pair : m.least_single;
+  if (c.t_kb < t_least) c.t_kb = t_least;
+  if (swiglu && bn % 64 != 0) c.t_kb *= m.uneven;
+  if (cg == 1) c.t_kb *= m.single;
+  // per unit: prologue + epilogue; the epilogue hides under the next main loop only when TMEM
+  // holds two accumulator sets
+  const bool single_acc = mt * bn * 2 > 512;
+  c.unit_fixed = m.unit + (single_acc ? m.per_col_single : m.per_col) * c.mt_eff * bn;
+  c.workers = ctas / cg > 0 ? ctas / cg : 1;
+  const int units = c.tiles * sk, kb_per = (num_kb + sk - 1) / sk;
+  double us = ((units + c.workers - 1) / c.workers) * (kb_per * c.t_kb + c.unit_fixed);
+  if (sk > 1) {
+    if (m.cluster > 0.0 && cluster_forms(g) && mt == 1 && sk * cg <= kSplitMaxCluster &&
+        c.tiles <= (cg == 2 ? resident_split_clusters<2>(sk * cg) : resident_split_clusters<1>(sk * cg)))
+      us += m.cluster + m.cluster_col * bn * (sk - 1) / sk;
+    else
+      us += m.reduce + (sk + 1.0) * g.M * static_cast<double>(g.N) * 4.0 / (m.reduce_rate * 1e6);  // partial write + reduce
+  }
+  c.us = weight_bound(m, g, swiglu, us);
+  return c;
+}
+
+Shape search_shape(const nfk_gemm_params& g, bool swiglu) {
   const ShapeModel& m = g.keep_order != 0 ? kEarlierModel : kModel;
-  const int ctas = g.num_ctas > 0 ? g.num_ctas : sm_count();
-  const int m_tiles = (g.M + BM - 1) / BM;
-  const int num_kb = (g.K + BK - 1) / BK;
-  const double weight_us = m.weight_rate > 0.0 ? static_cast<double>(g.N) * g.K * (swiglu ? 4.0 : 2.0) / (m.weight_rate * 1e6) : 0.0;
+  const int m_tiles = (g.M + BM - 1) / BM, num_kb = (g.K + BK - 1) / BK;
   Shape best{256, 1, 1, 1, false}, best_tail{256, 1, 1, 1, true};
   double best_cost = 1e30, best_tail_cost = 1e30;
   const int cg_lo = g.cta_group == 2 ? 2 : 1, cg_hi = g.cta_group == 1 ? 1 : 2;
-  auto bounded = [&](double c) {
-    const double w = weight_us + 0.25 * c;
-    return m.weight_rate > 0.0 && w > c ? w : c;
-  };
   for (int cg = cg_lo; cg <= cg_hi; ++cg) {
     for (int mt = 1; mt <= (cg == 2 ? 1 : 4); mt *= 2) {
       for (int bn = swiglu ? 128 : 64; bn <= 256; bn += 32) {
@@ -1578,49 +1656,26 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
         // the single TMEM accumulator set would serialise epilogue and main loop for nothing.
         if (mt > 1 && (m_tiles > 4 || m_tiles <= mt / 2)) continue;
         if (cg == 2 && m_tiles < 2) continue;    // a pair covers two M tiles
-        const int out_bn = swiglu ? bn / 2 : bn;
-        const int m_groups = (m_tiles + mt * cg - 1) / (mt * cg);
-        const int n_blocks = n_block_count(g.groups > 1 ? g.groups : 1, g.N / (g.groups > 1 ? g.groups : 1), out_bn);
-        const int tiles = m_groups * n_blocks;
-        const int mt_eff = m_tiles < mt ? m_tiles : mt;
-        // per k-block and SM (a CTA of a pair stages only half of the weight tile)
-        const double t_mma = 2.0 * BM * mt_eff * bn * BK / (m.mma * 1e6);
-        const double t_fill = (mt_eff * 16384.0 + bn * 128.0 / cg) / (m.fill * 1e3);
-        double t_kb = t_mma > t_fill ? t_mma : t_fill;
-        const double t_least = cg == 2 ? m.least_pair : m.least_single;
-        if (t_kb < t_least) t_kb = t_least;
-        if (swiglu && bn % 64 != 0) t_kb *= m.uneven;
-        if (cg == 1) t_kb *= m.single;
-        // per unit: prologue + epilogue; the epilogue hides under the next main loop only when TMEM
-        // holds two accumulator sets
-        const bool single_acc = mt * bn * 2 > 512;
-        const double unit_fixed = m.unit + (single_acc ? m.per_col_single : m.per_col) * mt_eff * bn;
-        const int workers = ctas / cg > 0 ? ctas / cg : 1;
         const int max_sk = (swiglu || g.workspace == nullptr || g.epilogue == NFK_EPI_REDUCE_SCATTER) ? 1 : 8;
         for (int sk = 1; sk <= max_sk; ++sk) {
           if (sk > 1 && (num_kb / sk < 8 || static_cast<long long>(sk) * g.M * g.N * 4 > g.workspace_bytes)) break;
-          const int units = tiles * sk;
-          const int waves = (units + workers - 1) / workers;
-          const int kb_per = (num_kb + sk - 1) / sk;
-          double cost = waves * (kb_per * t_kb + unit_fixed);
-          if (sk > 1) cost += m.reduce + (sk + 1.0) * g.M * static_cast<double>(g.N) * 4.0 / (m.reduce_rate * 1e6);  // partial write + reduce
-          cost = bounded(cost);
-          if (cost < best_cost) {
-            best_cost = cost;
+          const TileCost c = tile_cost(m, g, swiglu, bn, mt, sk, cg);
+          if (c.us < best_cost) {
+            best_cost = c.us;
             best = Shape{bn, mt, sk, cg, false};
           }
           // the same shape with a stream-K tail: full waves as above, then one round of k ranges whose
           // pieces are written out as fp32 and summed by a second pass
           if (sk == 1 && g.stream_k < 2 && g.workspace != nullptr && g.epilogue != NFK_EPI_REDUCE_SCATTER) {
-            const SkPlan pl = plan_stream_k(tiles, workers, num_kb);
+            const SkPlan pl = plan_stream_k(c.tiles, c.workers, num_kb);
             const long long need = static_cast<long long>(pl.rest) * pl.max_pieces * cg * mt * BM * bn * 4;
             if (pl.q > 0 && need <= g.workspace_bytes) {
-              const double tile_bytes = mt_eff * BM * bn * 4.0;          // one fp32 copy of a CTA's tile rows
+              const double tile_bytes = c.mt_eff * BM * bn * 4.0;          // one fp32 copy of a CTA's tile rows
               const double pieces = static_cast<double>(num_kb) / pl.q + 1.0;
               // a worker's range may straddle two tiles
               const double fix_us = m.fix + pl.rest * cg * pieces * tile_bytes / (m.fix_rate * 1e6);
-              const double tail = pl.q * t_kb + 2.0 * unit_fixed + tile_bytes / (m.copy_rate * 1e3) + fix_us;
-              const double c2 = bounded((tiles / workers) * (kb_per * t_kb + unit_fixed) + tail);
+              const double tail = pl.q * c.t_kb + 2.0 * c.unit_fixed + tile_bytes / (m.copy_rate * 1e3) + fix_us;
+              const double c2 = weight_bound(m, g, swiglu, (c.tiles / c.workers) * (num_kb * c.t_kb + c.unit_fixed) + tail);
               if (c2 < best_tail_cost) {
                 best_tail_cost = c2;
                 best_tail = Shape{bn, mt, 1, cg, true};
@@ -1631,8 +1686,83 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
       }
     }
   }
-  if (g.stream_k == 1 && best_tail_cost < 1e30) return best_tail;
-  return best_tail_cost < m.tail_gain * best_cost ? best_tail : best;
+  const bool tail = (g.stream_k == 1 && best_tail_cost < 1e30) || best_tail_cost < m.tail_gain * best_cost;
+  Shape s = tail ? best_tail : best;
+  // (what kModel says of a shape that the earlier one has chosen)
+  s.us = g.keep_order == 0 ? (tail ? best_tail_cost : best_cost) : tile_cost(kModel, g, swiglu, s.bn, s.mt, s.split_k, s.cg).us;
+  return s;
+}
+
+// The search looks at some 200 shapes, 4 us of a launch's host time, and the layers of an iteration ask for the same few
+// products: a thread keeps the answers to its last questions, by everything that the search reads (sizes and forms, no address).
+Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
+  constexpr int kKept = 16;
+  struct Question {
+    long long workspace;
+    int M, N, K, groups, num_ctas, cta_group, stream_k, device, forms;
+    bool operator==(const Question& o) const {
+      return workspace == o.workspace && M == o.M && N == o.N && K == o.K && groups == o.groups && num_ctas == o.num_ctas &&
+             cta_group == o.cta_group && stream_k == o.stream_k && device == o.device && forms == o.forms;
+    }
+  };
+  struct Kept {
+    Question q;
+    Shape s;
+  };
+  thread_local Kept kept[kKept];
+  thread_local int n = 0, next = 0;
+  const Question q{g.workspace != nullptr ? g.workspace_bytes : -1, g.M, g.N, g.K, g.groups, g.num_ctas, g.cta_group, g.stream_k, device_slot(),
+                   (swiglu ? 1 : 0) | (g.keep_order != 0 ? 2 : 0) | (g.epilogue == NFK_EPI_REDUCE_SCATTER ? 4 : 0) | (cluster_forms(g) ? 8 : 0)};
+  for (int i = 0; i < n; ++i)
+    if (kept[i].q == q) return kept[i].s;
+  const Shape s = search_shape(g, swiglu);
+  kept[next] = Kept{q, s};
+  next = (next + 1) % kKept;
+  if (n < kKept) ++n;
+  return s;
+}
+
+// Whether the mid-rows kernel takes a call for which the tile kernel would have shape `s`, and with how many parts of K (stages
+// 0: it does not). rows_kernel 4 asks for it with split_k parts.
+//
+// Its cost by the same model, fitted to 15 numbers of rows from 64 to 1000 of ten products: what a k-block takes is the largest
+// of the products (1.24 ns per token), what enters the SMs of all pairs at once (11.7 TB/s), the weights' way from HBM (7.2 TB/s)
+// and 0.21 us. The two models' choice is 0.8 % slower than the best of all shapes on average, at worst 12 %; the tile kernel
+// alone, with the constants before, 3.4 % slower than the best of its own. us, tile kernel -> this one: 8192 x 28672 at 160 rows
+// 96 -> 82, 288 153 -> 107, 384 163 -> 133, 700 254 -> 232; 8192 x 8192 at 160 39.5 -> 31, 333 49 -> 42; 4096 x 14336 at 288
+// 45 -> 39; 28672 x 2 x 8192 at 288 285 -> 266. On the other side of the line: 8192 x 28672 at 512 166 (170 here), 1000 315 (317);
+// 4096 x 4096 at 333 21.4 (23.2); 14336 x 2 x 4096 at 256 52 (70), 333 81 (84).
+//
+// With keep_order K stays cut as the tile kernel's shape cuts it, which gives the same bits.
+MidPlan mid_rows_takes(const nfk_gemm_params& g, const Shape& s) {
+  const bool gated = g.epilogue == NFK_EPI_SWIGLU;
+  if (!cluster_forms(g) || g.groups > 1) return MidPlan{};
+  if (g.rows_kernel != 4 && (g.rows_kernel != 0 || g.M > 1024 || g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0 ||
+                             g.stream_k != 0 || (g.keep_order != 0 && s.stream_k)))
+    return MidPlan{};
+  MidPlan best{};
+  double best_us = g.rows_kernel == 4 ? 1e30 : s.us - 4.35;
+  const int lo = g.rows_kernel == 4 ? (g.split_k > 0 ? g.split_k : 1) : g.keep_order != 0 ? s.split_k : 1;
+  const int hi = g.rows_kernel == 4 || g.keep_order != 0 ? lo : g.workspace == nullptr ? 1 : 4;   // without a workspace: one sum in the order of k
+  for (int split = lo; split <= hi; ++split) {
+    const MidPlan f = mid_rows_plan(g.M, g.N, g.K, gated, split);
+    if (f.stages < 2 || f.round_tokens < 32) continue;
+    const int fit = f.nb2 > 0 ? (gated ? resident_mid_clusters<true, true>(2 * split) : resident_mid_clusters<false, true>(2 * split))
+                              : (gated ? resident_mid_clusters<true, false>(2 * split) : resident_mid_clusters<false, false>(2 * split));
+    const int tiles = f.n_tiles * f.tok_tiles, cols = f.nb + f.nb2, pairs = (tiles < fit ? tiles : fit) * split;
+    double kb = 1.24e-3 * cols;
+    const double enter = pairs * 2.0 * (kFewWBytes + 64.0 * cols) / 11.7e6, weights = pairs * 2.0 * kFewWBytes / f.tok_tiles / 7.16e6;
+    kb = kb > enter ? kb : enter;
+    kb = kb > weights ? kb : weights;
+    kb = kb > 0.206 ? kb : 0.206;
+    const double one = f.kb_per * kb + 3.98 + 0.0203 * cols + (split > 1 ? 0.56 : 0.0) + 1.25 * ((cols + f.round_tokens - 1) / f.round_tokens - 1);
+    const double us = one * ((tiles + fit - 1) / fit);
+    if (us < best_us) {
+      best_us = us;
+      best = f;
+    }
+  }
+  return best;
 }
 
 // A shape measured at another number of rows (tuned_rows) says little about this call: it holds for calls with as many
@@ -1738,6 +1868,8 @@ extern "C" int nfk_gemm_describe(const nfk_gemm_params* given, nfk_gemm_plan* ou
   out->stages = geo.stages;
   out->smem_bytes = geo.smem_bytes;
   out->few_rows = few_rows_takes(*g) ? 1 : 0;
+  const MidPlan mid = out->few_rows != 0 ? MidPlan{} : mid_rows_takes(*g, s);
+  out->mid_rows = mid.stages >= 2 ? mid.split : 0;
   return NF_OK;
 }
 
@@ -1792,8 +1924,16 @@ extern "C" int nfk_gemm_bf16(const nfk_gemm_params* given, cudaStream_t stream) 
 
   if (few_rows_takes(*g)) return few_rows(*g, stream);
   Shape s;
-  const int rcs = resolve_shape(*g, swiglu, rs, s);
-  if (rcs != NF_OK) return rcs;
+  if (g->rows_kernel != 4) {
+    const int rcs = resolve_shape(*g, swiglu, rs, s);
+    if (rcs != NF_OK) return rcs;
+  }
+  const MidPlan mid = mid_rows_takes(*g, s);
+  if (mid.stages >= 2) {
+    if (mid.nb2 > 0) return swiglu ? launch_mid_rows<true, true>(*g, mid, stream) : launch_mid_rows<false, true>(*g, mid, stream);
+    return swiglu ? launch_mid_rows<true, false>(*g, mid, stream) : launch_mid_rows<false, false>(*g, mid, stream);
+  }
+  if (g->rows_kernel == 4) return NF_ERR_UNSUPPORTED;
   if (swiglu) {
     if ((s.bn / 2) % 16 != 0) return NF_ERR_UNSUPPORTED;
     if (g->bias != nullptr) return launch_mt<kGatedBias>(*g, s.bn, s.mt, s.cg, 1, s.stream_k, stream);

@@ -90,7 +90,8 @@ typedef struct nfk_gemm_params {
   float act_limit, act_alpha, act_shift;   // constants of NFK_ACT_CAPPED
   const void* bias2;    // gated epilogue: [N] bf16 bias of the up half (`bias` is the gate half's), null = none
   int rows_kernel;      // the kernel for few rows (gemm_few_rows.cuh): 0 = by rule; 1 = it (`cta_group` 1 / 2 and `split_k`
-                        // as given, 0 = choose); 2 = the tile kernel; 3 = the tile kernel, a split of K in two launches
+                        // as given, 0 = choose); 2 = the tile kernel; 3 = the tile kernel, a split of K in two launches; 4 = the
+                        // mid-rows kernel (gemm_mid_rows.cuh) with split_k parts, 0 = one
   int weights_ready;    // B and B2 are complete (weights of a loaded model): with early_start they may be fetched while the
                         // launches before this one, back to the last that was not early, still run
   int tuned_rows;       // rows that the pinned shape was measured at: calls of other sizes leave the shape to the rules (another
@@ -114,6 +115,7 @@ typedef struct nfk_gemm_plan {
   int tail_first_tile, tail_range_kb, tail_max_pieces;   // stream-K tail (tail_range_kb 0 = none)
   int stages, smem_bytes;
   int few_rows;                        // 1 = the call goes to the few-rows kernel, and the rest is what the tile kernel would do
+  int mid_rows;                        // > 0: the call goes to the mid-rows kernel with so many parts of K, likewise
 } nfk_gemm_plan;
 int nfk_gemm_describe(const nfk_gemm_params* p, nfk_gemm_plan* out);
 

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from nanoflow_b200 import ops
+from nanoflow_b200.ops import layer_list as K
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +52,19 @@ def test_rows_apart():
     src[:, 8:2056] = a
     outs = [ops.gemm(src[:, 8:2056], w, out=wide.clone()[:, 40:560], rows_kernel=k, **kw) for k in (2, 3)]
     assert torch.equal(*outs) and torch.equal(outs[0], ops.gemm(a, w, rows_kernel=2, **kw))
+
+
+@pytest.mark.parametrize("cta_group,split", [(1, 4), (2, 2)])
+def test_blocks_on_the_diagonal_and_32_bit_columns(cta_group, split):
+    a, w, _, _ = _operands(200, 4 * 136, 4 * 512)
+    kw = dict(workspace=torch.empty(16 << 20, device="cuda"), tile_m=1, tile_n=64, cta_group=cta_group, split_k=split, stream_k=2)
+    blocks = [K.gemm(a, w[:, :512].contiguous(), groups=4, group_k=512, k=512, rows_kernel=r, **kw) for r in (2, 3)]
+    assert torch.equal(*blocks)
+    want = torch.cat([a[:, 512 * i:512 * i + 512].double() @ w[136 * i:136 * i + 136, :512].double().T for i in range(4)], 1)
+    assert ((blocks[0].double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+    wide = [torch.zeros(200, 344, device="cuda") for _ in range(2)]
+    outs = [K.gemm(a, w, out32=o, f32_col0=200, lin_act="tanh", rows_kernel=r, **kw) for o, r in zip(wide, (2, 3))]
+    assert torch.equal(*outs) and torch.equal(*wide)
+    want = torch.tanh(a.double() @ w.double().T)
+    assert ((wide[0].double() - want[:, 200:]).abs() <= 1e-4).all()
+    assert ((outs[0].double() - want[:, :200]).abs() <= want[:, :200].abs() * 2.0 ** -8 + 1e-4).all()
