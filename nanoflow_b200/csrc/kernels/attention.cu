@@ -109,15 +109,17 @@ struct DecCfg {
 
 // Work items are handed out through a counter: a CTA takes its first item by its index and every further
 // one with an atomic increment, so CTAs that run slower (an SM shared with another kernel's CTA, a long
-// context) take fewer items instead of holding up the launch. One counter pair per launch slot; launches
-// cycle through the slots, and the last CTA of a launch to finish resets its slot.
-constexpr int kDecodeCounterSlots = 64;
+// context) take fewer items instead of holding up the launch. The last CTA of a launch to finish sets the
+// counter back. It lives with the caller's workspace (`counts`), which launches that may run at the same time
+// do not share; a caller that passes none gets one of these, and the launches of all forms take turns at them.
+constexpr int kDecodeCounterSlots = 1024;
 __device__ unsigned int g_decode_counters[kDecodeCounterSlots][2];
+std::atomic<unsigned int> g_decode_launches{0};
 
-// Chunks of a (request, KV head) that have left their partial result, per launch slot: the last one to arrive merges them and
-// sets its count back to zero.
-constexpr int kDecArrivals = 8192;
-__device__ unsigned int g_decode_arrived[kDecodeCounterSlots][kDecArrivals];
+// Behind the two words of the work counter, `counts` holds the chunks of each (request, KV head) that have left their partial
+// result: the last one to arrive merges them and sets the count back to zero. Only in the caller's memory: a count that two
+// launches step at once would stay wrong for good, and so would every merge after that.
+constexpr int kDecArrivals = NFK_ATTN_DECODE_COUNTS - 2;
 
 // What the token at the end of a request sees: its position, the page slot that the page list starts with, and how many
 // pages of the list lie before the token's chunk.
@@ -244,7 +246,7 @@ attn_decode_kernel(nfk_attn_params p, int slot, int merge) {
   const float scale = p.sm_scale * kLog2e;
   const uint32_t warp_smem = smem_u32(smem) + warp * Cfg::WARP_BYTES;
 
-  unsigned int* counters = g_decode_counters[slot];
+  unsigned int* counters = p.counts != nullptr ? p.counts : g_decode_counters[slot];
   long long item = blockIdx.x;
   while (item < total) {
     // the index of the item after this one is fetched now (thread 0 keeps it) and handed to the CTA through
@@ -464,7 +466,7 @@ attn_decode_kernel(nfk_attn_params p, int slot, int merge) {
       __syncthreads();                                        // this chunk's partial rows are written
       int last = 0;
       if (threadIdx.x == 0) {
-        unsigned int* arrived = &g_decode_arrived[slot][bl * p.kv_heads + kvh];
+        unsigned int* arrived = p.counts + 2 + bl * p.kv_heads + kvh;
         __threadfence();
         last = atomicAdd(arrived, 1u) == static_cast<unsigned int>(n_chunks - 1) ? 1 : 0;
         if (last != 0) {
@@ -725,9 +727,8 @@ int launch_decode_form(const nfk_attn_params* p, cudaStream_t stream) {
   const long long total = static_cast<long long>(p->req_count) * p->kv_heads * max_chunks;
   long long ctas = p->num_ctas > 0 ? p->num_ctas : 2LL * sm_count_attn();
   if (ctas > total) ctas = total;
-  static std::atomic<unsigned int> launch_seq{0};
-  const int slot = static_cast<int>(launch_seq.fetch_add(1u) % kDecodeCounterSlots);
-  const bool merge = LIST && static_cast<long long>(p->req_count) * p->kv_heads <= kDecArrivals;
+  const bool merge = LIST && p->counts != nullptr && static_cast<long long>(p->req_count) * p->kv_heads <= kDecArrivals;
+  const int slot = p->counts != nullptr ? 0 : static_cast<int>(g_decode_launches.fetch_add(1u) % kDecodeCounterSlots);
   cudaError_t e = launch_kernel(early_first(p->early_start), attn_decode_kernel<HD, ST, EXT, LIST>, static_cast<int>(ctas),
                                 kDecThreads, bytes, stream, 1, *p, slot, merge ? 1 : 0);
   if (e == cudaSuccess && !merge && p->chunk_pages > 0 && max_chunks > 1)

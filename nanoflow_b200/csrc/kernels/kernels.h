@@ -238,7 +238,12 @@ typedef struct nfk_attn_params {
   const float* dist;       // [q_heads][2] (a, b): score <- score - a ln(1 + b (i - j)); null = none
   int chunk;               // > 0: position i sees j only if i / chunk = j / chunk
   int early_start;         // nfk_attn_decode, nfk_attn_prefill_ws: see nfk_gemm_params
+  // nfk_attn_decode: NFK_ATTN_DECODE_COUNTS words, zero before their first use (every launch leaves them zero), of which
+  // launches that may run at the same time each need their own, like `workspace`. With them a split context's chunks are merged
+  // in the same launch where that is built; null: by a second launch.
+  unsigned int* counts;
 } nfk_attn_params;
+enum { NFK_ATTN_DECODE_COUNTS = 2 + 8192 };
 int nfk_attn_decode(const nfk_attn_params* p, cudaStream_t stream);
 // The same with the pages copied by a TMA producer warp into a ring of decode_stages (2, 3 or 4) pages per
 // consumer warp, one work item per warp (attention_dec.cu): full bandwidth from one CTA per SM, for sharing

@@ -79,7 +79,7 @@ class AttnParams(Structure):
                 ("items", c_void_p), ("num_items", c_int), ("status", c_void_p), ("decode_stages", c_int),
                 ("window", c_int), ("sinks", c_void_p), ("kv_ld", c_int), ("k_col", c_int), ("v_col", c_int),
                 ("q_rows", c_int), ("ld_q", c_int), ("softcap", c_float), ("precise", c_int), ("kv_first", c_void_p),
-                ("dist", c_void_p), ("chunk", c_int), ("early_start", c_int)]
+                ("dist", c_void_p), ("chunk", c_int), ("early_start", c_int), ("counts", c_void_p)]
 
 
 BF16, F32 = 0, 1                                        # storage type of a kernel's activations and weights
@@ -647,14 +647,32 @@ def _attn_common(q, out, kv_pool, qo_indptr, kv_indptr, kv_indices, kv_last_page
     return p
 
 
+DECODE_COUNTS = 2 + 8192      # NFK_ATTN_DECODE_COUNTS
+
+
+def decode_counts(device="cuda") -> torch.Tensor:
+    """Counts of decode attention launches that run one after the other: zeros, and zeros again after each launch."""
+    return torch.zeros(DECODE_COUNTS, dtype=torch.int32, device=device)
+
+
+def _decode_counts(counts: Optional[torch.Tensor]) -> c_void_p:
+    if counts is not None:
+        _i32(counts, "counts")
+        if counts.numel() < DECODE_COUNTS or not counts.is_contiguous():
+            raise RuntimeError(f"attn_decode: counts are {DECODE_COUNTS} contiguous words (decode_counts)")
+    return _p(counts)
+
+
 def attn_decode(q, out, kv_pool, qo_indptr, kv_indptr, kv_indices, kv_last_page_len, *,
                 q_heads: int, req_begin: int, req_count: int, sm_scale: Optional[float] = None,
                 num_ctas: int = 0, chunk_pages: int = 0, workspace: Optional[torch.Tensor] = None,
-                max_chunks: int = 1, status: Optional[torch.Tensor] = None, stages: int = 0, impl: str = ""):
+                max_chunks: int = 1, status: Optional[torch.Tensor] = None, stages: int = 0, impl: str = "",
+                counts: Optional[torch.Tensor] = None):
     """Single-query attention for requests [req_begin, req_begin+req_count) over the paged pool.
     ``stages``: pages in flight per warp, 3 (default) or 2 (64 KB of shared memory per CTA instead of 96).
     ``impl``: "" = per-warp cp.async rings, "tma" = pages copied by a TMA producer warp (head_dim 128;
-    ``stages`` may then also be 4)."""
+    ``stages`` may then also be 4). ``counts``: ``decode_counts()`` that no launch running at the same time uses; chunks are then
+    merged without a second launch."""
     p = _attn_common(q, out, kv_pool, qo_indptr, kv_indptr, kv_indices, kv_last_page_len, q_heads,
                      sm_scale, num_ctas, status)
     p.decode_stages = stages
@@ -666,6 +684,7 @@ def attn_decode(q, out, kv_pool, qo_indptr, kv_indptr, kv_indices, kv_last_page_
         if workspace is None or workspace.dtype != torch.float32 or workspace.numel() < need:
             raise RuntimeError("attn_decode: split-KV needs an fp32 workspace of "
                                f"{need} elements")
+    p.counts = _decode_counts(counts)
     if impl == "tma":
         _check(lib().nfk_attn_decode_tma(byref(p), _stream()), "nfk_attn_decode_tma")
     else:

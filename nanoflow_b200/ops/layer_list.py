@@ -13,7 +13,7 @@ import torch
 
 from . import (ACTS, CONV_ACTS, LIN_ACTS, NORMS, ROUTER_SCORES, AttnParams, DeltaParams, GemmParams, GqaAppendParams, GqaAttnParams, HeadNormGateParams,
                LatentAppendParams, LatentAttnParams, LatentGatherParams, MlstmParams, MoeGemmParams, MoePermuteParams,
-               MoeRouteParams, ResidualNormParams, RgLruParams, ShortConvParams, TalkAttnParams, TokenShiftParams, WkvParams, _check, _i32, _p, _stream, dtype_code, lib)
+               MoeRouteParams, ResidualNormParams, RgLruParams, ShortConvParams, TalkAttnParams, TokenShiftParams, WkvParams, _check, _decode_counts, _i32, _p, _stream, dtype_code, lib)
 
 
 def _f32(t: Optional[torch.Tensor], name: str) -> None:
@@ -257,7 +257,7 @@ def gqa_attention(q, pool, out, positions, token_req, kv_indptr, kv_indices, kv_
 def paged_attention(q, pool, out, qo_indptr, kv_indptr, kv_indices, kv_last_page_len, *, heads: int, scale: float,
                     softcap: float = 0.0, sinks=None, items=None, req_count: int = 0, chunk_pages: int = 0,
                     max_chunks: int = 1, workspace=None, dist=None, chunk: int = 0, kv_first=None, ld_q: int = 0,
-                    status=None) -> None:
+                    status=None, counts=None) -> None:
     """The tensor-core kernels with capped scores, sinks, distance biases, chunks and probabilities in two parts: portions (``items`` [n, 3]: request,
     first token, tokens) on the prefill kernel, else single tokens of the first ``req_count`` requests."""
     _f32(sinks, "sinks"); _f32(dist, "dist")
@@ -273,6 +273,7 @@ def paged_attention(q, pool, out, qo_indptr, kv_indptr, kv_indices, kv_last_page
         _check(lib().nfk_attn_prefill_ws(byref(p), _stream()), "nfk_attn_prefill_ws")
         return
     p.req_count, p.chunk_pages, p.max_chunks, p.workspace = req_count, chunk_pages, max_chunks, _p(workspace)
+    p.counts = _decode_counts(counts)
     _check(lib().nfk_attn_decode(byref(p), _stream()), "nfk_attn_decode")
 
 

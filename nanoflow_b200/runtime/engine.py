@@ -201,6 +201,7 @@ class Engine:
             status=torch.zeros(1, dtype=torch.int32, device=dev),
             decode_ws=torch.empty(DECODE_SPLIT_ROWS * DECODE_MAX_CHUNKS * (m.head_dim + 2), dtype=torch.float32,
                                   device=dev),
+            decode_counts=ops.decode_counts(dev),
             meta=meta, nano_items=nano_items,
             gemm_ws=torch.zeros(GEMM_WS_BYTES // 4, dtype=torch.float32, device=dev),
             rope_table=torch.zeros(T, m.head_dim // 2, 2, dtype=torch.float32, device=dev),

@@ -317,6 +317,7 @@ class LayerListEngine(Engine):
         self.moe_zeros = torch.zeros_like(self.moe_counts)
         self.moe_counts_of = [c for c in self.moe_counts[:sum(sizes)].split(sizes)] if sum(sizes) else [None] * len(sizes)
         self.decode_ws = torch.empty(max(8, self._decode_ws_floats()), dtype=f32, device=dev)
+        self.decode_counts = ops.decode_counts(dev)
         self.chunk_ws = torch.empty(max(8, self._chunk_scratch_floats()), dtype=f32, device=dev)
         self.h_s = P(self.S_cap, m.width_p, dt, "sample_h")
         self.logits = P(self.S_cap, m.vocab_p, f32, "logits")
@@ -656,7 +657,7 @@ class LayerListEngine(Engine):
                 return p
 
             d = params()
-            d.workspace, d.max_chunks = _ptr(self.decode_ws), 1
+            d.workspace, d.counts, d.max_chunks = _ptr(self.decode_ws), _ptr(self.decode_counts), 1
             self._op(f"R{r}.attn_decode", d, kernel="nfk_attn_decode",
                      dyn=[("req_count", "n_dec"), ("chunk_pages", g.symbol("dec_chunk_pages")),
                           ("max_chunks", g.symbol("dec_max_chunks"))], layer=r)

@@ -68,6 +68,7 @@ class Buffers:
     attn_full: Optional[torch.Tensor] = None  # [T, q_size] symmetric: all ranks' attention outputs side by side
                                               # (only with nano-batches whose O projection takes the all-gather form)
     rope_table: Optional[torch.Tensor] = None  # [T, head_dim/2, 2] fp32 angles of the iteration's tokens
+    decode_counts: Optional[torch.Tensor] = None   # of the decode attention launches, which all share one stream
 
 
 class CollectiveHooks:
@@ -304,7 +305,7 @@ def build_graph(model: ModelConfig, eng: EngineConfig, w: RankWeights, bufs: Buf
                 dp.num_ctas = _ops.sm_count(st.device)   # one CTA per SM: a second would not fit beside a GEMM CTA
             if dp.decode_stages == 0:
                 dp.decode_stages = 2 # 64 KB: leaves room for a collective's CTA beside GEMM + decode
-        dp.workspace = _ptr(bufs.decode_ws)
+        dp.workspace, dp.counts = _ptr(bufs.decode_ws), _ptr(bufs.decode_counts)
         dec_kernel = "nfk_attn_decode_tma" if (eng.decode_impl == "tma" and hd == 128) else "nfk_attn_decode"
         dec = g.add(f"L{l}.nb{k}.attn_decode", dp, S("attn"), deps=[ro], kernel=dec_kernel,
                     dyn=[("req_begin", nb_dec0[k]), ("req_count", nb_decn[k]), ("chunk_pages", nb_chunk_pages[k]),

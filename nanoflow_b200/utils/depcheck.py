@@ -13,6 +13,7 @@ from __future__ import annotations
 
 from typing import Dict, List, Tuple
 
+from ..ops import DECODE_COUNTS
 from ..runtime.graph import OpGraph
 
 Range = Tuple[int, int]   # [begin, end) device addresses
@@ -128,6 +129,8 @@ def graph_access(graph: OpGraph, nano_starts: List[int], nano_sizes: List[int], 
             half = cap // 2
             if op.kernel == "nfk_attn_decode":
                 add(writes, rng(p.out + r0 * w * 2, half, w, w))
+                if p.counts:
+                    add(writes, (int(p.counts), int(p.counts) + 4 * DECODE_COUNTS))
             else:
                 add(writes, rng(p.out + (r0 + half) * w * 2, cap - half, w, w))
             if kv_pool_bytes:

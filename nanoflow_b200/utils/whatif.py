@@ -103,6 +103,7 @@ def structural_graph(tp: int, nano: Sequence[int], layers: int, pipeline_type: s
 
     from ..config import builtin_config
     from ..models import random_full_weights, shard_weights
+    from ..ops import decode_counts
     from ..parallel.collectives import TpCollectives
     from ..runtime.pipeline import Buffers, IoSpec, build_graph
 
@@ -134,7 +135,7 @@ def structural_graph(tp: int, nano: Sequence[int], layers: int, pipeline_type: s
                    logits=z(B, w.lm_head.shape[0]), cand_val=sym(tp, B, dtype=torch.float32),
                    cand_idx=sym(tp, B, dtype=torch.int32), sampled=z(B, dtype=torch.int32), kv_pool=pools,
                    inv_freq=torch.zeros(m.head_dim // 2), status=torch.zeros(1, dtype=torch.int32),
-                   decode_ws=torch.zeros(1024), meta=meta,
+                   decode_ws=torch.zeros(1024), decode_counts=decode_counts("cpu"), meta=meta,
                    nano_items=[torch.zeros(s + 2, 3, dtype=torch.int32) for s in sizes],
                    gemm_ws=torch.zeros(1 << 16))
     g = build_graph(m, e, w, bufs, coll, IoSpec(meta_dev, 4 * T, 8 * T))
