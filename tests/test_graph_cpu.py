@@ -6,7 +6,6 @@ import torch
 
 from nanoflow_b200.config import builtin_config
 from nanoflow_b200.models import random_full_weights, shard_weights
-from nanoflow_b200.ops import DECODE_COUNTS, decode_counts
 from nanoflow_b200.parallel.collectives import TpCollectives
 from nanoflow_b200.runtime.pipeline import Buffers, IoSpec, build_graph
 from nanoflow_b200.utils import depcheck
@@ -46,7 +45,7 @@ def _host_graph(pipeline_type, tp, nano, gbs=48, fuse_rs=False, net_streams=1, f
                    logits=z(B, w.lm_head.shape[0]), cand_val=sym(tp, B, dtype=torch.float32),
                    cand_idx=sym(tp, B, dtype=torch.int32), sampled=z(B, dtype=torch.int32), kv_pool=pools,
                    inv_freq=torch.zeros(m.head_dim // 2), status=torch.zeros(1, dtype=torch.int32),
-                   decode_ws=torch.zeros(1024), decode_counts=decode_counts("cpu"), meta=meta,
+                   decode_ws=torch.zeros(1024), meta=meta,
                    nano_items=[torch.zeros(s + 2, 3, dtype=torch.int32) for s in sizes],
                    gemm_ws=torch.zeros(1 << 16),
                    attn_full=sym(T, m.q_size_local * tp) if (o_allgather and tp > 1) else None)
@@ -593,19 +592,3 @@ def test_an_engine_cuts_per_nano_batch(budget):
     for k, p in enumerate((per[:12], per[12:], per[:0])):
         assert (sym[f"nb{k}_chunk_pages"], sym[f"nb{k}_max_chunks"]) == E.decode_split(p, 32, 8, ctas)
     assert sym["nb0_max_chunks"] > 1 and sym["nb2_chunk_pages"] == 0
-
-
-@pytest.mark.parametrize("pipeline_type,tp,nano", [("NON_OVERLAP_LOCAL", 1, None), ("LOCAL", 1, [16, 32]), ("PLLM", 2, [16, 16, 16])])
-def test_decode_launches_count_in_memory_of_their_own_engine(pipeline_type, tp, nano):
-    """Work and finished chunks are counted in the engine's own words (two engines on one GPU may run at the same time), which
-    the engine's own launches use one after the other."""
-    graphs = [_host_graph(pipeline_type, tp, nano) for _ in range(2)]
-    used = [{op.params.counts for op in g.ops if op.kernel == "nfk_attn_decode"} for g, _, _ in graphs]
-    for (g, acc, (bufs, *_)), mine in zip(graphs, used):
-        assert mine == {bufs.decode_counts.data_ptr()} and bufs.decode_counts.numel() >= DECODE_COUNTS
-        assert not depcheck.check(g, acc)
-        # launches that were not ordered would be seen
-        at = [i for i, op in enumerate(g.ops) if op.kernel == "nfk_attn_decode"]
-        g.ops[at[1]].stream, g.ops[at[1]].deps = "elsewhere", []
-        assert any(at[1] in pair for pair in depcheck.check(g, acc))
-    assert not used[0] & used[1]
