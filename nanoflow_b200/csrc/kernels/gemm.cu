@@ -374,9 +374,14 @@ struct Walk {
 // its own so that the others keep their registers.
 constexpr int kGatedBias = 3;
 constexpr bool gated_epi(int epi) { return epi == 1 || epi == kGatedBias; }
+// Most registers of a thread: what other streams' kernels find beside a GEMM's CTA hangs on it. An SM's registers are four banks
+// of 16384 for the warps of one scheduler each, and two of the six warps share two of them: at 104 registers 9728 are left there
+// (a decode CTA, or two small collective CTAs of 152 registers a thread), at the 154 that the plain epilogue would take 6144. Gated
+// epilogues keep what they take (111 to 128).
+constexpr int gemm_registers(int mt, int epi) { return epi != 0 ? 255 : mt == 1 ? 104 : 120; }
 
 template <int MT, int EPI, int CG, bool WIDE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __maxnreg__(gemm_registers(MT, EPI))
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
                     const __grid_constant__ CUtensorMap tmB1, DevParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -703,72 +708,94 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               gated_acts<16>(gsum, usum, p.act);
               if (row_ok && col < tile_col_end) store_cols16(p, row, col, tile_col_end, gsum);
             }
-            continue;
-          }
-          // What the residual adds to a chunk of 32 columns is requested a chunk ahead: D may be C itself, so the compiler
-          // cannot move these loads over the stores of the chunk before, and each eight columns would wait for HBM.
-          const __nv_bfloat16* crow =
-              (EPI == 0 && p.C != nullptr && p.partial == nullptr && mode == 0 && row_ok) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
-          uint4 c_next[4];
-          auto request_c = [&](int c) {
+          } else if constexpr (EPI == 0) {
+            // What the residual adds to 16 columns is requested 32 columns ahead: D may be C itself, so the compiler cannot move
+            // these loads over the stores before them, and each eight columns would wait for HBM. 16 columns at a time: 32 and the
+            // residual of 64 took 154 registers (see gemm_registers).
+            const __nv_bfloat16* crow =
+                (p.C != nullptr && p.partial == nullptr && mode == 0 && row_ok) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
+            uint4 c_in[4] = {};
+            auto request_c = [&](int h, int c) {
 #pragma unroll
-            for (int g8 = 0; g8 < 4; ++g8) {
-              const int col = nb.col0 + c * 32 + g8 * 8;
-              c_next[g8] = col < tile_col_end ? *reinterpret_cast<const uint4*>(crow + col) : make_uint4(0, 0, 0, 0);
-            }
-          };
-          if (EPI == 0 && crow != nullptr) request_c(0);
-#pragma unroll 1
-          for (int c = 0; c * 32 < OUT_BN; ++c) {
-            uint32_t r[32];
-            float v[32];
-            const bool tail16 = (c * 32 + 16 == OUT_BN);               // width = 32k + 16: last chunk is half
-            const int nval = tail16 ? 16 : 32;
-            if (tail16) tmem_ld_32x32b_x16(t_lane + mt * BN + c * 32, r);
-            else tmem_ld_32x32b_x32(t_lane + mt * BN + c * 32, r);
-            uint4 c_now[4];
-            if (EPI == 0 && crow != nullptr) {
-#pragma unroll
-              for (int g8 = 0; g8 < 4; ++g8) c_now[g8] = c_next[g8];
-              if ((c + 1) * 32 < OUT_BN) request_c(c + 1);
-            }
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
-            if (EPI == 0 && mode == 1) {
-              if (row_ok) {
-                float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
-#pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8)
-                  if (g8 * 8 < nval) store_part8(own + c * 32 + g8 * 8, v + g8 * 8, p.part_wide);
+              for (int g8 = 0; g8 < 2; ++g8) {
+                const int col = nb.col0 + c + g8 * 8;
+                if (col < tile_col_end) c_in[h * 2 + g8] = *reinterpret_cast<const uint4*>(crow + col);
               }
-              continue;
+            };
+            if (crow != nullptr) {
+              request_c(0, 0);
+              request_c(1, 16);
             }
-            const int col0 = nb.col0 + c * 32;
-            if (EPI == 0 && p.partial != nullptr) {
-              if (row_ok && col0 < tile_col_end) {
-                float* prow = p.partial + (static_cast<long long>(sg.ks) * p.M + row) * p.N;
+#pragma unroll 1
+            for (int c0 = 0; c0 < OUT_BN; c0 += 32) {
 #pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8) {
-                  const int col = col0 + g8 * 8;
-                  if (col < tile_col_end) store_part8(prow + col, v + g8 * 8, p.part_wide);
+              for (int h = 0; h < 2; ++h) {
+                const int c = c0 + h * 16, col0 = nb.col0 + c;
+                uint32_t r[16];
+                float v[16];
+                tmem_ld_32x32b_x16n(t_lane + mt * BN + c, r);
+                const uint4 c_now[2] = {c_in[h * 2], c_in[h * 2 + 1]};
+                if (crow != nullptr && c + 32 < OUT_BN) request_c(h, c + 32);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
+                if (mode == 1) {
+                  if (row_ok) {
+                    float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
+#pragma unroll
+                    for (int g8 = 0; g8 < 2; ++g8) store_part8(own + c + g8 * 8, v + g8 * 8, p.part_wide);
+                  }
+                } else if (p.partial != nullptr) {
+                  if (row_ok) {
+                    float* prow = p.partial + (static_cast<long long>(sg.ks) * p.M + row) * p.N;
+#pragma unroll
+                    for (int g8 = 0; g8 < 2; ++g8)
+                      if (col0 + g8 * 8 < tile_col_end) store_part8(prow + col0 + g8 * 8, v + g8 * 8, p.part_wide);
+                  }
+                } else if (row_ok && col0 < tile_col_end) {
+#pragma unroll
+                  for (int g8 = 0; g8 < 2; ++g8) {
+                    const int col = col0 + g8 * 8;
+                    if (col < tile_col_end) {  // N is a multiple of 8
+                      float* vv = v + g8 * 8;
+                      if (p.bias != nullptr) add_bias8(vv, p.bias + col);
+                      if (crow != nullptr) {
+                        const uint32_t cw[4] = {c_now[g8].x, c_now[g8].y, c_now[g8].z, c_now[g8].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                          const float2 f = unpack_bf16x2(cw[j]);
+                          vv[2 * j] += p.beta * f.x;
+                          vv[2 * j + 1] += p.beta * f.y;
+                        }
+                      }
+                    }
+                  }
+                  store_cols16(p, row, col0, tile_col_end, v);
                 }
               }
-              continue;
             }
-            if (EPI == 2 && p.rs_staged) {
-              // Staged push: this lane's 32 columns go to its row of the warp's staging piece; when a
-              // run of 128 columns (or the tile's last columns) is complete, one bulk copy per lane
-              // sends the row's run to the owner's slab. A lane only ever reads back what it wrote, so
-              // the generic -> async proxy fence is all the ordering the copy needs.
-              uint8_t* stage_row = smem + STAGES * STAGE_BYTES + (q * 32 + lane) * kRsRowPitch;
-              // the bulk copy of the previous run reads this row: it must be done reading before the first
-              // write of a new run (waiting here, not right after the copy, lets the copy run under the
-              // accumulator loads in between)
-              if ((c & 3) == 0) tma_store_wait_read<0>();
+          } else {
+#pragma unroll 1
+            for (int c = 0; c * 32 < OUT_BN; ++c) {
+              uint32_t r[32];
+              float v[32];
+              tmem_ld_32x32b_x32(t_lane + mt * BN + c * 32, r);
+              tmem_ld_wait();
 #pragma unroll
-              for (int g8 = 0; g8 < 4; ++g8) {
-                if (g8 * 8 < nval) {
+              for (int j = 0; j < 32; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
+              const int col0 = nb.col0 + c * 32;
+              if (p.rs_staged) {
+                // Staged push: this lane's 32 columns go to its row of the warp's staging piece; when a
+                // run of 128 columns (or the tile's last columns) is complete, one bulk copy per lane
+                // sends the row's run to the owner's slab. A lane only ever reads back what it wrote, so
+                // the generic -> async proxy fence is all the ordering the copy needs.
+                uint8_t* stage_row = smem + STAGES * STAGE_BYTES + (q * 32 + lane) * kRsRowPitch;
+                // the bulk copy of the previous run reads this row: it must be done reading before the first
+                // write of a new run (waiting here, not right after the copy, lets the copy run under the
+                // accumulator loads in between)
+                if ((c & 3) == 0) tma_store_wait_read<0>();
+#pragma unroll
+                for (int g8 = 0; g8 < 4; ++g8) {
                   const float* vv = v + g8 * 8;
                   uint4 o;
                   o.x = pack_bf16x2(vv[0], vv[1]);
@@ -777,27 +804,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                   o.w = pack_bf16x2(vv[6], vv[7]);
                   *reinterpret_cast<uint4*>(stage_row + (c & 3) * 64 + g8 * 16) = o;
                 }
-              }
-              const bool run_done = (c & 3) == 3 || (c + 1) * 32 >= OUT_BN;
-              if (run_done) {
-                const int run_col0 = n_blk * OUT_BN + (c & ~3) * 32;
-                int run_end = n_blk * OUT_BN + c * 32 + nval;
-                if (run_end > tile_col_end) run_end = tile_col_end;
-                fence_proxy_async_smem();
-                if (row_ok && run_end > run_col0) {
-                  const int owner = row % p.rs_nranks;
-                  __nv_bfloat16* srow = reinterpret_cast<__nv_bfloat16*>(p.rs_heap[owner] + p.rs_slab_off) +
-                                        (static_cast<long long>(p.rs_rank) * p.rs_rows_cap + row / p.rs_nranks) * p.N;
-                  bulk_store_1d(srow + run_col0, stage_row, static_cast<uint32_t>(run_end - run_col0) * 2u);
+                const bool run_done = (c & 3) == 3 || (c + 1) * 32 >= OUT_BN;
+                if (run_done) {
+                  const int run_col0 = n_blk * OUT_BN + (c & ~3) * 32;
+                  int run_end = n_blk * OUT_BN + (c + 1) * 32;
+                  if (run_end > tile_col_end) run_end = tile_col_end;
+                  fence_proxy_async_smem();
+                  if (row_ok && run_end > run_col0) {
+                    const int owner = row % p.rs_nranks;
+                    __nv_bfloat16* srow = reinterpret_cast<__nv_bfloat16*>(p.rs_heap[owner] + p.rs_slab_off) +
+                                          (static_cast<long long>(p.rs_rank) * p.rs_rows_cap + row / p.rs_nranks) * p.N;
+                    bulk_store_1d(srow + run_col0, stage_row, static_cast<uint32_t>(run_end - run_col0) * 2u);
+                  }
+                  tma_store_commit();
                 }
-                tma_store_commit();
-              }
-              continue;
-            }
-            if (EPI == 2) {
-              // push the partial row to its owner's slab (posted NVLink stores; the flag raised at
-              // the end of the kernel orders them for the reader)
-              if (row_ok && col0 < tile_col_end) {
+              } else if (row_ok && col0 < tile_col_end) {
+                // push the partial row to its owner's slab (posted NVLink stores; the flag raised at
+                // the end of the kernel orders them for the reader)
                 const int owner = row % p.rs_nranks;
                 __nv_bfloat16* srow = reinterpret_cast<__nv_bfloat16*>(p.rs_heap[owner] + p.rs_slab_off) +
                                       (static_cast<long long>(p.rs_rank) * p.rs_rows_cap + row / p.rs_nranks) * p.N;
@@ -815,29 +838,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                   }
                 }
               }
-              continue;
-            }
-            if (row_ok && col0 < tile_col_end) {
-#pragma unroll
-              for (int g8 = 0; g8 < 4; ++g8) {
-                const int col = col0 + g8 * 8;
-                if (EPI == 0 && col < tile_col_end) {  // N is a multiple of 8
-                  float* vv = v + g8 * 8;
-                  if (p.bias != nullptr) add_bias8(vv, p.bias + col);
-                  if (crow != nullptr) {
-                    const uint32_t cw[4] = {c_now[g8].x, c_now[g8].y, c_now[g8].z, c_now[g8].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                      const float2 f = unpack_bf16x2(cw[j]);
-                      vv[2 * j] += p.beta * f.x;
-                      vv[2 * j + 1] += p.beta * f.y;
-                    }
-                  }
-                }
-              }
-#pragma unroll
-              for (int g16 = 0; g16 < 2; ++g16)
-                if (col0 + g16 * 16 < tile_col_end) store_cols16(p, row, col0 + g16 * 16, tile_col_end, v + g16 * 16);
             }
           }
         }

@@ -1,0 +1,21 @@
+"""Registers that a CTA of the linear GEMM leaves to other streams' kernels on its SM."""
+import re
+import subprocess
+
+from nanoflow_b200.ops.build import ARCH_FLAGS, KERNEL_DIR, NVCC, NVCC_FLAGS
+
+BANK = 16384                                   # an SM's registers are four banks, one to a scheduler
+GEMM_WARPS = 2                                 # most of the six warps of a CTA that share a bank
+
+
+def test_a_linear_gemm_leaves_registers_for_its_neighbours(tmp_path):
+    log = subprocess.run([NVCC, *ARCH_FLAGS, *NVCC_FLAGS, "-Xptxas", "-v", "-I", str(KERNEL_DIR), "-c", str(KERNEL_DIR / "gemm.cu"),
+                          "-o", str(tmp_path / "gemm.o")], capture_output=True, text=True, check=True).stderr
+    # gemm_tcgen05_kernel<M tiles, epilogue, CTAs per tile, wide> with epilogue 0 (mangled: Li1ELi0E...)
+    found = re.findall(r"entry function '\S*gemm_tcgen05_kernelILi(\d)ELi0ELi(\d)ELb(\d)E\S*' for.*?(\d+) bytes spill stores.*?Used (\d+) registers", log, re.S)
+    assert len(found) == 5                     # 1, 2 and 4 M tiles; pairs; pairs with wide tiles
+    for m_tiles, ctas, wide, spilled, regs in found:
+        left = BANK - GEMM_WARPS * 32 * (-(-int(regs) // 8) * 8)
+        # two CTAs of four warps with 152 registers a thread (a collective without a norm), or with several M tiles 136
+        need = 2 * 32 * (152 if m_tiles == "1" else 136)
+        assert int(spilled) == 0 and left >= need, (m_tiles, ctas, wide, regs)
