@@ -26,6 +26,7 @@
 #include "gated_act.cuh"
 #include "kernels.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace nf {
@@ -1722,26 +1723,44 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
   return s;
 }
 
+// us of `tiles` tiles of the mid-rows kernel at once, one to a cluster.
+double mid_rows_round(const MidPlan& f, int cols, int tiles) {
+  const double pairs = static_cast<double>(tiles) * f.split;
+  const double pair_us = 1.25e-3 * cols;                                            // a pair's products, per k-block
+  const double chip_us = pairs * cols * (2.0 * 256 * BK) / 1.41e9;                  // those of all pairs under the power limit: 1.41 PFLOP/s
+  const double weight_us = 0.0835 + pairs * 2.0 * kFewWBytes / f.tok_tiles / 7.57e6;   // the weights' way from HBM
+  return f.kb_per * std::max(std::max(pair_us, chip_us), weight_us) + 2.37 + 0.0233 * cols;   // set-up; a token's way out
+}
+
 // Whether the mid-rows kernel takes a call for which the tile kernel would have shape `s`, and with how many parts of K (stages
 // 0: it does not). rows_kernel 4 asks for it with split_k parts.
 //
-// Its cost by the same model, fitted to 15 numbers of rows from 64 to 1000 of ten products: what a k-block takes is the largest
-// of the products (1.24 ns per token), what enters the SMs of all pairs at once (11.7 TB/s), the weights' way from HBM (7.2 TB/s)
-// and 0.21 us. The two models' choice is 0.8 % slower than the best of all shapes on average, at worst 12 %; the tile kernel
-// alone, with the constants before, 3.4 % slower than the best of its own. us, tile kernel -> this one: 8192 x 28672 at 160 rows
-// 96 -> 82, 288 153 -> 107, 384 163 -> 133, 700 254 -> 232; 8192 x 8192 at 160 39.5 -> 31, 333 49 -> 42; 4096 x 14336 at 288
-// 45 -> 39; 28672 x 2 x 8192 at 288 285 -> 266. On the other side of the line: 8192 x 28672 at 512 166 (170 here), 1000 315 (317);
-// 4096 x 4096 at 333 21.4 (23.2); 14336 x 2 x 4096 at 256 52 (70), 333 81 (84).
+// The line is drawn by the two kernels' models; 7 % are in hand for their errors, and the tile kernel's counts 1.2 us less of
+// what a product costs beside its loop. K is cut only where all tiles run at once (a second round of clusters starts late:
+// 28672 x 2 x 8192 at 333 rows 328 us in two parts, 318 in one, tile kernel 278). Fitted to 21 products (2048 to 128256 columns,
+// K 2048 to 28672, five of them gated) at 30 numbers of rows from 64 to 1100, in a chain of products with cold weights, with the
+// residual in place where a model has one. Beside the fastest of both kernels the choice is 0.4 % slower on average and at worst
+// 13 % (5120 x 5120 at 97 rows, which the tile kernel gets: 18.9 us, here 16.7); fitted to half of the products, as good on the
+// others. With no limit on the products of all pairs together it was 1.9 % and 29 %, up to 23 % slower than without this kernel.
+// us, tile kernel -> this one where it is taken: 8192 x 28672 at 160 rows 99 -> 87, 288 156 -> 114, 384 161 -> 144, 576 257 -> 222;
+// 8192 x 8192 at 160 37 -> 33, 288 51 -> 41, 576 81 -> 66; 4096 x 14336 at 288 45 -> 39, 576 70 -> 58; 32000 x 8192 at 288 152 -> 139;
+// 18944 x 2 x 3584 at 288 84 -> 77. On the other side of the line: 8192 x 28672 at 256 rows 108 (here 112), 512 176 (188), 1000 325
+// (370); 4096 x 4096 at 333 19 (24); 10240 x 8192 at 160 42 (44); 32000 x 8192 at 333 155 (168), 896 337 (377); 14336 x 2 x 4096 at 256
+// 56 (74), 333 77 (90); 28672 x 2 x 8192 at 288 272 (274), 896 596 (781).
+// Fewer rows come here where the few-rows kernel does not take them. Without a workspace (one sum in the order of k) 4096 x 4096
+// at 8 rows 26.3 -> 19.5, 96 22.0 -> 21.1, 128 22.2 -> 21.9; 4096 x 14336 at 64 60.4 -> 51.4; from 129 to 256, where the tile kernel
+// works in pairs of 256 rows, it stays: 160 20.2 (here 23.1), 4096 x 14336 51.4 (54.1). With keep_order 128256 x 4096 at 16
+// rows stays (166; here 193).
 //
 // With keep_order K stays cut as the tile kernel's shape cuts it, which gives the same bits.
 MidPlan mid_rows_takes(const nfk_gemm_params& g, const Shape& s) {
   const bool gated = g.epilogue == NFK_EPI_SWIGLU;
   if (!cluster_forms(g) || g.groups > 1) return MidPlan{};
   if (g.rows_kernel != 4 && (g.rows_kernel != 0 || g.M > 1024 || g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0 ||
-                             g.stream_k != 0 || (g.keep_order != 0 && s.stream_k)))
+                             g.stream_k != 0 || (g.keep_order != 0 && s.stream_k) || (g.workspace == nullptr && g.M > 128 && g.M <= 256)))
     return MidPlan{};
   MidPlan best{};
-  double best_us = g.rows_kernel == 4 ? 1e30 : s.us - 4.35;
+  double best_us = g.rows_kernel == 4 ? 1e30 : 0.93 * s.us + 1.2;
   const int lo = g.rows_kernel == 4 ? (g.split_k > 0 ? g.split_k : 1) : g.keep_order != 0 ? s.split_k : 1;
   const int hi = g.rows_kernel == 4 || g.keep_order != 0 ? lo : g.workspace == nullptr ? 1 : 4;   // without a workspace: one sum in the order of k
   for (int split = lo; split <= hi; ++split) {
@@ -1749,14 +1768,9 @@ MidPlan mid_rows_takes(const nfk_gemm_params& g, const Shape& s) {
     if (f.stages < 2 || f.round_tokens < 32) continue;
     const int fit = f.nb2 > 0 ? (gated ? resident_mid_clusters<true, true>(2 * split) : resident_mid_clusters<false, true>(2 * split))
                               : (gated ? resident_mid_clusters<true, false>(2 * split) : resident_mid_clusters<false, false>(2 * split));
-    const int tiles = f.n_tiles * f.tok_tiles, cols = f.nb + f.nb2, pairs = (tiles < fit ? tiles : fit) * split;
-    double kb = 1.24e-3 * cols;
-    const double enter = pairs * 2.0 * (kFewWBytes + 64.0 * cols) / 11.7e6, weights = pairs * 2.0 * kFewWBytes / f.tok_tiles / 7.16e6;
-    kb = kb > enter ? kb : enter;
-    kb = kb > weights ? kb : weights;
-    kb = kb > 0.206 ? kb : 0.206;
-    const double one = f.kb_per * kb + 3.98 + 0.0203 * cols + (split > 1 ? 0.56 : 0.0) + 1.25 * ((cols + f.round_tokens - 1) / f.round_tokens - 1);
-    const double us = one * ((tiles + fit - 1) / fit);
+    const int tiles = f.n_tiles * f.tok_tiles, cols = f.nb + f.nb2;
+    if (g.rows_kernel != 4 && split > 1 && tiles > fit) continue;
+    const double us = (tiles / fit) * mid_rows_round(f, cols, fit) + (tiles % fit != 0 ? mid_rows_round(f, cols, tiles % fit) : 0.0);
     if (us < best_us) {
       best_us = us;
       best = f;
