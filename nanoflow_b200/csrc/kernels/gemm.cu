@@ -710,11 +710,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               if (row_ok && col < tile_col_end) store_cols16(p, row, col, tile_col_end, gsum);
             }
           } else if constexpr (EPI == 0) {
+            // Partial sums, of a split K or of a piece of a stream-K tail, as they are.
+            if (mode == 1 || p.partial != nullptr) {
+              float* prow = mode == 1 ? sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local
+                                      : p.partial + (static_cast<long long>(sg.ks) * p.M + row) * p.N + nb.col0;
+              const int end = !row_ok ? 0 : mode == 1 ? OUT_BN : tile_col_end - nb.col0;
+#pragma unroll 1
+              for (int c = 0; c < OUT_BN; c += 32) {
+                uint32_t r[32];
+                float v[32];
+                tmem_ld_32x32b_x32(t_lane + mt * BN + c, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
+#pragma unroll
+                for (int g8 = 0; g8 < 4; ++g8)
+                  if (c + g8 * 8 < end) store_part8(prow + c + g8 * 8, v + g8 * 8, p.part_wide);
+              }
+              continue;
+            }
             // What the residual adds to 16 columns is requested 32 columns ahead: D may be C itself, so the compiler cannot move
             // these loads over the stores before them, and each eight columns would wait for HBM. 16 columns at a time: 32 and the
             // residual of 64 took 154 registers (see gemm_registers).
-            const __nv_bfloat16* crow =
-                (p.C != nullptr && p.partial == nullptr && mode == 0 && row_ok) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
+            const __nv_bfloat16* crow = (p.C != nullptr && row_ok) ? p.C + static_cast<long long>(row) * p.ldc : nullptr;
             uint4 c_in[4] = {};
             auto request_c = [&](int h, int c) {
 #pragma unroll
@@ -740,20 +758,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = empty_range ? 0.f : __uint_as_float(r[j]);
-                if (mode == 1) {
-                  if (row_ok) {
-                    float* own = sk_tile_base + (static_cast<long long>(sg.piece) * CG + rank) * slot_floats + row_local;
-#pragma unroll
-                    for (int g8 = 0; g8 < 2; ++g8) store_part8(own + c + g8 * 8, v + g8 * 8, p.part_wide);
-                  }
-                } else if (p.partial != nullptr) {
-                  if (row_ok) {
-                    float* prow = p.partial + (static_cast<long long>(sg.ks) * p.M + row) * p.N;
-#pragma unroll
-                    for (int g8 = 0; g8 < 2; ++g8)
-                      if (col0 + g8 * 8 < tile_col_end) store_part8(prow + col0 + g8 * 8, v + g8 * 8, p.part_wide);
-                  }
-                } else if (row_ok && col0 < tile_col_end) {
+                if (row_ok && col0 < tile_col_end) {
 #pragma unroll
                   for (int g8 = 0; g8 < 2; ++g8) {
                     const int col = col0 + g8 * 8;
