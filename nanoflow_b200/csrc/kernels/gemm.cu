@@ -1469,7 +1469,7 @@ int resident_clusters(Kernel* kernel, int size, int& known) {
   return known;
 }
 
-// What a B200 answers, for planning without one.
+// What one B200 answers (another 45, 33, 26, 22, 15, 15 from three CTAs on), for planning without one.
 constexpr int kResidentClusters[kSplitMaxCluster + 1] = {0, 148, 74, 47, 35, 27, 22, 18, 14};
 
 template <int CG>
@@ -1908,6 +1908,8 @@ extern "C" int nfk_gemm_describe(const nfk_gemm_params* given, nfk_gemm_plan* ou
   out->few_rows = few_rows_takes(*g) ? 1 : 0;
   const MidPlan mid = out->few_rows != 0 ? MidPlan{} : mid_rows_takes(*g, s);
   out->mid_rows = mid.stages >= 2 ? mid.split : 0;
+  const SplitPlan split = out->few_rows != 0 || out->mid_rows != 0 ? SplitPlan{} : split_in_cluster(*g, s);
+  out->cluster_parts = split.stages >= 2 ? split.split : 0;
   return NF_OK;
 }
 

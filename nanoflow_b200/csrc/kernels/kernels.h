@@ -116,6 +116,7 @@ typedef struct nfk_gemm_plan {
   int stages, smem_bytes;
   int few_rows;                        // 1 = the call goes to the few-rows kernel, and the rest is what the tile kernel would do
   int mid_rows;                        // > 0: the call goes to the mid-rows kernel with so many parts of K, likewise
+  int cluster_parts;                   // > 0: one launch whose clusters add so many parts of K; 0 = split_k in two launches, or K whole
 } nfk_gemm_plan;
 int nfk_gemm_describe(const nfk_gemm_params* p, nfk_gemm_plan* out);
 

@@ -385,7 +385,8 @@ class GemmPlan(Structure):
     _fields_ = [("tile_n", c_int), ("tile_m", c_int), ("cta_group", c_int), ("split_k", c_int), ("stream_k", c_int),
                 ("tiles", c_int), ("workers", c_int), ("num_kb", c_int),
                 ("tail_first_tile", c_int), ("tail_range_kb", c_int), ("tail_max_pieces", c_int),
-                ("stages", c_int), ("smem_bytes", c_int), ("few_rows", c_int), ("mid_rows", c_int)]
+                ("stages", c_int), ("smem_bytes", c_int), ("few_rows", c_int), ("mid_rows", c_int),
+                ("cluster_parts", c_int)]
 
 
 def gemm_plan(M: int, N: int, K: int, *, swiglu: bool = False, tile_n: int = 0, tile_m: int = 0, cta_group: int = 0,
