@@ -190,11 +190,13 @@ gemm_mid_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_cons
     // what the residual adds to an item is requested an item ahead, the first one's while the pieces are on their way
     uint4 c_next[4] = {};
     auto request_c = [&](int i) {
-      const int col = nb.col0 + (i % GR) * 8, row = tok0 + t0 + first + i / GR * 4;
-      if (GATED || p.C == nullptr || i >= items || col >= nb.col_end) return;
+      if constexpr (!GATED) {
+        const int col = nb.col0 + (i % GR) * 8, row = tok0 + t0 + first + i / GR * 4;
+        if (p.C == nullptr || i >= items || col >= nb.col_end) return;
 #pragma unroll
-      for (int t = 0; t < 4; ++t)
-        if (row + t < p.M) c_next[t] = *reinterpret_cast<const uint4*>(p.C + static_cast<long long>(row + t) * p.ldc + col);
+        for (int t = 0; t < 4; ++t)
+          if (row + t < p.M) c_next[t] = *reinterpret_cast<const uint4*>(p.C + static_cast<long long>(row + t) * p.ldc + col);
+      }
     };
     request_c(threadIdx.x);
     if (warp >= 2 && have) {
