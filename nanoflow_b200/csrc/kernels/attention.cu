@@ -96,7 +96,8 @@ constexpr int kDecThreads = 128;
 
 // ST = pages in flight per warp (pipeline stages). 3 is the default (96 KB per CTA at head_dim 128, two
 // CTAs per SM); 2 (64 KB) is for the case where a decode CTA shares an SM with a GEMM CTA and a
-// collective's CTA (130 KB + 64 KB + the per-CTA reserve leave room, 130 KB + 96 KB do not).
+// collective's CTA (130 KB + 64 KB + the per-CTA reserve leave room, 130 KB + 96 KB do not; by their
+// registers 104 of a GEMM and 168 here leave room for a collective with up to 136).
 template <int HD, int ST>
 struct DecCfg {
   static constexpr int PAGE_BYTES = kPage * HD * 2;            // one head's K (or V) page

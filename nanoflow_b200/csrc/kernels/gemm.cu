@@ -376,10 +376,12 @@ struct Walk {
 constexpr int kGatedBias = 3;
 constexpr bool gated_epi(int epi) { return epi == 1 || epi == kGatedBias; }
 // Most registers of a thread: what other streams' kernels find beside a GEMM's CTA hangs on it. An SM's registers are four banks
-// of 16384 for the warps of one scheduler each, and two of the six warps share two of them: at 104 registers 9728 are left there
-// (a decode CTA, or two small collective CTAs of 152 registers a thread), at the 154 that the plain epilogue would take 6144. Gated
-// epilogues keep what they take (111 to 128).
-constexpr int gemm_registers(int mt, int epi) { return epi != 0 ? 255 : mt == 1 ? 104 : 120; }
+// of 16384 for the warps of one scheduler each, and two of the six warps share two of them. At 104 registers 9728 are left there:
+// a decode CTA of three stages (232 registers a thread), or one of two stages (168) and a collective's of up to 136; at the 154
+// that the plain epilogue would take 6144, one CTA of 168. (With known kernels: 192 threads of up to 88 registers leave room for two
+// CTAs of 128 threads with 168, of 96 to 160 for one.) Gated epilogues: 120 (124 without the limit); those with a bias and those of
+// several M tiles keep what they take (111 to 128).
+constexpr int gemm_registers(int mt, int epi) { return epi == 0 ? (mt == 1 ? 104 : 120) : epi == 1 && mt == 1 ? 120 : 255; }
 
 template <int MT, int EPI, int CG, bool WIDE>
 __global__ void __maxnreg__(gemm_registers(MT, EPI))
@@ -1571,16 +1573,16 @@ bool few_rows_takes(const nfk_gemm_params& g) {
   if (g.norm_w != nullptr && (g.ldd != g.N || g.norm_ld != g.N)) return false;
   if (g.rows_kernel == 1) return g.cta_group != 2 || g.groups <= 1;
   if (g.tile_n != 0 || g.tile_m != 0 || g.split_k != 0 || g.cta_group != 0 || g.workspace == nullptr) return false;
-  // Measured in a chain with a small kernel between products, cold weights, this kernel fetching weights early (us, tile kernel
+  // Measured in a chain with a small kernel between products, cold weights, both kernels fetching weights early (us, tile kernel
   // with its own rule -> this one). What it loses by is the tokens that each CTA stages beside its weights.
-  //   Linear: 4096 x 4096 at 48 rows 14.1 -> 12.8, 96 16.2 -> 17.0; 8192 x 8192 at 96 35.1 -> 31.9; 32000 x 8192 at 96
-  //   89.5 -> 91.0; 128256 x 4096 at 48 173 -> 167, at 96 174 -> 199. With fewer CTAs than SMs (1280 x 8192: 80) 64 rows
-  //   16.7 -> 16.4, 96 rows 17.5 -> 19.8.
-  //   Gated, all tiles at once (two CTAs on an SM): 14336 x 4096 at 112 rows 75 -> 54, 192 93 -> 66, 240 99 -> 73; at 256, where
-  //   the tile kernel's rows are full, 73.5 -> 75.2, 18944 x 3584 72 -> 77, 2048 x 4096 28 -> 35. Very few tiles (1024 x 4096,
-  //   64 CTAs): 160 rows 21.8 -> 21.8, 192 21.9 -> 27.1.
-  //   Gated, more than one round: 28672 x 8192 at 112 rows 187 -> 177, 144 214 -> 197, 192 216 -> 222, 256 211 -> 247; 22016 x 8192
-  //   at 112 168 -> 166, 128 159 -> 172, 144 168 -> 172, 192 171 -> 204.
+  //   Linear: 4096 x 4096 at 64 rows 14.3 -> 13.8, 96 14.5 -> 16.8; 8192 x 8192 at 64 32.6 -> 32.9, 96 31.4 -> 34.0; 32000 x 8192
+  //   at 64 89.9 -> 89.1, 96 89.1 -> 93.7; 128256 x 4096 at 48 173 -> 167, 64 171 -> 189.
+  //   Gated, all tiles at once (two CTAs on an SM): 14336 x 4096 at 64 rows 46.1 -> 46.9, 112 46.3 -> 51.9, 224 54.8 -> 66.1; 256,
+  //   on the other side of the line, 55.5 -> 70.3; 18944 x 3584 at 64 49.7 -> 51.0, 224 57.9 -> 70.3.
+  //   Gated, more than one round: 28672 x 8192 at 64 rows 150 -> 156, 112 153 -> 178, 144 183 -> 189, 192 189 -> 234; 22016 x 8192 at
+  //   64 126 -> 141, 144 143 -> 168.
+  // The lines are from before the tile kernel added its parts of K in a cluster and drained gated tiles without a branch per
+  // element (14336 x 4096 at 112 rows then 75 -> 54); as the two kernels are now, all of them would lie at about 64 rows.
   const int groups = g.groups > 1 ? g.groups : 1;
   const bool gated = g.epilogue == NFK_EPI_SWIGLU;
   const int ctas = n_block_count(groups, g.N / groups, gated ? 64 : 128);    // before K is cut

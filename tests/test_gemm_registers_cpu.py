@@ -27,6 +27,11 @@ def test_a_linear_gemm_leaves_registers_for_its_neighbours(log):
         assert int(spilled) == 0 and left >= need, (m_tiles, ctas, wide, regs)
 
 
+def test_a_gated_gemm_takes_no_more_than_120(log):
+    found = re.findall(r"entry function '\S*gemm_tcgen05_kernelILi1ELi1ELi(\d)ELb0E\S*' for.*?(\d+) bytes spill stores.*?Used (\d+) registers", log, re.S)
+    assert len(found) == 2 and all(int(spilled) == 0 and int(regs) <= 120 for _, spilled, regs in found)
+
+
 def test_the_second_pass_of_split_k_keeps_four_blocks_on_an_sm(log):
     spilled, regs = re.search(r"entry function '\S*splitk_reduce_kernel\S*' for.*?(\d+) bytes spill stores.*?Used (\d+) registers", log, re.S).groups()
     assert int(spilled) == 0 and 4 * 256 * int(regs) <= 4 * BANK
