@@ -448,6 +448,15 @@ def small_case(which: str):
         ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
         for _ in range(4):
             ops.gemm_swiglu(a, w, up, workspace=ws)
+    elif which == "gemm_mid":
+        # some hundred rows, 134 MB of weights per call: 288 go to the mid-rows kernel, 256 to a split of K within clusters
+        N, K = 8192, 8192
+        w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02
+        ws = torch.zeros(160 << 20, dtype=torch.uint8, device="cuda")
+        for M in (288, 256):
+            a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+            for _ in range(4):
+                ops.gemm(a, w, workspace=ws)
     elif which == "gemm_shapes":
         # one launch per kernel shape: CTA pair 256 wide, CTA pair 128 wide, single CTA 256 wide
         M, N, K = 4096, 8192, 8192
