@@ -1715,8 +1715,10 @@ Shape search_shape(const nfk_gemm_params& g, bool swiglu) {
   }
   const bool tail = (g.stream_k == 1 && best_tail_cost < 1e30) || best_tail_cost < m.tail_gain * best_cost;
   Shape s = tail ? best_tail : best;
-  // (what kModel says of a shape that the earlier one has chosen)
-  s.us = g.keep_order == 0 ? (tail ? best_tail_cost : best_cost) : tile_cost(kModel, g, swiglu, s.bn, s.mt, s.split_k, s.cg).us;
+  // What kModel says of a shape that the earlier one has chosen. Four M tiles of 128 columns, which it does not choose itself, take
+  // 1.55 times that: 32000 x 8192 at 300 rows 295 us, said 189; 128256 x 4096 555, said 350.
+  s.us = g.keep_order == 0 ? (tail ? best_tail_cost : best_cost)
+                           : tile_cost(kModel, g, swiglu, s.bn, s.mt, s.split_k, s.cg).us * (s.mt == 4 ? 1.55 : 1.0);
   return s;
 }
 
@@ -1752,22 +1754,24 @@ Shape choose_shape(const nfk_gemm_params& g, bool swiglu) {
 // us of `tiles` tiles of the mid-rows kernel at once, one to a cluster.
 double mid_rows_round(const MidPlan& f, int cols, int tiles) {
   const double pairs = static_cast<double>(tiles) * f.split;
-  const double pair_us = 1.25e-3 * cols;                                            // a pair's products, per k-block
-  const double chip_us = pairs * cols * (2.0 * 256 * BK) / 1.41e9;                  // those of all pairs under the power limit: 1.41 PFLOP/s
-  const double weight_us = 0.0835 + pairs * 2.0 * kFewWBytes / f.tok_tiles / 7.57e6;   // the weights' way from HBM
-  return f.kb_per * std::max(std::max(pair_us, chip_us), weight_us) + 2.37 + 0.0233 * cols;   // set-up; a token's way out
+  const double pair_us = 1.33e-3 * cols;                                            // a pair's products, per k-block
+  const double chip_us = pairs * cols * (2.0 * 256 * BK) / 1.42e9;                  // those of all pairs under the power limit: 1.42 PFLOP/s
+  const double weight_us = 0.0964 + pairs * 2.0 * kFewWBytes / f.tok_tiles / 8.6e6;    // the weights' way from HBM
+  return f.kb_per * std::max(std::max(pair_us, chip_us), weight_us) + 3.38 + 0.026 * cols;    // set-up; a token's way out
 }
 
 // Whether the mid-rows kernel takes a call for which the tile kernel would have shape `s`, and with how many parts of K (stages
 // 0: it does not). rows_kernel 4 asks for it with split_k parts.
 //
-// The line is drawn by the two kernels' models; 7 % are in hand for their errors, and the tile kernel's counts 1.2 us less of
+// The line is drawn by the two kernels' models; 8 % are in hand for their errors, and the tile kernel's counts 2.4 us less of
 // what a product costs beside its loop. K is cut only where all tiles run at once (a second round of clusters starts late:
-// 28672 x 2 x 8192 at 333 rows 328 us in two parts, 318 in one, tile kernel 278). Fitted to 21 products (2048 to 128256 columns,
-// K 2048 to 28672, five of them gated) at 30 numbers of rows from 64 to 1100, in a chain of products with cold weights, with the
-// residual in place where a model has one. Beside the fastest of both kernels the choice is 0.4 % slower on average and at worst
-// 13 % (5120 x 5120 at 97 rows, which the tile kernel gets: 18.9 us, here 16.7); fitted to half of the products, as good on the
-// others. With no limit on the products of all pairs together it was 1.9 % and 29 %, up to 23 % slower than without this kernel.
+// 28672 x 2 x 8192 at 333 rows 328 us in two parts, 318 in one, tile kernel 278). The constants are those that choose best over
+// 21 products (2048 to 128256 columns, K 2048 to 28672, five of them gated) at 30 numbers of rows from 64 to 1100, in a chain of
+// products with cold weights, with the residual in place where a model has one, and over ten of them with the order kept and
+// without a workspace. Beside the fastest of both kernels the choice is 0.2 % slower on average; 13 of 916 are more than 5 % behind,
+// at worst 20 % (2048 x 8192 at 700 rows in the kept order's three parts: 33.4 us, tile kernel 27.9; 5120 x 5120 at 97 rows, which the
+// tile kernel gets: 18.8, here 16.5). With no limit on the products of all pairs together it was 1.9 % and 29 %, up to 23 % slower
+// than without this kernel.
 // us, tile kernel -> this one where it is taken: 8192 x 28672 at 160 rows 99 -> 87, 288 156 -> 114, 384 161 -> 144, 576 257 -> 222;
 // 8192 x 8192 at 160 37 -> 33, 288 51 -> 41, 576 81 -> 66; 4096 x 14336 at 288 45 -> 39, 576 70 -> 58; 32000 x 8192 at 288 152 -> 139;
 // 18944 x 2 x 3584 at 288 84 -> 77. On the other side of the line: 8192 x 28672 at 256 rows 108 (here 112), 512 176 (188), 1000 325
@@ -1786,7 +1790,7 @@ MidPlan mid_rows_takes(const nfk_gemm_params& g, const Shape& s) {
                              g.stream_k != 0 || (g.keep_order != 0 && s.stream_k) || (g.workspace == nullptr && g.M > 128 && g.M <= 256)))
     return MidPlan{};
   MidPlan best{};
-  double best_us = g.rows_kernel == 4 ? 1e30 : 0.93 * s.us + 1.2;
+  double best_us = g.rows_kernel == 4 ? 1e30 : 0.92 * s.us + 2.4;
   const int lo = g.rows_kernel == 4 ? (g.split_k > 0 ? g.split_k : 1) : g.keep_order != 0 ? s.split_k : 1;
   const int hi = g.rows_kernel == 4 || g.keep_order != 0 ? lo : g.workspace == nullptr ? 1 : 4;   // without a workspace: one sum in the order of k
   for (int split = lo; split <= hi; ++split) {

@@ -9,7 +9,7 @@ from nanoflow_b200 import ops
     (288, 8192, 28672, 0, 2), (576, 8192, 28672, 0, 1), (288, 8192, 8192, 0, 2), (576, 8192, 8192, 0, 1), (576, 4096, 14336, 0, 2), (288, 32000, 8192, 0, 1),
     (288, 18944, 3584, 1, 1),
     (256, 8192, 28672, 0, 0), (512, 8192, 28672, 0, 0), (960, 8192, 28672, 0, 0), (1000, 8192, 28672, 0, 0), (1000, 8192, 8192, 0, 0), (160, 10240, 8192, 0, 0),
-    (416, 10240, 8192, 0, 0), (333, 32000, 8192, 0, 0), (480, 32000, 8192, 0, 0), (896, 32000, 8192, 0, 0), (448, 128256, 4096, 0, 0), (960, 5120, 13824, 0, 0),
+    (416, 10240, 8192, 0, 0), (333, 32000, 8192, 0, 0), (480, 32000, 8192, 0, 0), (896, 32000, 8192, 0, 0), (448, 128256, 4096, 0, 0), (960, 5120, 13824, 0, 0), (320, 5120, 5120, 0, 0), (416, 4096, 14336, 0, 0), (288, 4096, 4096, 0, 0), (288, 14336, 4096, 1, 0), (192, 2048, 8192, 0, 0),
     (333, 28672, 8192, 1, 0), (416, 28672, 8192, 1, 0), (896, 28672, 8192, 1, 0), (448, 22016, 8192, 1, 0), (700, 22016, 8192, 1, 0), (896, 18944, 3584, 1, 0)])
 def test_each_side(M, N, K, gated, parts):
     assert ops.gemm_plan(M, N, K, swiglu=bool(gated), workspace_bytes=160 << 20)["mid_rows"] == parts
@@ -18,6 +18,13 @@ def test_each_side(M, N, K, gated, parts):
 @pytest.mark.parametrize("M", [1, 16, 32])
 def test_few_rows_of_a_head_in_kept_order(M):
     assert ops.gemm_plan(M, 128256, 4096, keep_order=True, workspace_bytes=160 << 20)["mid_rows"] == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 32000, 8192), (333, 32000, 8192), (333, 128256, 4096)])
+def test_some_rows_of_a_head_in_kept_order(M, N, K):
+    """Whose other shape is four M tiles of 128 columns, half as fast."""
+    plan = ops.gemm_plan(M, N, K, keep_order=True, workspace_bytes=160 << 20)
+    assert plan["tile_m"] == 4 and plan["mid_rows"] == 1
 
 
 @pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (64, 4096, 4096), (64, 4096, 14336), (96, 8192, 8192)])
