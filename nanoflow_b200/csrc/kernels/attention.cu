@@ -6,7 +6,7 @@
 //                   alternate pages of the item, each with its own cp.async ring, and merge their
 //                   softmax states in shared memory at the end. Optional split-KV writes per-chunk
 //                   partials to a workspace; the chunk that finishes last merges them, or a second
-//                   launch where the chunks are not listed.
+//                   launch where they are not listed or the caller has no words to count them in.
 // nfk_attn_prefill  causal, ragged query lengths (chunked prefill). A work item is (request, first
 //                   token, token count <= 128/group) x kv head; 8 warps x 16 rows, K/V tiles of 64
 //                   tokens double-buffered in shared memory and shared by all warps.
